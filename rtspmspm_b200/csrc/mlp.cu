@@ -137,12 +137,6 @@ constexpr int kOffW3 = kOffB2 + kMlpHidden;
 constexpr int kOffB3 = kOffW3 + kMlpHidden * kMlpOut;
 static_assert(kOffB3 + kMlpOut == kMlpParams, "parameter layout");
 
-// Loads the BF16 parameters (weights and biases) into shared memory as FP32.
-__device__ __forceinline__ void load_params(const __nv_bfloat16* w, float* sw) {
-  for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) sw[i] = __bfloat162float(w[i]);
-  __syncthreads();
-}
-
 // ---------------------------------------------------------------------------
 // Tensor-core inference: the MLP on 16-row tiles with mma.sync m16n8k16
 // (BF16 operands, FP32 accumulation).  Weights live in shared memory
@@ -398,123 +392,209 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_learned_plan(DCsr A, DCsr B
   }
 }
 
-// Training, step 1 of 3 (one thread per row of the minibatch): forward
-// with BF16 weights; keeps h1, z2 and dL/do for the backward kernels.
+// Training step on a minibatch: k_mlp_step runs forward and backward of
+// kStepRows rows at a time in shared memory and keeps its rows' share of
+// every gradient in registers; k_mlp_fold adds the CTAs' shares in CTA order
+// (deterministic, no atomics).
 // Loss = 0.5 * mean over rows of sum_o w_o (y_o - t_o)^2 with w = (1, 1/4).
-constexpr int kTrainThreads = 128;
+//
+// Bound: launch latency and the dependent FMA chains of one tile (4,096 rows
+// are 128 tiles, under one a SM; 0.1 GFLOP in all).  One thread per parameter
+// walking all the rows in turn took 298 us of a 373 us step at 4,096 rows
+// (cold, summed over its four launches), and every layer's activations went
+// through memory; 32-row tiles fill the SMs from 4,736 rows up and leave each
+// thread a 2 x 4 (rows x units) or 4 x 4 (unit x unit gradient) register
+// tile.  spg_mlp_grad of 4,096 rows: 304 -> 62 us a call.
 constexpr float kLossW0 = 1.0f;
 constexpr float kLossW1 = 0.25f;
+constexpr int kStepThreads = 256;
+constexpr int kStepRows = 32;
+constexpr int kStepPitch = kMlpHidden + 4;  // row pitch: 16-byte aligned, rows on different banks
+constexpr int kStepSums = kMlpParams + 1;   // every gradient and the loss
 
-__global__ void __launch_bounds__(kTrainThreads) k_mlp_fwd(const __nv_bfloat16* w, const float* feats,
+struct StepSmem {
+  float w1[kMlpIn * kMlpHidden], w2[kMlpHidden * kMlpHidden], w2t[kMlpHidden * kStepPitch];
+  float w3[kMlpHidden * kMlpOut], b1[kMlpHidden], b2[kMlpHidden];
+  float x[kStepRows * kMlpIn], h1[kStepRows * kStepPitch], z2[kStepRows * kStepPitch];
+  float dz1[kStepRows * kStepPitch], dz2[kStepRows * kStepPitch];
+  float dout[kStepRows * kMlpOut], loss[kStepRows], b3[kMlpOut];
+};
+
+__global__ void __launch_bounds__(kStepThreads) k_mlp_step(const __nv_bfloat16* w, const float* feats,
                                                              const float* targets, int64_t n, float inv_n,
-                                                             float* h1_out, float* z2_out, float* do_out,
-                                                             float* loss_rows) {
-  extern __shared__ float sw[];
-  load_params(w, sw);
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-    const volatile float* vw = sw;
-    float x[kMlpIn], h1[kMlpHidden];
+                                                             float* sums) {
+  extern __shared__ float4 sm_step[];
+  StepSmem& sm = *reinterpret_cast<StepSmem*>(sm_step);
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  for (int i = tid; i < kMlpIn * kMlpHidden; i += kStepThreads) sm.w1[i] = __bfloat162float(w[kOffW1 + i]);
+  for (int i = tid; i < kMlpHidden * kMlpHidden; i += kStepThreads) {
+    const float v = __bfloat162float(w[kOffW2 + i]);
+    sm.w2[i] = v;
+    sm.w2t[(i % kMlpHidden) * kStepPitch + i / kMlpHidden] = v;
+  }
+  for (int i = tid; i < kMlpHidden * kMlpOut; i += kStepThreads) sm.w3[i] = __bfloat162float(w[kOffW3 + i]);
+  for (int i = tid; i < kMlpHidden; i += kStepThreads) {
+    sm.b1[i] = __bfloat162float(w[kOffB1 + i]);
+    sm.b2[i] = __bfloat162float(w[kOffB2 + i]);
+  }
+  if (tid < kMlpOut) sm.b3[tid] = __bfloat162float(w[kOffB3 + tid]);
+  // this CTA's share of the gradients: W2[4 ty ..][4 tx ..] and two of W1 in
+  // every thread; one of W3 (threads 0..127), b1 (128..191), b2 (192..255),
+  // b3 and the loss (0..2)
+  float g2[4][4] = {}, g1[2] = {}, g3 = 0.f, gb = 0.f;
+  const int64_t ntiles = (n + kStepRows - 1) / kStepRows;
+  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const int64_t r0 = t * kStepRows;
+    const int nr = (int)min((int64_t)kStepRows, n - r0);
+    __syncthreads();  // weights stored; the previous tile's rows read
+    sm.x[tid] = tid < nr * kMlpIn ? feats[r0 * kMlpIn + tid] : 0.f;
+    __syncthreads();
+    // rows 2 ty, 2 ty + 1, units 4 tx .. 4 tx + 3
 #pragma unroll
-    for (int i = 0; i < kMlpIn; ++i) x[i] = feats[r * kMlpIn + i];
+    for (int rr = 0; rr < 2; ++rr) {
+      const int r = 2 * ty + rr;
 #pragma unroll
-    for (int j = 0; j < kMlpHidden; ++j) {
-      float a = vw[kOffB1 + j];
+      for (int c = 0; c < 4; ++c) {
+        const int j = 4 * tx + c;
+        float a = sm.b1[j];
 #pragma unroll
-      for (int i = 0; i < kMlpIn; ++i) a += x[i] * vw[kOffW1 + i * kMlpHidden + j];
-      h1[j] = a > 0.f ? a : 0.f;
-      h1_out[r * kMlpHidden + j] = h1[j];
+        for (int i = 0; i < kMlpIn; ++i) a = fmaf(sm.x[r * kMlpIn + i], sm.w1[i * kMlpHidden + j], a);
+        sm.h1[r * kStepPitch + j] = a > 0.f ? a : 0.f;
+      }
     }
-    float o0 = vw[kOffB3], o1 = vw[kOffB3 + 1];
-#pragma unroll 1
-    for (int j = 0; j < kMlpHidden; ++j) {
-      float a = vw[kOffB2 + j];
+    __syncthreads();
+    {
+      float z[2][4];
 #pragma unroll
-      for (int i = 0; i < kMlpHidden; ++i) a += h1[i] * vw[kOffW2 + i * kMlpHidden + j];
-      z2_out[r * kMlpHidden + j] = a;
-      const float h = a > 0.f ? a : 0.f;
-      o0 += h * vw[kOffW3 + j * kMlpOut + 0];
-      o1 += h * vw[kOffW3 + j * kMlpOut + 1];
+      for (int c = 0; c < 4; ++c) z[0][c] = z[1][c] = sm.b2[4 * tx + c];
+#pragma unroll 8
+      for (int i = 0; i < kMlpHidden; ++i) {
+        const float4 wv = *reinterpret_cast<const float4*>(&sm.w2[i * kMlpHidden + 4 * tx]);
+#pragma unroll
+        for (int rr = 0; rr < 2; ++rr) {
+          const float h = sm.h1[(2 * ty + rr) * kStepPitch + i];
+          z[rr][0] = fmaf(h, wv.x, z[rr][0]);
+          z[rr][1] = fmaf(h, wv.y, z[rr][1]);
+          z[rr][2] = fmaf(h, wv.z, z[rr][2]);
+          z[rr][3] = fmaf(h, wv.w, z[rr][3]);
+        }
+      }
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr)
+        *reinterpret_cast<float4*>(&sm.z2[(2 * ty + rr) * kStepPitch + 4 * tx]) =
+            make_float4(z[rr][0], z[rr][1], z[rr][2], z[rr][3]);
     }
-    const float e0 = o0 - targets[r * kMlpOut + 0];
-    const float e1 = o1 - targets[r * kMlpOut + 1];
-    do_out[r * kMlpOut + 0] = kLossW0 * e0 * inv_n;
-    do_out[r * kMlpOut + 1] = kLossW1 * e1 * inv_n;
-    loss_rows[r] = 0.5f * (kLossW0 * e0 * e0 + kLossW1 * e1 * e1);
+    __syncthreads();
+    // outputs, one thread each; rows past n add nothing to any sum
+    if (tid < kStepRows * kMlpOut) {
+      const int r = tid >> 1, o = tid & 1;
+      float e = 0.f;
+      if (r < nr) {
+        float y = sm.b3[o];
+#pragma unroll 8
+        for (int j = 0; j < kMlpHidden; ++j) {
+          const float z = sm.z2[r * kStepPitch + j];
+          y = fmaf(z > 0.f ? z : 0.f, sm.w3[j * kMlpOut + o], y);
+        }
+        e = y - targets[(r0 + r) * kMlpOut + o];
+      }
+      const float lw = o == 0 ? kLossW0 : kLossW1;
+      sm.dout[tid] = lw * e * inv_n;
+      const float mine = lw * e * e;
+      const float other = __shfl_xor_sync(kFull, mine, 1);
+      if (o == 0) sm.loss[r] = 0.5f * (mine + other);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) {
+      const int r = 2 * ty + rr;
+      const float d0 = sm.dout[r * kMlpOut], d1 = sm.dout[r * kMlpOut + 1];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int j = 4 * tx + c;
+        sm.dz2[r * kStepPitch + j] =
+            sm.z2[r * kStepPitch + j] > 0.f ? d0 * sm.w3[j * kMlpOut] + d1 * sm.w3[j * kMlpOut + 1] : 0.f;
+      }
+    }
+    __syncthreads();
+    {
+      float d[2][4] = {};
+#pragma unroll 8
+      for (int j = 0; j < kMlpHidden; ++j) {
+        const float4 wv = *reinterpret_cast<const float4*>(&sm.w2t[j * kStepPitch + 4 * tx]);
+#pragma unroll
+        for (int rr = 0; rr < 2; ++rr) {
+          const float z = sm.dz2[(2 * ty + rr) * kStepPitch + j];
+          d[rr][0] = fmaf(z, wv.x, d[rr][0]);
+          d[rr][1] = fmaf(z, wv.y, d[rr][1]);
+          d[rr][2] = fmaf(z, wv.z, d[rr][2]);
+          d[rr][3] = fmaf(z, wv.w, d[rr][3]);
+        }
+      }
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int at = (2 * ty + rr) * kStepPitch + 4 * tx + c;
+          sm.dz1[at] = sm.h1[at] > 0.f ? d[rr][c] : 0.f;
+        }
+    }
+    __syncthreads();
+    // the tile's share of the gradients, rows in order
+#pragma unroll 4
+    for (int r = 0; r < kStepRows; ++r) {
+      const float4 hv = *reinterpret_cast<const float4*>(&sm.h1[r * kStepPitch + 4 * ty]);
+      const float4 dv = *reinterpret_cast<const float4*>(&sm.dz2[r * kStepPitch + 4 * tx]);
+      const float h[4] = {hv.x, hv.y, hv.z, hv.w}, d[4] = {dv.x, dv.y, dv.z, dv.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) g2[i][j] = fmaf(h[i], d[j], g2[i][j]);
+      const float z1 = sm.dz1[r * kStepPitch + (tid & 63)];
+      g1[0] = fmaf(sm.x[r * kMlpIn + (tid >> 6)], z1, g1[0]);
+      g1[1] = fmaf(sm.x[r * kMlpIn + (tid >> 6) + 4], z1, g1[1]);
+      if (tid < kMlpHidden * kMlpOut) {
+        const float z = sm.z2[r * kStepPitch + (tid >> 1)];
+        g3 = fmaf(z > 0.f ? z : 0.f, sm.dout[r * kMlpOut + (tid & 1)], g3);
+        if (tid < 3) gb += tid < kMlpOut ? sm.dout[r * kMlpOut + tid] : sm.loss[r];
+      } else {
+        gb += tid < 192 ? sm.dz1[r * kStepPitch + tid - 128] : sm.dz2[r * kStepPitch + tid - 192];
+      }
+    }
+  }
+  float* mine = sums + (int64_t)blockIdx.x * kStepSums;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) mine[kOffW2 + (4 * ty + i) * kMlpHidden + 4 * tx + j] = g2[i][j];
+  mine[kOffW1 + tid] = g1[0];
+  mine[kOffW1 + 4 * kMlpHidden + tid] = g1[1];
+  if (tid < kMlpHidden * kMlpOut) {
+    mine[kOffW3 + tid] = g3;
+    if (tid < 3) mine[kOffB3 + tid] = gb;
+  } else {
+    mine[tid < 192 ? kOffB1 + tid - 128 : kOffB2 + tid - 192] = gb;
   }
 }
 
-// Training, step 2 of 3 (one thread per row): back-propagates dL/do into
-// dL/dz2 and dL/dz1 (pre-activation gradients of both hidden layers).
-__global__ void __launch_bounds__(kTrainThreads) k_mlp_bwd_rows(const __nv_bfloat16* w, int64_t n, const float* h1_in,
-                                                                  const float* z2_in, const float* do_in,
-                                                                  float* dz1_out, float* dz2_out) {
-  extern __shared__ float sw[];
-  load_params(w, sw);
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-    const volatile float* vw = sw;
-    const float d0 = do_in[r * kMlpOut + 0], d1 = do_in[r * kMlpOut + 1];
-    float dh1[kMlpHidden];
-#pragma unroll
-    for (int i = 0; i < kMlpHidden; ++i) dh1[i] = 0.f;
-#pragma unroll 1
-    for (int j = 0; j < kMlpHidden; ++j) {
-      const float z = z2_in[r * kMlpHidden + j];
-      const float dz = z > 0.f ? d0 * vw[kOffW3 + j * kMlpOut + 0] + d1 * vw[kOffW3 + j * kMlpOut + 1] : 0.f;
-      dz2_out[r * kMlpHidden + j] = dz;
-#pragma unroll
-      for (int i = 0; i < kMlpHidden; ++i) dh1[i] += dz * vw[kOffW2 + i * kMlpHidden + j];
-    }
-#pragma unroll
-    for (int i = 0; i < kMlpHidden; ++i)
-      dz1_out[r * kMlpHidden + i] = h1_in[r * kMlpHidden + i] > 0.f ? dh1[i] : 0.f;
-  }
-}
-
-// Training, step 3 of 3 (one thread per parameter): each gradient is a sum
-// over the minibatch rows in row order -- deterministic, no atomics.
-__global__ void k_mlp_grad_reduce(const float* feats, int64_t n, const float* h1, const float* z2, const float* d_o,
-                                  const float* dz1, const float* dz2, float* grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kMlpParams) return;
-  float g = 0.f;
-  if (p < kOffB1) {  // W1[f][i]
-    const int f = (p - kOffW1) / kMlpHidden, i = (p - kOffW1) % kMlpHidden;
-    for (int64_t r = 0; r < n; ++r) g += feats[r * kMlpIn + f] * dz1[r * kMlpHidden + i];
-  } else if (p < kOffW2) {  // b1[i]
-    const int i = p - kOffB1;
-    for (int64_t r = 0; r < n; ++r) g += dz1[r * kMlpHidden + i];
-  } else if (p < kOffB2) {  // W2[i][j]
-    const int i = (p - kOffW2) / kMlpHidden, j = (p - kOffW2) % kMlpHidden;
-    for (int64_t r = 0; r < n; ++r) g += h1[r * kMlpHidden + i] * dz2[r * kMlpHidden + j];
-  } else if (p < kOffW3) {  // b2[j]
-    const int j = p - kOffB2;
-    for (int64_t r = 0; r < n; ++r) g += dz2[r * kMlpHidden + j];
-  } else if (p < kOffB3) {  // W3[j][k]
-    const int j = (p - kOffW3) / kMlpOut, k = (p - kOffW3) % kMlpOut;
-    for (int64_t r = 0; r < n; ++r) {
-      const float z = z2[r * kMlpHidden + j];
-      g += (z > 0.f ? z : 0.f) * d_o[r * kMlpOut + k];
-    }
-  } else {  // b3[k]
-    const int k = p - kOffB3;
-    for (int64_t r = 0; r < n; ++r) g += d_o[r * kMlpOut + k];
-  }
-  grad[p] = g;
-}
-
-// Sum of per-row losses divided by n (single CTA, fixed order per thread).
-__global__ void k_loss_mean(const float* loss_rows, int64_t n, float inv_n, float* out) {
-  __shared__ float sh[32];
+// The CTAs' shares added up: 32 parameters a CTA (the loss is the last), warp
+// w taking shares w, w + 8, ... of them, then the warps' sums in warp order.
+__global__ void __launch_bounds__(256) k_mlp_fold(const float* sums, int parts, float inv_n, float* grad,
+                                                  float* loss) {
+  __shared__ float sh[8][32];
+  const int lane = lane_id(), wib = threadIdx.x >> 5;
+  const int p = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int64_t r = threadIdx.x; r < n; r += blockDim.x) s += loss_rows[r];
-  s = warp_sum(s);
-  if (lane_id() == 0) sh[threadIdx.x >> 5] = s;
+  if (p < kStepSums)
+#pragma unroll 4
+    for (int i = wib; i < parts; i += 8) s += sums[(int64_t)i * kStepSums + p];
+  sh[wib][lane] = s;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    float v = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.f;
-    v = warp_sum(v);
-    if (threadIdx.x == 0) *out = v * inv_n;
-  }
+  if (wib != 0 || p >= kStepSums) return;
+#pragma unroll
+  for (int i = 1; i < 8; ++i) s += sh[i][lane];
+  if (p < kMlpParams) grad[p] = s;
+  else if (loss) *loss = s * inv_n;
 }
 
 // Adam with decoupled weight decay on the FP32 master weights; refreshes
@@ -621,26 +701,26 @@ void launch_learned_plan_batch(const BatchMat* mats, const int32_t* row_mat, int
       cap, need_exact, n_exact);
 }
 
-void launch_mlp_fwd_bwd(const void* w16, const float* feats, const float* targets, int64_t n, float* work,
-                        float* grad, float* loss, const LaunchCtx& lc) {
-  if (n == 0) return;
-  float* h1 = work;
-  float* z2 = h1 + n * kMlpHidden;
-  float* dz1 = z2 + n * kMlpHidden;
-  float* dz2 = dz1 + n * kMlpHidden;
-  float* d_o = dz2 + n * kMlpHidden;
-  float* lrows = d_o + n * kMlpOut;
-  const int blocks = mlp_blocks(n, kTrainThreads, lc.sms);
-  const size_t smem = kMlpParams * sizeof(float);
-  const float inv_n = 1.0f / (float)n;
-  k_mlp_fwd<<<blocks, kTrainThreads, smem, lc.stream>>>((const __nv_bfloat16*)w16, feats, targets, n, inv_n, h1, z2,
-                                                        d_o, lrows);
-  k_mlp_bwd_rows<<<blocks, kTrainThreads, smem, lc.stream>>>((const __nv_bfloat16*)w16, n, h1, z2, d_o, dz1, dz2);
-  k_mlp_grad_reduce<<<(kMlpParams + 127) / 128, 128, 0, lc.stream>>>(feats, n, h1, z2, d_o, dz1, dz2, grad);
-  if (loss) k_loss_mean<<<1, 1024, 0, lc.stream>>>(lrows, n, inv_n, loss);
+// CTAs of the training step: a tile each, up to two an SM.
+static int step_parts(int64_t n, int sms) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>((n + kStepRows - 1) / kStepRows, (int64_t)sms * 2));
 }
 
-int64_t mlp_work_floats(int64_t n) { return n * (4 * kMlpHidden + kMlpOut + 1); }
+cudaError_t launch_mlp_fwd_bwd(const void* w16, const float* feats, const float* targets, int64_t n, float* work,
+                               float* grad, float* loss, const LaunchCtx& lc) {
+  if (n == 0) return cudaSuccess;
+  const int parts = step_parts(n, lc.sms);
+  const float inv_n = 1.0f / (float)n;
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_mlp_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StepSmem));
+  if (e != cudaSuccess) return e;
+  k_mlp_step<<<parts, kStepThreads, sizeof(StepSmem), lc.stream>>>((const __nv_bfloat16*)w16, feats, targets, n, inv_n,
+                                                                   work);
+  k_mlp_fold<<<(kStepSums + 31) / 32, 256, 0, lc.stream>>>(work, parts, inv_n, grad, loss);
+  return cudaGetLastError();
+}
+
+int64_t mlp_work_floats(int64_t n, int sms) { return (int64_t)step_parts(n, sms) * kStepSums; }
 
 void launch_adam(float* master, void* w16, float* grad, float* m, float* v, float lr, float beta1, float beta2,
                  float eps, float wd, int step, const LaunchCtx& lc) {

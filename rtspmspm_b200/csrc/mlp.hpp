@@ -27,11 +27,12 @@ struct BatchMat;
 void launch_learned_plan_batch(const BatchMat* mats, const int32_t* row_mat, int64_t R, const void* w16, float margin,
                                int slack, int64_t learn_cap, int force_overflow, int64_t* prod, int64_t* cap,
                                uint8_t* need_exact, unsigned long long* n_exact, const LaunchCtx& lc);
-// Forward + backward over n rows; `work` holds mlp_work_floats(n) floats;
-// grad gets the full gradient (overwritten); loss (device) the mean loss.
-void launch_mlp_fwd_bwd(const void* w16, const float* feats, const float* targets, int64_t n, float* work,
-                        float* grad, float* loss, const LaunchCtx& lc);
-int64_t mlp_work_floats(int64_t n);
+// Forward + backward over n rows; `work` holds mlp_work_floats(n, sms) floats;
+// grad gets the full gradient (overwritten); loss (a word the device can
+// write, or null) the mean loss.
+cudaError_t launch_mlp_fwd_bwd(const void* w16, const float* feats, const float* targets, int64_t n, float* work,
+                               float* grad, float* loss, const LaunchCtx& lc);
+int64_t mlp_work_floats(int64_t n, int sms);
 void launch_adam(float* master, void* w16, float* grad, float* m, float* v, float lr, float beta1, float beta2,
                  float eps, float wd, int step, const LaunchCtx& lc);
 void launch_to_bf16(const float* src, void* dst, int n, const LaunchCtx& lc);

@@ -208,16 +208,17 @@ spg_status spg_mlp_grad(spg_ctx* ctx, const float* d_features, const float* d_ta
   if (!ctx || rows <= 0 || !d_features || !d_targets || !grads) return SPG_ERR_INVALID_ARG;
   SPG_CUDA(ctx, cudaSetDevice(ctx->device));
   SPG_TRY(ensure_mlp(ctx));
-  DevBuf work, g, l;
-  SPG_TRY(work.alloc(ctx, (size_t)mlp_work_floats(rows) * 4));
+  DevBuf work, g;
+  SPG_TRY(work.alloc(ctx, (size_t)mlp_work_floats(rows, ctx->sms) * 4));
   SPG_TRY(g.alloc(ctx, kMlpParams * 4));
-  SPG_TRY(l.alloc(ctx, 4));
-  launch_mlp_fwd_bwd(ctx->mlp_w16, d_features, d_targets, rows, work.as<float>(), g.as<float>(), l.as<float>(),
-                     launch_ctx(ctx));
+  // the kernel writes the loss into a mapped staging word
+  constexpr int kLossSlot = 31;
+  SPG_CUDA(ctx, launch_mlp_fwd_bwd(ctx->mlp_w16, d_features, d_targets, rows, work.as<float>(), g.as<float>(),
+                                   reinterpret_cast<float*>(ctx->h_stage_dev + kLossSlot), launch_ctx(ctx)));
   SPG_CUDA(ctx, cudaMemcpyAsync(grads, g.get(), kMlpParams * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  float lh = 0.f;
-  SPG_CUDA(ctx, cudaMemcpyAsync(&lh, l.get(), 4, cudaMemcpyDeviceToHost, ctx->stream));
   SPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  float lh = 0.f;
+  std::memcpy(&lh, &ctx->h_stage[kLossSlot], sizeof lh);
   if (loss) *loss = lh;
   return SPG_OK;
 }
@@ -308,7 +309,7 @@ spg_status spg_mlp_train(spg_ctx* ctx, int32_t n, const spg_csr* A, const spg_cs
   SPG_TRY(perm.alloc(ctx, (size_t)R * 4));
   SPG_TRY(bfeat.alloc(ctx, (size_t)bs * kMlpIn * 4));
   SPG_TRY(btgt.alloc(ctx, (size_t)bs * kMlpOut * 4));
-  SPG_TRY(work.alloc(ctx, (size_t)mlp_work_floats(bs) * 4));
+  SPG_TRY(work.alloc(ctx, (size_t)mlp_work_floats(bs, ctx->sms) * 4));
   SPG_TRY(grad.alloc(ctx, kMlpParams * 4));
   SPG_TRY(m1.alloc(ctx, kMlpParams * 4));
   SPG_TRY(m2.alloc(ctx, kMlpParams * 4));
@@ -328,8 +329,8 @@ spg_status spg_mlp_train(spg_ctx* ctx, int32_t n, const spg_csr* A, const spg_cs
       const int64_t cnt = std::min<int64_t>(bs, R - s0);
       launch_gather_rows(dfeat.as<float>(), perm.as<int32_t>() + s0, cnt, kMlpIn, bfeat.as<float>(), lc);
       launch_gather_rows(dtgt.as<float>(), perm.as<int32_t>() + s0, cnt, kMlpOut, btgt.as<float>(), lc);
-      launch_mlp_fwd_bwd(ctx->mlp_w16, bfeat.as<float>(), btgt.as<float>(), cnt, work.as<float>(), grad.as<float>(),
-                         losses.as<float>() + step, lc);
+      SPG_CUDA(ctx, launch_mlp_fwd_bwd(ctx->mlp_w16, bfeat.as<float>(), btgt.as<float>(), cnt, work.as<float>(),
+                                       grad.as<float>(), losses.as<float>() + step, lc));
       ++step;
       const float lr = o.lr * 0.5f * (1.0f + std::cos(3.14159265f * (float)step / (float)total_steps));
       launch_adam(ctx->mlp_master, ctx->mlp_w16, grad.as<float>(), m1.as<float>(), m2.as<float>(), lr, 0.9f, 0.999f,

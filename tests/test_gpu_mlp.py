@@ -32,6 +32,23 @@ def test_backward_matches_fp64_reference(engine):
     assert err < 1e-3, err
 
 
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 9473, 20000])
+def test_step_tiles_match_fp64_reference(engine, rows):
+    """One row, around one 32-row tile, and past two tiles a CTA (2 x 148 x
+    32 = 9,472 rows).  An FP32 gradient passes through about 150 roundings a
+    row and as many in the sums: 300 x 2^-24 = 1.8e-5 of the largest, held
+    to 1e-4."""
+    import torch
+
+    engine.mlp_init(11)
+    p = engine.mlp_params()
+    x, t = _batch(rows, rows)
+    loss, g = engine.mlp_grad(torch.from_numpy(x).cuda(), torch.from_numpy(t).cuda())
+    rl, rg = mlp_oracle.loss_and_grad(p, x, t)
+    assert abs(loss - rl) <= 1e-4 * max(1.0, abs(rl))
+    assert np.abs(g - rg).max() <= 1e-4 * np.abs(rg).max()
+
+
 def test_tensor_core_inference_matches_reference(engine):
     import torch
 
