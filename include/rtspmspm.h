@@ -180,8 +180,8 @@ spg_status spg_multiply_into_host(spg_ctx* ctx, const spg_csr* A, const spg_csr*
  * are counted from C's sorted columns).  C->col_idx is rewritten with the
  * same columns.  As with cuSPARSE's reuse, the caller guarantees that A and
  * B keep the structure C was computed from; a differing count of distinct
- * columns in a row (in a column tile holding entries of C, for rows beyond
- * the warp tables) fails the call with SPG_ERR_INVALID_ARG.
+ * columns in a row (in a run of column tiles holding entries of C, for rows
+ * beyond the warp tables) fails the call with SPG_ERR_INVALID_ARG.
  * report->products is not computed (0).
  * Replaces: cusparseSpGEMMreuse_compute after the structure phase
  * (cuSparse/src/main.cpp:98-296, second compute with new values :286-296).
@@ -395,11 +395,12 @@ typedef struct spg_tuning {
     float   predict_margin;    /* learned: capacity = margin * predicted + slack */
     int32_t predict_slack;
     float   learned_load;      /* learned: table load factor at the predicted capacity */
-    int32_t heavy_path;        /* rows beyond the warp tables: 0 = every column tile rescans
-                                  its row of A; 1 = products staged once per tile in HBM
-                                  buckets when they fit (else as 0); 2 = as 0, with B-row
-                                  segments of 64+ entries in a tile copied into shared
-                                  memory by bulk copies (cp.async.bulk, mbarrier) */
+    int32_t heavy_path;        /* rows beyond the warp tables: 0 = units of consecutive column
+                                  tiles with accumulators for their output entries; 1 =
+                                  products staged once per tile in HBM buckets when they fit
+                                  (else as 0); 2 = every column tile rescans its row of A,
+                                  with B-row segments of 64+ entries copied into shared
+                                  memory by bulk copies (cp.async.bulk, mbarrier; else as 0) */
     int32_t block_min_nnz;     /* > 0: rows with more output entries than this (and at most
                                   8192) use a CTA-wide hash table; 0 or -1 (default): off,
                                   warp tables and heavy-row tiles only */

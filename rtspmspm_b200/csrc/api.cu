@@ -240,6 +240,9 @@ namespace {
 
 // Largest blocked index of B built for the heavy-row tiles (bytes).
 constexpr size_t kBlockedIndexMaxBytes = size_t(4) << 30;
+// Largest set of column bitmaps the symbolic pass leaves for the heavy-row
+// units (bytes).
+constexpr size_t kBitmapMaxBytes = size_t(8) << 30;
 // Largest list of non-empty heavy-row tiles (bytes).
 constexpr size_t kWorkListMaxBytes = size_t(4) << 30;
 
@@ -263,6 +266,7 @@ struct Pipeline {
   DevBuf big_slot;    // int32 rows
   DevBuf tile_cnt;    // int32 nbig * ntiles
   DevBuf tile_off;    // int32 nbig * ntiles
+  DevBuf bitmap;      // uint32 nbig * bitmap_stride(), or empty
   DevBuf scan_tmp;    // int64
   int64_t h_off[kNumBins + 1] = {};
   int64_t nbig = 0;
@@ -306,6 +310,9 @@ struct Pipeline {
     return SPG_OK;
   }
 
+  // Words of a big row's column bitmap.
+  int64_t bitmap_stride() const { return (int64_t)ntiles * (kTileCols / 32); }
+
   int64_t bin_size(int b) const { return h_off[b + 1] - h_off[b]; }
   const int32_t* bin_rows(int b) { return lists.as<int32_t>() + h_off[b]; }
 
@@ -326,6 +333,21 @@ struct Pipeline {
       SPG_TRY(tile_cnt.alloc(ctx, tb));
       SPG_TRY(tile_off.alloc(ctx, tb));
       SPG_CUDA(ctx, cudaMemsetAsync(tile_cnt.get(), 0, tb, ctx->stream));
+      // when one bitmap window holds a row and the budget all big rows'
+      // bitmaps, every big row takes the bitmap kernel and leaves its bitmap
+      // for the units (which else walk their products once more for it)
+      const size_t bitmap_bytes = (size_t)nbig * (size_t)bitmap_stride() * 4;
+      size_t free_b = 0, total_b = 0;
+      cudaMemGetInfo(&free_b, &total_b);
+      if (tune.heavy_path == 0 && bitmap_stride() <= kDenseWindowWords && bitmap_bytes <= kBitmapMaxBytes &&
+          bitmap_bytes < free_b / 8)
+        SPG_TRY(bitmap.alloc(ctx, bitmap_bytes));
+      if (bitmap.get()) {
+        launch_sym_dense(A.view, B.view, bin_rows(kBinBlock), nbig, 0, nnz.as<int64_t>(), big_slot.as<int32_t>(),
+                         tile_cnt.as<int32_t>(), ntiles, bitmap.as<uint32_t>(), ctx->d_flags, lc);
+        ++ctx->launches;
+        return SPG_OK;
+      }
       if (nblock) {
         launch_sym_block(A.view, B.view, bin_rows(kBinBlock), nblock, block_table_log(tune), 0, nnz.as<int64_t>(),
                          big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles, ctx->d_flags, lc);
@@ -333,11 +355,26 @@ struct Pipeline {
       }
       if (ndense) {
         launch_sym_dense(A.view, B.view, bin_rows(kBinDense), ndense, nblock, nnz.as<int64_t>(),
-                         big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles, ctx->d_flags, lc);
+                         big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles, nullptr, ctx->d_flags, lc);
         ++ctx->launches;
       }
     }
     return SPG_OK;
+  }
+
+  // C's column and value arrays; gives the bitmaps back (the units then find
+  // their columns themselves) when the device has no room beside them.
+  spg_status alloc_entries(int64_t total, DevBuf& c_col, DevBuf& c_val) {
+    spg_status st = SPG_OK;
+    for (int pass = 0; pass < 2; ++pass) {
+      st = c_col.alloc(ctx, (size_t)total * 4);
+      if (st == SPG_OK) st = c_val.alloc(ctx, (size_t)total * 4);
+      if (st != SPG_ERR_OUT_OF_MEMORY || !bitmap.get()) break;
+      c_col.reset();
+      bitmap.reset();
+      SPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    }
+    return st;
   }
 
   // Numeric pass for the rows in the current (numeric) binning, into C.
@@ -352,7 +389,52 @@ struct Pipeline {
     return e;
   }
 
-  spg_status numeric(const int64_t* c_rp, int32_t* c_col, float* c_val, spg_report* rep,
+  // The opt-in heavy paths, every 2^kTileShift-column tile by itself:
+  // heavy_path 1, each heavy row's products walked once into per-tile
+  // buckets (measured slower than rescanning on R-MAT: the bucket writes
+  // scatter over a buffer far larger than L2), and heavy_path 2, tiles that
+  // rescan their row with bulk copies of long segments.  *done stays false
+  // when the path does not apply (buckets or alignment).
+  spg_status numeric_tiles(const int64_t* c_rp, int32_t* c_col, float* c_val, const int32_t* bidx, size_t free_b,
+                           bool* done) {
+    const int64_t nheavy = bin_size(kBinHeavy);
+    if (tune.heavy_path == 2 && !bulk_aligned(B.view)) return SPG_OK;
+    // the list of non-empty (row, tile) units for the tile kernel, when it
+    // fits: rows of wide products touch a small part of their tiles
+    const size_t work_bytes = (size_t)nheavy * (size_t)ntiles * 8;
+    const bool use_list = tune.heavy_path == 2 && ntiles > 1 && work_bytes <= kWorkListMaxBytes &&
+                          work_bytes < free_b / 4;
+    DevBuf nz, work;
+    if (use_list) SPG_TRY(nz.alloc(ctx, (size_t)(nheavy + 1) * 8));
+    launch_tile_offsets(bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles,
+                        tile_off.as<int32_t>(), use_list ? nz.as<int64_t>() : nullptr, lc);
+    ++ctx->launches;
+    if (tune.heavy_path == 1)
+      return heavy_staged(ctx, A.view, B.view, bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(),
+                          tile_cnt.as<int32_t>(), tile_off.as<int32_t>(), ntiles, c_rp, c_col, c_val, done);
+    if (use_list) {
+      SPG_TRY(work.alloc(ctx, work_bytes));
+      launch_excl_scan(nz.as<int64_t>(), nheavy, nz.as<int64_t>(), scan_tmp.as<int64_t>(), lc);
+      launch_tile_worklist(bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles,
+                           nz.as<int64_t>(), work.as<int64_t>(), lc);
+      ctx->launches += 5;
+    }
+    DevBuf tocc;
+    if (bidx) {
+      SPG_TRY(tocc.alloc(ctx, (size_t)B.view.rows * (size_t)((ntiles + 31) / 32) * 4));
+      launch_build_tile_occupancy(B.view.rows, bidx, ntiles, tocc.as<uint32_t>(), lc);
+      ++ctx->launches;
+    }
+    launch_num_tile(A.view, B.view, bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(),
+                    tile_off.as<int32_t>(), ntiles, c_rp, c_col, c_val, bidx, tocc.as<uint32_t>(),
+                    use_list ? work.as<int64_t>() : nullptr, use_list ? nz.as<int64_t>() + nheavy : nullptr,
+                    ctx->d_counter, ctx->d_flags, lc);
+    ++ctx->launches;
+    *done = true;
+    return SPG_OK;
+  }
+
+  spg_status numeric(const int64_t* c_rp, int32_t* c_col, float* c_val, int64_t c_nnz, spg_report* rep,
                      const int64_t* row_prod = nullptr) {
     const EscArgs esc = esc_args(row_prod);
     for (int b = 0; b < kNumWarpBins; ++b) {
@@ -373,49 +455,26 @@ struct Pipeline {
       if (B.complete) SPG_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, B.complete, 0));
       size_t free_b = 0, total_b = 0;
       cudaMemGetInfo(&free_b, &total_b);
-      // the list of non-empty (row, tile) units for the tile kernel, when it
-      // fits: rows of wide products touch a small part of their tiles
-      const size_t work_bytes = (size_t)nheavy * (size_t)ntiles * 8;
-      const bool use_list = tune.heavy_path != 1 && ntiles > 1 && work_bytes <= kWorkListMaxBytes &&
-                            work_bytes < free_b / 4;
-      DevBuf nz, work;
-      if (use_list) SPG_TRY(nz.alloc(ctx, (size_t)(nheavy + 1) * 8));
-      launch_tile_offsets(bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles,
-                          tile_off.as<int32_t>(), use_list ? nz.as<int64_t>() : nullptr, lc);
-      if (use_list) {
-        SPG_TRY(work.alloc(ctx, work_bytes));
-        launch_excl_scan(nz.as<int64_t>(), nheavy, nz.as<int64_t>(), scan_tmp.as<int64_t>(), lc);
-        launch_tile_worklist(bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles,
-                             nz.as<int64_t>(), work.as<int64_t>(), lc);
-        ctx->launches += 5;
+      // a blocked index of B when it fits the budget (else per-unit binary
+      // searches)
+      DevBuf bidx;
+      const size_t bidx_bytes = (size_t)B.view.rows * (size_t)(ntiles + 1) * 4;
+      const bool use_index = ntiles > 1 && bidx_bytes <= kBlockedIndexMaxBytes && bidx_bytes < free_b / 4;
+      if (use_index) {
+        SPG_TRY(bidx.alloc(ctx, bidx_bytes));
+        launch_build_blocked_index(B.view, ntiles, bidx.as<int32_t>(), lc);
+        ++ctx->launches;
       }
-      // staged path (opt-in): each heavy row's products walked once into
-      // per-tile buckets; measured slower than rescanning on R-MAT (the
-      // bucket writes scatter over a buffer far larger than L2)
-      bool staged = false;
-      if (tune.heavy_path == 1)
-        SPG_TRY(heavy_staged(ctx, A.view, B.view, bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(),
-                             tile_cnt.as<int32_t>(), tile_off.as<int32_t>(), ntiles, c_rp, c_col, c_val, &staged));
-      if (!staged) {
-        // rescanning tile kernel, with a blocked index of B when it fits the
-        // budget (else per-tile binary searches)
-        DevBuf bidx;
-        const size_t bidx_bytes = (size_t)B.view.rows * (size_t)(ntiles + 1) * 4;
-        const bool use_index = ntiles > 1 && bidx_bytes <= kBlockedIndexMaxBytes && bidx_bytes < free_b / 4;
-        DevBuf tocc;
-        if (use_index) {
-          SPG_TRY(bidx.alloc(ctx, bidx_bytes));
-          SPG_TRY(tocc.alloc(ctx, (size_t)B.view.rows * (size_t)((ntiles + 31) / 32) * 4));
-          launch_build_blocked_index(B.view, ntiles, bidx.as<int32_t>(), lc);
-          launch_build_tile_occupancy(B.view.rows, bidx.as<int32_t>(), ntiles, tocc.as<uint32_t>(), lc);
-          ctx->launches += 2;
-        }
-        launch_num_tile(A.view, B.view, bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(),
-                        tile_cnt.as<int32_t>(), tile_off.as<int32_t>(), ntiles, c_rp, c_col, c_val,
-                        use_index ? bidx.as<int32_t>() : nullptr, use_index ? tocc.as<uint32_t>() : nullptr,
-                        use_list ? work.as<int64_t>() : nullptr, use_list ? nz.as<int64_t>() + nheavy : nullptr,
-                        ctx->d_counter, ctx->d_flags, lc, tune.heavy_path == 2);
-        ctx->launches += 2;
+      bool done = false;
+      if (tune.heavy_path != 0) SPG_TRY(numeric_tiles(c_rp, c_col, c_val, bidx.as<int32_t>(), free_b, &done));
+      if (!done) {
+        const int64_t room = heavy_unit_bound(nheavy, ntiles, c_nnz);
+        DevBuf units;
+        SPG_TRY(units.alloc(ctx, (size_t)room * sizeof(int4)));
+        launch_num_units(A.view, B.view, bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(),
+                         ntiles, c_rp, c_col, c_val, bidx.as<int32_t>(), bitmap.as<uint32_t>(), bitmap_stride(),
+                         units.as<int4>(), room, ctx->d_counter + 8, ctx->d_flags, lc);
+        ++ctx->launches;
       }
       ++ctx->launches;
     }
@@ -505,10 +564,10 @@ spg_status multiply_plain(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opts&
   const int64_t total = extra[0];
   if (rep) rep->products = extra[1];
   DevBuf c_col, c_val;
-  SPG_TRY(c_col.alloc(ctx, (size_t)total * 4));
-  SPG_TRY(c_val.alloc(ctx, (size_t)total * 4));
+  SPG_TRY(P.alloc_entries(total, c_col, c_val));
   tm.mark(SPG_STAGE_NUMERIC);
-  SPG_TRY(P.numeric(P.nnz.as<int64_t>(), c_col.as<int32_t>(), c_val.as<float>(), rep, P.prod.as<int64_t>()));
+  SPG_TRY(P.numeric(P.nnz.as<int64_t>(), c_col.as<int32_t>(), c_val.as<float>(), total, rep,
+                      P.prod.as<int64_t>()));
   SPG_TRY(finish_output(ctx, P, total, o, c_col, c_val, C));
   if (rep) rep->nnz_c = total;
   return SPG_OK;
@@ -640,15 +699,15 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
     }
   }
   DevBuf c_col, c_val;
-  SPG_TRY(c_col.alloc(ctx, (size_t)total * 4));
-  SPG_TRY(c_val.alloc(ctx, (size_t)total * 4));
+  SPG_TRY(P.alloc_entries(total, c_col, c_val));
   tm.mark(SPG_STAGE_COMPACT);
   launch_compact_rows(compact_list, light, need.as<uint8_t>(), slab_off.as<int64_t>(), slab_col.as<int32_t>(),
                       slab_val.as<float>(), P.nnz.as<int64_t>(), c_col.as<int32_t>(), c_val.as<float>(), lc);
   ++ctx->launches;
   if (exact_needed) {
     tm.mark(SPG_STAGE_NUMERIC);
-    SPG_TRY(P.numeric(P.nnz.as<int64_t>(), c_col.as<int32_t>(), c_val.as<float>(), rep, P.prod.as<int64_t>()));
+    SPG_TRY(P.numeric(P.nnz.as<int64_t>(), c_col.as<int32_t>(), c_val.as<float>(), total, rep,
+                      P.prod.as<int64_t>()));
   }
   SPG_TRY(finish_output(ctx, P, total, o, c_col, c_val, C));
   if (rep) rep->nnz_c = total;
@@ -794,7 +853,7 @@ spg_status multiply_reuse_device(spg_ctx* ctx, const DevMat& A, const DevMat& B,
     ++ctx->launches;
   }
   tm.mark(SPG_STAGE_NUMERIC);
-  SPG_TRY(P.numeric(P.nnz.as<int64_t>(), C->col_idx, C->val, rep));
+  SPG_TRY(P.numeric(P.nnz.as<int64_t>(), C->col_idx, C->val, C->nnz, rep));
   tm.finish(rep);
   int f = 0;
   SPG_TRY(read_flags(ctx, &f));
@@ -867,8 +926,8 @@ spg_status spg_create(spg_ctx** out, int32_t device) {
   SPG_CUDA(ctx.get(), cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &thr));
   SPG_CUDA(ctx.get(), cudaMalloc(&ctx->d_flags, 64));
   SPG_CUDA(ctx.get(), cudaMemset(ctx->d_flags, 0, 64));
-  SPG_CUDA(ctx.get(), cudaMalloc(&ctx->d_counter, 8 * sizeof(unsigned long long)));
-  SPG_CUDA(ctx.get(), cudaMemset(ctx->d_counter, 0, 8 * sizeof(unsigned long long)));
+  SPG_CUDA(ctx.get(), cudaMalloc(&ctx->d_counter, 16 * sizeof(unsigned long long)));
+  SPG_CUDA(ctx.get(), cudaMemset(ctx->d_counter, 0, 16 * sizeof(unsigned long long)));
   // mapped, so small read-backs can be written by a kernel (stage_read)
   SPG_CUDA(ctx.get(), cudaHostAlloc((void**)&ctx->h_stage, 64 * sizeof(int64_t), cudaHostAllocMapped));
   SPG_CUDA(ctx.get(), cudaHostGetDevicePointer((void**)&ctx->h_stage_dev, ctx->h_stage, 0));

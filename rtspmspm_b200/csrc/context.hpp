@@ -31,7 +31,7 @@ struct spg_ctx {
   bool mlp_loaded = false;
   // small device scratch
   int* d_flags = nullptr;
-  unsigned long long* d_counter = nullptr;  // tile queue / retry counters (4 entries)
+  unsigned long long* d_counter = nullptr;  // tile queue / retry / unit counters (16 words)
   // pinned host staging for small device->host reads
   int64_t* h_stage = nullptr;      // 64 words, mapped
   int64_t* h_stage_dev = nullptr;  // the same words seen from the device

@@ -315,7 +315,8 @@ __global__ void __launch_bounds__(512, 2) k_sym_warp(DCsr A, DCsr B, const int32
 // no particular order: f(c).  A's row is taken NTHR entries at a time; a
 // CTA-wide exclusive scan of their B-row lengths goes to shared memory
 // (sh_excl[NTHR + 1], sh_bs[NTHR]) and the chunk's product stream is split
-// evenly among the warps.  A warp walks its share 32 products per step: a
+// evenly among the warps.  In its share a warp takes pieces of 32 or more
+// products of one segment with four loads a lane in flight; for shorter ones a
 // window of the next 32 segment starts (one shared load per lane) and a
 // shuffle search give each lane its segment, so hub rows of B are spread
 // over every warp and short rows leave no lane idle.
@@ -363,16 +364,28 @@ __device__ __forceinline__ void cta_for_each_product(const DCsr& A, const DCsr& 
       }
       int kc = i0;
       for (Off pos = lo; pos < hi;) {
+        // a long piece of segment kc: whole-warp loads, four a lane at once
+        const Off seg0 = sh_excl[kc], seg_end = min(sh_excl[kc + 1], hi);
+        if (seg_end - pos >= 32) {
+          const int32_t* src = B.col + sh_bs[kc] + (pos - seg0);
+          const int n = (int)(seg_end - pos);
+          for (int q0 = 0; q0 < n; q0 += 4 * 32) {
+            int32_t c[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int q = q0 + u * 32 + lane;
+              c[u] = q < n ? src[q] : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (c[u] >= 0) f(c[u]);
+          }
+          pos = seg_end;
+          continue;
+        }
         // starts of the segments after kc, kc + 1, ..., kc + 31
         const int wi = kc + 1 + lane;
         const Off nxt = wi <= cnt ? sh_excl[wi] : (Off)(R32 ? 0x7fffffff : INT64_MAX);
-        // the next 32 products all inside segment kc (long rows of B): no search
-        const Off seg_end = __shfl_sync(kFull, nxt, 0);
-        if (pos >= sh_excl[kc] && pos + 32 <= seg_end && pos + 32 <= hi) {
-          f(B.col[sh_bs[kc] + (pos - sh_excl[kc]) + (Off)lane]);
-          pos += 32;
-          continue;
-        }
         const Off wend = __shfl_sync(kFull, nxt, 31);
         if (wend <= pos) {
           // more than 31 empty segments in a row: slide the window on
@@ -441,13 +454,13 @@ __global__ void __launch_bounds__(kSymBlockThreads) k_sym_block(DCsr A, DCsr B, 
 
 // One CTA per row; a bitmap over the row's column span in shared memory
 // (windows of `max_words` 32-bit words, a multiple of one tile).  Records
-// the per-tile counts for the heavy numeric pass.
-constexpr int kSymDenseThreads = 1024;
-template <bool R32>
-__global__ void __launch_bounds__(kSymDenseThreads) k_sym_dense(DCsr A, DCsr B, const int32_t* rows, int64_t nrows,
+// the per-tile counts for the heavy numeric pass and, when `bitmap` is given,
+// the tiles of the span there (ntiles * kTileWords words a slot).
+template <bool R32, int kSymDenseThreads>
+__global__ void __launch_bounds__(kSymDenseThreads, 2048 / kSymDenseThreads) k_sym_dense(DCsr A, DCsr B, const int32_t* rows, int64_t nrows,
                                                                 int max_words, int64_t slot_base, int64_t* nnz_out,
                                                                 int32_t* big_slot, int32_t* tile_cnt, int ntiles,
-                                                                int* flags) {
+                                                                uint32_t* bitmap, int* flags) {
   using Off = typename RowOff<R32>::T;
   extern __shared__ uint32_t sm_bits[];
   __shared__ Off sh_excl[kSymDenseThreads + 1], sh_bs[kSymDenseThreads], sh_wsum[kSymDenseThreads / 32 + 1];
@@ -484,16 +497,22 @@ __global__ void __launch_bounds__(kSymDenseThreads) k_sym_dense(DCsr A, DCsr B, 
     const int64_t wcols = (int64_t)max_words * 32;
     for (int64_t w0 = span_lo; w0 <= span_hi; w0 += wcols) {
       const int64_t w1 = min(w0 + wcols, (int64_t)span_hi + 1);
+      const uint32_t wspan = (uint32_t)(w1 - w0);
       const int nwords = (int)((w1 - w0 + 31) >> 5);
       const int nwords_tiles = ((nwords + kTileWords - 1) / kTileWords) * kTileWords;
       for (int t = threadIdx.x; t < nwords_tiles; t += blockDim.x) sm_bits[t] = 0u;
       __syncthreads();
       cta_for_each_product<kSymDenseThreads, R32>(A, B, row, sh_excl, sh_bs, sh_wsum, [&](int32_t c) {
-        if (c >= w0 && c < w1) {
-          const int off = (int)(c - w0);
-          atomicOr(&sm_bits[off >> 5], 1u << (off & 31));
+        const uint32_t off = (uint32_t)(c - (int32_t)w0);
+        if (off < wspan) {
+          const uint32_t bit = 1u << (off & 31);
+          if (!(sm_bits[off >> 5] & bit)) atomicOr(&sm_bits[off >> 5], bit);
         }
       });
+      if (bitmap) {
+        uint32_t* bm = bitmap + (slot_base + idx) * ((int64_t)ntiles * kTileWords) + (w0 >> 5);
+        for (int t = threadIdx.x; t < nwords_tiles; t += blockDim.x) bm[t] = sm_bits[t];
+      }
       // per-tile popcounts: one warp per tile
       const int ntile_w = nwords_tiles / kTileWords;
       for (int tw = w; tw < ntile_w; tw += nwarps) {
@@ -1068,9 +1087,9 @@ __device__ __forceinline__ bool tile_segment_bulk(const DCsr& B, Off bs, int len
 // warp, runs of short ones packed.  Accumulator: a dense tile of floats plus
 // an occupancy bitmap, emitted in column order with coalesced stores and
 // cleared as it is read.
-// BULK: long segments through tile_segment_bulk (kBulkWarpWords more words
-// of shared memory per warp, after the tile accumulators).
-template <bool R32, bool BULK>
+// Long segments go through tile_segment_bulk (kBulkWarpWords more words of
+// shared memory per warp, after the tile accumulators).
+template <bool R32>
 __global__ void __launch_bounds__(kTileWarps * 32) k_num_tile(DCsr A, DCsr B, const int32_t* heavy_rows, int64_t nheavy,
                                                         const int32_t* big_slot, const int32_t* tile_cnt,
                                                         const int32_t* tile_off, int ntiles, const int64_t* c_rp,
@@ -1089,7 +1108,7 @@ __global__ void __launch_bounds__(kTileWarps * 32) k_num_tile(DCsr A, DCsr B, co
   float* st_val = reinterpret_cast<float*>(st_col + kBulkPiece);
   const uint32_t mbar = smem_u32(st_col + 2 * kBulkPiece);
   uint32_t phase = 0;
-  if (BULK && lane == 0) mbar_init(mbar);
+  if (lane == 0) mbar_init(mbar);
   for (int s = lane; s < kTileCols; s += 32) acc[s] = 0.f;
   for (int s = lane; s < kTileWords; s += 32) bits[s] = 0u;
   __syncwarp();
@@ -1158,7 +1177,7 @@ __global__ void __launch_bounds__(kTileWarps * 32) k_num_tile(DCsr A, DCsr B, co
           const Off sbs = __shfl_sync(kFull, bs, idx);
           const int sl = __shfl_sync(kFull, len, idx);
           const float sa = __shfl_sync(kFull, a, idx);
-          if (BULK && sl >= kBulkMin) {
+          if (sl >= kBulkMin) {
             if (!tile_segment_bulk(B, sbs, sl, sa, c0, acc, bits, st_col, st_val, mbar, phase, flags)) return;
           } else {
             tile_segment(B, sbs, sl, sa, c0, acc, bits, flags);
@@ -1550,24 +1569,40 @@ void launch_sym_block(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t
   else sym_block_one<false>(A, B, rows, nrows, log_table, slot_base, nnz, big_slot, tile_cnt, ntiles, flags, lc);
 }
 
-template <bool R32>
+template <bool R32, int THREADS>
 static void sym_dense_one(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, int64_t slot_base,
-                          int64_t* nnz, int32_t* big_slot, int32_t* tile_cnt, int ntiles, int* flags,
-                          const LaunchCtx& lc) {
-  const int max_words = kDenseWindowWords;
+                          int64_t* nnz, int32_t* big_slot, int32_t* tile_cnt, int ntiles, uint32_t* bitmap, int* flags,
+                          int max_words, const LaunchCtx& lc) {
+  auto kernel = k_sym_dense<R32, THREADS>;
   const size_t smem = (size_t)max_words * sizeof(uint32_t);
-  cudaFuncSetAttribute(k_sym_dense<R32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const int blocks = (int)std::min<int64_t>(nrows, (int64_t)lc.sms);
-  k_sym_dense<R32><<<blocks, kSymDenseThreads, smem, lc.stream>>>(A, B, rows, nrows, max_words, slot_base, nnz, big_slot,
-                                                      tile_cnt, ntiles, flags);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, smem);
+  const int blocks = (int)std::min<int64_t>(nrows, (int64_t)lc.sms * std::max(1, per_sm));
+  kernel<<<blocks, THREADS, smem, lc.stream>>>(A, B, rows, nrows, max_words, slot_base, nnz, big_slot, tile_cnt, ntiles,
+                                               bitmap, flags);
 }
 
 void launch_sym_dense(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, int64_t slot_base,
-                      int64_t* nnz, int32_t* big_slot, int32_t* tile_cnt, int ntiles, int* flags,
+                      int64_t* nnz, int32_t* big_slot, int32_t* tile_cnt, int ntiles, uint32_t* bitmap, int* flags,
                       const LaunchCtx& lc) {
   if (nrows == 0) return;
-  if (B.rp32) sym_dense_one<true>(A, B, rows, nrows, slot_base, nnz, big_slot, tile_cnt, ntiles, flags, lc);
-  else sym_dense_one<false>(A, B, rows, nrows, slot_base, nnz, big_slot, tile_cnt, ntiles, flags, lc);
+  // no more bitmap than the columns need.  While four bitmaps fit an SM
+  // (393,216 columns, 48 KB each) rows go to 512-thread CTAs, whose barriers
+  // cost less (R-MAT 17: 1,024 threads 3.25 ms, 512 2.65, 256 3.43); beyond,
+  // 1,024 threads keep the SM's warps
+  const int max_words = (int)std::min<int64_t>(kDenseWindowWords, (int64_t)ntiles * kTileWords);
+#define SPG_SD(R, T) \
+  sym_dense_one<R, T>(A, B, rows, nrows, slot_base, nnz, big_slot, tile_cnt, ntiles, bitmap, flags, max_words, lc)
+  const bool narrow = max_words <= 12288;
+  if (B.rp32) {
+    if (narrow) SPG_SD(true, 512);
+    else SPG_SD(true, 1024);
+  } else {
+    if (narrow) SPG_SD(false, 512);
+    else SPG_SD(false, 1024);
+  }
+#undef SPG_SD
 }
 
 template <int LOGT, bool R32>
@@ -1760,46 +1795,42 @@ void launch_build_blocked_index(const DCsr& B, int ntiles, int32_t* bidx, const 
   k_build_blocked_index<<<grid_for(B.rows, 256, 32, lc.sms * 16), 256, 0, lc.stream>>>(B, ntiles, bidx);
 }
 
-template <bool R32, bool BULK>
+template <bool R32>
 static void num_tile_one(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, int64_t nheavy,
                          const int32_t* big_slot, const int32_t* tile_cnt, const int32_t* tile_off, int ntiles,
                          const int64_t* c_rp, int32_t* c_col, float* c_val, const int32_t* bidx,
                          const uint32_t* tocc, const int64_t* work, const int64_t* nwork,
                          unsigned long long* tile_counter, int* flags, const LaunchCtx& lc) {
-  const size_t smem = (size_t)kTileWarps * (kTileWarpWords + (BULK ? kBulkWarpWords : 0)) * 4;
+  const size_t smem = (size_t)kTileWarps * (kTileWarpWords + kBulkWarpWords) * 4;
   const int twords = (ntiles + 31) / 32;
-  cudaFuncSetAttribute(k_num_tile<R32, BULK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k_num_tile<R32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_num_tile<R32, BULK>, kTileWarps * 32, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_num_tile<R32>, kTileWarps * 32, smem);
   if (per_sm < 1) per_sm = 1;
   const int64_t tiles = nheavy * (int64_t)ntiles;
   const int blocks = (int)std::min<int64_t>((tiles + kTileWarps - 1) / kTileWarps, (int64_t)lc.sms * per_sm);
   cudaMemsetAsync(tile_counter, 0, sizeof(unsigned long long), lc.stream);
-  k_num_tile<R32, BULK><<<blocks, kTileWarps * 32, smem, lc.stream>>>(A, B, heavy_rows, nheavy, big_slot, tile_cnt,
+  k_num_tile<R32><<<blocks, kTileWarps * 32, smem, lc.stream>>>(A, B, heavy_rows, nheavy, big_slot, tile_cnt,
                                                                       tile_off, ntiles, c_rp, c_col, c_val, bidx,
                                                                       tocc, twords, work, nwork, tile_counter,
                                                                       flags);
 }
 
+bool bulk_aligned(const DCsr& B) {
+  return ((reinterpret_cast<uintptr_t>(B.col) | reinterpret_cast<uintptr_t>(B.val)) & 15u) == 0;
+}
+
 void launch_num_tile(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, int64_t nheavy, const int32_t* big_slot,
                      const int32_t* tile_cnt, const int32_t* tile_off, int ntiles, const int64_t* c_rp,
                      int32_t* c_col, float* c_val, const int32_t* bidx, const uint32_t* tocc, const int64_t* work,
-                     const int64_t* nwork, unsigned long long* tile_counter, int* flags, const LaunchCtx& lc,
-                     bool bulk) {
+                     const int64_t* nwork, unsigned long long* tile_counter, int* flags, const LaunchCtx& lc) {
   if (nheavy == 0) return;
-  // the bulk copies need 16-byte aligned column and value arrays
-  bulk = bulk && ((reinterpret_cast<uintptr_t>(B.col) | reinterpret_cast<uintptr_t>(B.val)) & 15u) == 0;
-#define SPG_NT(R, K)                                                                                          \
-  num_tile_one<R, K>(A, B, heavy_rows, nheavy, big_slot, tile_cnt, tile_off, ntiles, c_rp, c_col, c_val, bidx, \
-                     tocc, work, nwork, tile_counter, flags, lc)
-  if (B.rp32) {
-    if (bulk) SPG_NT(true, true);
-    else SPG_NT(true, false);
-  } else {
-    if (bulk) SPG_NT(false, true);
-    else SPG_NT(false, false);
-  }
-#undef SPG_NT
+  if (B.rp32)
+    num_tile_one<true>(A, B, heavy_rows, nheavy, big_slot, tile_cnt, tile_off, ntiles, c_rp, c_col, c_val, bidx, tocc,
+                       work, nwork, tile_counter, flags, lc);
+  else
+    num_tile_one<false>(A, B, heavy_rows, nheavy, big_slot, tile_cnt, tile_off, ntiles, c_rp, c_col, c_val, bidx, tocc,
+                        work, nwork, tile_counter, flags, lc);
 }
 
 void launch_build_tile_occupancy(int64_t rows, const int32_t* bidx, int ntiles, uint32_t* tocc, const LaunchCtx& lc) {

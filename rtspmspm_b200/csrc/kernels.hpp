@@ -36,6 +36,18 @@ constexpr int kBinLearned = 2;
 // many CTAs per SM as fit.
 constexpr int kTileWarpBytes = ((1 << SPG_TILE_SHIFT) + (1 << SPG_TILE_SHIFT) / 32 + 32) * 4;
 constexpr int kTileWarps = (227 * 1024) / kTileWarpBytes > 8 ? 8 : (227 * 1024) / kTileWarpBytes;
+// Heavy-row units (heavy_unit.cu): threads and 32-bit words of shared memory
+// a CTA, and the words a unit's rank words and entries may take (a spare word
+// behind them).
+#ifndef SPG_UNIT_WORDS
+#define SPG_UNIT_WORDS 5600
+#endif
+#ifndef SPG_UNIT_THREADS
+#define SPG_UNIT_THREADS 128
+#endif
+constexpr int kUnitThreads = SPG_UNIT_THREADS;
+constexpr int kUnitWords = SPG_UNIT_WORDS;
+constexpr int kUnitCost = kUnitWords - 4;
 constexpr int kDenseWindowWords = 40960;   // 1,310,720 columns of bitmap per window
 
 struct BinParams {
@@ -102,7 +114,7 @@ void launch_sym_block(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t
                       int64_t slot_base, int64_t* nnz, int32_t* big_slot, int32_t* tile_cnt, int ntiles, int* flags,
                       const LaunchCtx& lc);
 void launch_sym_dense(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, int64_t slot_base,
-                      int64_t* nnz, int32_t* big_slot, int32_t* tile_cnt, int ntiles, int* flags,
+                      int64_t* nnz, int32_t* big_slot, int32_t* tile_cnt, int ntiles, uint32_t* bitmap, int* flags,
                       const LaunchCtx& lc);
 // Default smallest product count of an expand-sort-fold row.
 constexpr int kEscMinProd = 128;
@@ -149,16 +161,27 @@ void launch_tile_worklist(const int32_t* heavy_rows, int64_t nheavy, const int32
 void launch_build_blocked_index(const DCsr& B, int ntiles, int32_t* bidx, const LaunchCtx& lc);
 // Tile occupancy bits of B from its blocked index (ceil(ntiles / 32) words per row).
 void launch_build_tile_occupancy(int64_t rows, const int32_t* bidx, int ntiles, uint32_t* tocc, const LaunchCtx& lc);
-// bidx: blocked index of B (launch_build_blocked_index) or null (binary
-// searches); tocc: its occupancy bits or null; work/nwork: the list of
-// non-empty tiles (launch_tile_worklist) and its length on the device, or
-// null (every tile is visited); bulk: segments of 64+ entries staged into
-// shared memory by bulk copies (when B's arrays are 16-byte aligned)
+// B's arrays take bulk copies (16-byte aligned).
+bool bulk_aligned(const DCsr& B);
+// Tiles by themselves, segments of 64+ entries staged into shared memory by
+// bulk copies (bulk_aligned(B) only).  bidx: blocked index of B
+// (launch_build_blocked_index) or null (binary searches); tocc: its occupancy
+// bits or null; work/nwork: the list of non-empty tiles (launch_tile_worklist)
+// and its length on the device, or null (every tile is visited)
 void launch_num_tile(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, int64_t nheavy, const int32_t* big_slot,
                      const int32_t* tile_cnt, const int32_t* tile_off, int ntiles, const int64_t* c_rp,
                      int32_t* c_col, float* c_val, const int32_t* bidx, const uint32_t* tocc, const int64_t* work,
-                     const int64_t* nwork, unsigned long long* tile_counter, int* flags, const LaunchCtx& lc,
-                     bool bulk = false);
+                     const int64_t* nwork, unsigned long long* tile_counter, int* flags, const LaunchCtx& lc);
+// Heavy rows as units of consecutive column tiles (heavy_unit.cu).  `units`
+// holds room = heavy_unit_bound(nheavy, ntiles, entries of those rows);
+// bidx as above; bitmap: the rows' column bitmaps at big_slot * stride words
+// (from launch_sym_dense), or null (each unit finds its columns itself);
+// counters: three device words.
+int64_t heavy_unit_bound(int64_t nheavy, int ntiles, int64_t entries);
+void launch_num_units(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, int64_t nheavy, const int32_t* big_slot,
+                      const int32_t* tile_cnt, int ntiles, const int64_t* c_rp, int32_t* c_col, float* c_val,
+                      const int32_t* bidx, const uint32_t* bitmap, int64_t stride, int4* units, int64_t room,
+                      unsigned long long* counters, int* flags, const LaunchCtx& lc);
 void launch_compact_rows(const int32_t* rows, int64_t nrows, const uint8_t* need_exact, const int64_t* slab_off,
                          const int32_t* slab_col, const float* slab_val, const int64_t* c_rp, int32_t* c_col,
                          float* c_val, const LaunchCtx& lc);
