@@ -19,39 +19,51 @@
 namespace spg {
 namespace {
 
-constexpr int kSortThreads = 256;
+constexpr int kSortThreads = 512;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 8;                        // per lane
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 entries per CTA
+constexpr int kSortItems = 8;                         // per lane
+constexpr int kSortTile = kSortThreads * kSortItems;  // entries per CTA
 constexpr int kDigits = 256;
+static_assert(kSortThreads >= kDigits, "a thread per digit");
 constexpr int kScatterSmem = kSortTile * (8 + 4);  // the tile's keys and values in digit order
 
-__global__ void k_coo_keys(const int32_t* ri, const int32_t* ci, int64_t n, int64_t rows, int64_t cols, uint64_t* key,
-                           int* flags) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t r = ri[i], c = ci[i];
-    if (r < 0 || r >= rows || c < 0 || c >= cols) {
-      atomicOr(flags, kFlagBadIndex);
-      key[i] = 0;
-    } else {
-      key[i] = ((uint64_t)(uint32_t)r << 32) | (uint32_t)c;
-    }
+// Where a sort pass reads its entries: the first one from the COO arrays
+// (entries outside the matrix get key 0 and raise a flag in the counting
+// kernel), the others from the previous pass.
+struct CooIn {
+  const int32_t* ri;
+  const int32_t* ci;
+  int64_t rows, cols;
+  int* flags;
+  const uint64_t* key;
+  const float* val;
+};
+
+template <bool FIRST>
+__device__ __forceinline__ uint64_t entry_key(const CooIn& in, int64_t i, bool check) {
+  if (!FIRST) return in.key[i];
+  const int32_t r = in.ri[i], c = in.ci[i];
+  if (r < 0 || r >= in.rows || c < 0 || c >= in.cols) {
+    if (check) atomicOr(in.flags, kFlagBadIndex);
+    return 0;
   }
+  return ((uint64_t)(uint32_t)r << 32) | (uint32_t)c;
 }
 
 // Digit counts of each tile: hist[d * ntiles + tile].
-__global__ void __launch_bounds__(kSortThreads) k_radix_hist(const uint64_t* key, int64_t n, int shift, int64_t ntiles,
+template <bool FIRST>
+__global__ void __launch_bounds__(kSortThreads) k_radix_hist(CooIn in, int64_t n, int shift, int64_t ntiles,
                                                              int64_t* hist) {
   __shared__ int cnt[kDigits];
-  cnt[threadIdx.x] = 0;
+  if (threadIdx.x < kDigits) cnt[threadIdx.x] = 0;
   __syncthreads();
   const int64_t t0 = blockIdx.x * (int64_t)kSortTile;
   for (int q = threadIdx.x; q < kSortTile; q += kSortThreads) {
     const int64_t i = t0 + q;
-    if (i < n) atomicAdd(&cnt[(int)((key[i] >> shift) & 0xffu)], 1);
+    if (i < n) atomicAdd(&cnt[(int)((entry_key<FIRST>(in, i, true) >> shift) & 0xffu)], 1);
   }
   __syncthreads();
-  hist[(int64_t)threadIdx.x * ntiles + blockIdx.x] = cnt[threadIdx.x];
+  if (threadIdx.x < kDigits) hist[(int64_t)threadIdx.x * ntiles + blockIdx.x] = cnt[threadIdx.x];
 }
 
 // Stable scatter of one tile: warp w owns entries [w * 32 * kSortItems, (w + 1) * 32 * kSortItems)
@@ -61,12 +73,21 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const uint64_t* key
 // lp = the digit's first position in the tile + the counts of earlier warps
 // + the entry's rank), then written out by consecutive threads, so each
 // digit's run of the tile goes to consecutive global positions (coalesced
-// stores; scattering straight from registers ran at 1.1 TB/s).  off:
+// stores; scattering straight from registers ran at 1.1 TB/s).
+//
+// Bound: __match_any_sync, whose time grows with the distinct digits of a warp
+// (2^23 entries: 98 us a pass of 8-bit digits, 66 us of 4-bit ones; the 24
+// bytes an entry moves take 31 us at the copy peak).  So it runs once an
+// entry, the rank kept in a register (143 -> 98 us against matching again for
+// the positions); eight ballots in its place were slower (153 us with two
+// rounds).  512 threads a tile: 256 took as long here but made twice the tiles
+// to count and scan (2^26 entries: 6.5 against 6.0 ms a call), 1,024 and 16
+// entries a lane were slower.  off:
 // exclusive scan of hist (digit-major), the first output position of each
 // (digit, tile).  Dynamic shared memory: kSortTile keys and values.
-__global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const uint64_t* kin, const float* vin, int64_t n,
-                                                                int shift, int64_t ntiles, const int64_t* off,
-                                                                uint64_t* kout, float* vout) {
+template <bool FIRST>
+__global__ void __launch_bounds__(kSortThreads) k_radix_scatter(CooIn in, int64_t n, int shift, int64_t ntiles,
+                                                                const int64_t* off, uint64_t* kout, float* vout) {
   __shared__ int base[kSortWarps][kDigits];
   __shared__ int first[kDigits];  // the digit's first position in the tile's digit order
   extern __shared__ uint64_t sm_sort[];
@@ -83,57 +104,59 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const uint64_t* 
 #pragma unroll
   for (int j = 0; j < kSortItems; ++j) {
     const int64_t i = w0 + j * 32 + lane;
-    k[j] = i < n ? kin[i] : 0;
-    v[j] = i < n ? vin[i] : 0.f;
+    k[j] = i < n ? entry_key<FIRST>(in, i, false) : 0;
+    v[j] = i < n ? in.val[i] : 0.f;
   }
-  // the warp's count per digit
+  // the warp's count per digit and, from the counts so far, each entry's rank
+  // among the warp's entries of its digit
+  int rank[kSortItems];
 #pragma unroll
   for (int j = 0; j < kSortItems; ++j) {
     const bool act = w0 + j * 32 + lane < n;
     const int d = act ? (int)((k[j] >> shift) & 0xffu) : kDigits + lane;
     const unsigned grp = __match_any_sync(kFull, d);
-    if (act && (grp & lt) == 0u) base[w][d] += __popc(grp);
+    const int before = act ? base[w][d] : 0;
+    rank[j] = before + __popc(grp & lt);
+    __syncwarp();
+    if (act && (grp & lt) == 0u) base[w][d] = before + __popc(grp);
     __syncwarp();
   }
   __syncthreads();
   // per digit: its total in the tile and, per warp, the start of the warp's entries
   {
+    constexpr int kDigitWarps = kDigits / 32;
+    __shared__ int wtot[kDigitWarps];
     const int d = threadIdx.x;
-    int run = 0;
+    int run = 0, incl = 0;
+    if (d < kDigits) {
 #pragma unroll
-    for (int x = 0; x < kSortWarps; ++x) {
-      const int c = base[x][d];
-      base[x][d] = run;
-      run += c;
+      for (int x = 0; x < kSortWarps; ++x) {
+        const int c = base[x][d];
+        base[x][d] = run;
+        run += c;
+      }
+      // exclusive scan of the digit totals across the CTA (digit d = thread d)
+      incl = warp_incl_scan(run);
+      if (lane == 31) wtot[w] = incl;
     }
-    // exclusive scan of the digit totals across the CTA (digit d = thread d)
-    const int incl = warp_incl_scan(run);
-    __shared__ int wtot[kSortWarps];
-    if (lane == 31) wtot[w] = incl;
     __syncthreads();
-    int pre = 0;
+    if (d < kDigits) {
+      int pre = incl - run;
 #pragma unroll
-    for (int x = 0; x < kSortWarps; ++x) pre += x < w ? wtot[x] : 0;
-    first[d] = pre + incl - run;
+      for (int x = 0; x < kDigitWarps; ++x) pre += x < w ? wtot[x] : 0;
+      first[d] = pre;
+#pragma unroll
+      for (int x = 0; x < kSortWarps; ++x) base[x][d] += pre;
+    }
   }
-  __syncthreads();
-  for (int d = threadIdx.x; d < kDigits; d += kSortThreads)
-    for (int x = 0; x < kSortWarps; ++x) base[x][d] += first[d];
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < kSortItems; ++j) {
-    const bool act = w0 + j * 32 + lane < n;
-    const int d = act ? (int)((k[j] >> shift) & 0xffu) : kDigits + lane;
-    const unsigned grp = __match_any_sync(kFull, d);
-    int lp = 0;
-    if (act) lp = base[w][d] + __popc(grp & lt);
-    __syncwarp();
-    if (act) {
+    if (w0 + j * 32 + lane < n) {
+      const int lp = base[w][(int)((k[j] >> shift) & 0xffu)] + rank[j];
       sk[lp] = k[j];
       sv[lp] = v[j];
-      if ((grp & lt) == 0u) base[w][d] += __popc(grp);
     }
-    __syncwarp();
   }
   __syncthreads();
   // the tile in digit order, written by consecutive threads
@@ -147,35 +170,72 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const uint64_t* 
   }
 }
 
-// head[i] = 1 where entry i starts a run of equal keys.
-__global__ void k_run_heads(const uint64_t* key, int64_t n, int64_t* head) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    head[i] = (i == 0 || key[i] != key[i - 1]) ? 1 : 0;
-}
+// Entries of each fold tile that start a run of equal keys.
+constexpr int kFoldThreads = 512;
+constexpr int kFoldItems = 4;  // per lane, 32 consecutive at a time
+constexpr int kFoldTile = kFoldThreads * kFoldItems;
 
-// One thread per run: its column and the left fold of its values into
-// output entry pos[i]; the entry's row into urow.
-__global__ void k_fold_runs(const uint64_t* key, const float* val, int64_t n, const int64_t* pos, int32_t* col,
-                            float* out_val, int32_t* urow) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = key[i];
-    if (i > 0 && key[i - 1] == k) continue;
-    float s = val[i];
-    for (int64_t q = i + 1; q < n && key[q] == k; ++q) s = __fadd_rn(s, val[q]);
-    const int64_t u = pos[i];
-    col[u] = (int32_t)(uint32_t)(k & 0xffffffffu);
-    out_val[u] = s;
-    urow[u] = (int32_t)(k >> 32);
+__device__ __forceinline__ bool run_head(const uint64_t* key, int64_t i, uint64_t k) { return i == 0 || key[i - 1] != k; }
+
+__global__ void __launch_bounds__(kFoldThreads) k_count_runs(const uint64_t* key, int64_t n, int64_t* runs) {
+  __shared__ int cnt[kFoldThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i0 = blockIdx.x * (int64_t)kFoldTile + w * (32 * kFoldItems) + lane;
+  int c = 0;
+#pragma unroll
+  for (int j = 0; j < kFoldItems; ++j) {
+    const int64_t i = i0 + j * 32;
+    c += i < n && run_head(key, i, key[i]);
+  }
+  c = __reduce_add_sync(kFull, c);
+  if (lane == 0) cnt[w] = c;
+  __syncthreads();
+  if (w == 0) {
+    c = __reduce_add_sync(kFull, lane < kFoldThreads / 32 ? cnt[lane] : 0);
+    if (lane == 0) runs[blockIdx.x] = c;
   }
 }
 
-// Row pointers from the rows of the m sorted unique entries: entry u opens
-// rows (urow[u - 1], urow[u]]; the rows after the last entry end at m.
-__global__ void k_rp_from_rows(const int32_t* urow, int64_t m, int64_t rows, int64_t* rp) {
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u <= m; u += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t prev = u == 0 ? -1 : (int64_t)urow[u - 1];
-    const int64_t cur = u == m ? rows : (int64_t)urow[u];
-    for (int64_t r = prev + 1; r <= cur; ++r) rp[r] = u;
+// One thread per run: its column and the left fold of its values into the
+// run's output entry (base[tile] = runs before the tile), and the row pointers
+// its entry opens: those of the rows after the row before it, up to its own.
+// The last entry also closes the rows behind it.
+__global__ void __launch_bounds__(kFoldThreads) k_fold_runs(const uint64_t* key, const float* val, int64_t n,
+                                                            const int64_t* base, int64_t m, int64_t rows,
+                                                            int32_t* col, float* out_val, int64_t* rp) {
+  __shared__ int cnt[kFoldThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i0 = blockIdx.x * (int64_t)kFoldTile + w * (32 * kFoldItems) + lane;
+  uint64_t k[kFoldItems];
+  unsigned heads[kFoldItems];
+  int c = 0;
+#pragma unroll
+  for (int j = 0; j < kFoldItems; ++j) {
+    const int64_t i = i0 + j * 32;
+    k[j] = i < n ? key[i] : 0;
+    heads[j] = __ballot_sync(kFull, i < n && run_head(key, i, k[j]));
+    c += __popc(heads[j]);
+  }
+  if (lane == 0) cnt[w] = c;
+  __syncthreads();
+  int64_t u0 = base[blockIdx.x];
+  for (int x = 0; x < w; ++x) u0 += cnt[x];
+#pragma unroll
+  for (int j = 0; j < kFoldItems; ++j) {
+    const int64_t i = i0 + j * 32;
+    if ((heads[j] >> lane) & 1u) {
+      const int64_t u = u0 + __popc(heads[j] & ((1u << lane) - 1u));
+      float s = val[i];
+      int64_t q = i + 1;
+      for (; q < n && key[q] == k[j]; ++q) s = __fadd_rn(s, val[q]);
+      col[u] = (int32_t)(uint32_t)(k[j] & 0xffffffffu);
+      out_val[u] = s;
+      const int64_t r = (int64_t)(k[j] >> 32);
+      for (int64_t x = i == 0 ? 0 : (int64_t)(key[i - 1] >> 32) + 1; x <= r; ++x) rp[x] = u;
+      if (q == n)
+        for (int64_t x = r + 1; x <= rows; ++x) rp[x] = m;
+    }
+    u0 += __popc(heads[j]);
   }
 }
 
@@ -184,8 +244,6 @@ int bits_for(int64_t n) {
   while (b < 62 && ((int64_t)1 << b) < n) ++b;
   return b;
 }
-
-int blocks_for(int64_t n, int sms) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sms * 8)); }
 
 }  // namespace
 
@@ -198,41 +256,47 @@ spg_status coo_to_csr_device(spg_ctx* ctx, int64_t rows, int64_t cols, int64_t n
   SPG_TRY(k1.alloc(ctx, (size_t)std::max<int64_t>(n, 1) * 8));
   SPG_TRY(v0.alloc(ctx, (size_t)std::max<int64_t>(n, 1) * 4));
   SPG_TRY(v1.alloc(ctx, (size_t)std::max<int64_t>(n, 1) * 4));
-  if (n > 0) {
-    k_coo_keys<<<blocks_for(n, lc.sms), 256, 0, lc.stream>>>(ri, ci, n, rows, cols, k0.as<uint64_t>(), ctx->d_flags);
-    SPG_CUDA(ctx, cudaMemcpyAsync(v0.get(), vi, (size_t)n * 4, cudaMemcpyDeviceToDevice, ctx->stream));
-  }
   // LSD passes over the column bits, then over the row bits
   const int cbits = bits_for(cols), rbits = bits_for(rows);
   const int64_t ntiles = (n + kSortTile - 1) / kSortTile;
   DevBuf hist, tmp;
   SPG_TRY(hist.alloc(ctx, (size_t)std::max<int64_t>(kDigits * ntiles + 1, 1) * 8));
-  SPG_TRY(tmp.alloc(ctx, (size_t)scan_temp_elems(std::max<int64_t>(kDigits * ntiles, n) + 1) * 8));
-  uint64_t* kin = k0.as<uint64_t>();
-  uint64_t* kout = k1.as<uint64_t>();
-  float* vin = v0.as<float>();
-  float* vout = v1.as<float>();
+  SPG_TRY(tmp.alloc(ctx, (size_t)scan_temp_elems(kDigits * ntiles + 1) * 8));
   std::vector<int> shifts;
   for (int s = 0; s < cbits; s += 8) shifts.push_back(s);
   for (int s = 0; s < rbits; s += 8) shifts.push_back(32 + s);
-  if (n > 1) {
-    SPG_CUDA(ctx, cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kScatterSmem));
-    for (int shift : shifts) {
-      k_radix_hist<<<(unsigned)ntiles, kSortThreads, 0, lc.stream>>>(kin, n, shift, ntiles, hist.as<int64_t>());
+  if (shifts.empty()) shifts.push_back(0);  // a 1 x 1 matrix: the pass checks the entries and makes their keys
+  CooIn in{ri, ci, rows, cols, ctx->d_flags, nullptr, vi};
+  const uint64_t* kin = nullptr;  // the sorted entries
+  const float* vin = nullptr;
+  if (n > 0) {
+    uint64_t* kout = k0.as<uint64_t>();
+    float* vout = v0.as<float>();
+    auto pass = [&](auto hist_kernel, auto scatter_kernel, int shift) -> spg_status {
+      SPG_CUDA(ctx, cudaFuncSetAttribute(scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kScatterSmem));
+      hist_kernel<<<(unsigned)ntiles, kSortThreads, 0, lc.stream>>>(in, n, shift, ntiles, hist.as<int64_t>());
       launch_excl_scan(hist.as<int64_t>(), kDigits * ntiles, hist.as<int64_t>(), tmp.as<int64_t>(), lc);
-      k_radix_scatter<<<(unsigned)ntiles, kSortThreads, kScatterSmem, lc.stream>>>(kin, vin, n, shift, ntiles,
-                                                                        hist.as<int64_t>(), kout, vout);
-      std::swap(kin, kout);
-      std::swap(vin, vout);
+      scatter_kernel<<<(unsigned)ntiles, kSortThreads, kScatterSmem, lc.stream>>>(in, n, shift, ntiles,
+                                                                                  hist.as<int64_t>(), kout, vout);
+      in.key = kin = kout;
+      in.val = vin = vout;
+      kout = kin == k0.as<uint64_t>() ? k1.as<uint64_t>() : k0.as<uint64_t>();
+      vout = vin == v0.as<float>() ? v1.as<float>() : v0.as<float>();
+      return SPG_OK;
+    };
+    for (size_t i = 0; i < shifts.size(); ++i) {
+      if (i == 0) SPG_TRY(pass(k_radix_hist<true>, k_radix_scatter<true>, shifts[i]));
+      else SPG_TRY(pass(k_radix_hist<false>, k_radix_scatter<false>, shifts[i]));
     }
   }
   // runs of equal keys -> unique entries
-  DevBuf pos;
-  SPG_TRY(pos.alloc(ctx, (size_t)(n + 1) * 8));
-  if (n > 0) k_run_heads<<<blocks_for(n, lc.sms), 256, 0, lc.stream>>>(kin, n, pos.as<int64_t>());
-  launch_excl_scan(pos.as<int64_t>(), n, pos.as<int64_t>(), tmp.as<int64_t>(), lc);
+  const int64_t nfold = (n + kFoldTile - 1) / kFoldTile;
+  DevBuf runs;
+  SPG_TRY(runs.alloc(ctx, (size_t)(nfold + 1) * 8));
+  if (n > 0) k_count_runs<<<(unsigned)nfold, kFoldThreads, 0, lc.stream>>>(kin, n, runs.as<int64_t>());
+  launch_excl_scan(runs.as<int64_t>(), nfold, runs.as<int64_t>(), tmp.as<int64_t>(), lc);
   int64_t m = 0;
-  SPG_TRY(stage_read(ctx, ctx->h_stage + 52, pos.as<int64_t>() + n, 8));
+  SPG_TRY(stage_read(ctx, ctx->h_stage + 52, runs.as<int64_t>() + nfold, 8));
   int f = 0;
   SPG_TRY(stage_read(ctx, ctx->h_stage + 53, ctx->d_flags, 4));
   SPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -242,15 +306,15 @@ spg_status coo_to_csr_device(spg_ctx* ctx, int64_t rows, int64_t cols, int64_t n
     SPG_CUDA(ctx, cudaMemsetAsync(ctx->d_flags, 0, sizeof(int), ctx->stream));
     if (f & kFlagBadIndex) return fail(ctx, SPG_ERR_INVALID_ARG, "COO entry outside [0, rows) x [0, cols)");
   }
-  DevBuf col, val, urow, rp;
+  DevBuf col, val, rp;
   SPG_TRY(col.alloc(ctx, (size_t)m * 4));
   SPG_TRY(val.alloc(ctx, (size_t)m * 4));
-  SPG_TRY(urow.alloc(ctx, (size_t)std::max<int64_t>(m, 1) * 4));
   SPG_TRY(rp.alloc(ctx, (size_t)(rows + 1) * 8));
   if (n > 0)
-    k_fold_runs<<<blocks_for(n, lc.sms), 256, 0, lc.stream>>>(kin, vin, n, pos.as<int64_t>(), col.as<int32_t>(),
-                                                               val.as<float>(), urow.as<int32_t>());
-  k_rp_from_rows<<<blocks_for(m + 1, lc.sms), 256, 0, lc.stream>>>(urow.as<int32_t>(), m, rows, rp.as<int64_t>());
+    k_fold_runs<<<(unsigned)nfold, kFoldThreads, 0, lc.stream>>>(kin, vin, n, runs.as<int64_t>(), m, rows,
+                                                                 col.as<int32_t>(), val.as<float>(), rp.as<int64_t>());
+  else
+    SPG_CUDA(ctx, cudaMemsetAsync(rp.get(), 0, (size_t)(rows + 1) * 8, ctx->stream));
   SPG_CUDA(ctx, cudaGetLastError());
   SPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   std::memset(out, 0, sizeof *out);

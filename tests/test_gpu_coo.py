@@ -106,6 +106,19 @@ def test_coo_to_csr_device_inputs_and_edges(eng):
     check(C.to_host(), 500, r, c, v)
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 1), (1, 300), (70000, 1), (5, 257)])
+@pytest.mark.parametrize("n", [1, 2047, 2049, 4095, 4096, 4097, 12289])
+def test_tile_edges_and_narrow_shapes(eng, rows, cols, n):
+    """Around the sort's 4,096-entry and the fold's 2,048-entry tiles, with one
+    row or column (no sort pass over it) and long runs of duplicates that cross
+    tiles: the same bits as the numpy restatement."""
+    g = np.random.default_rng(n + rows)
+    r = g.integers(0, rows, n).astype(np.int32)
+    c = g.integers(0, cols, n).astype(np.int32)
+    v = g.uniform(-1, 1, n).astype(np.float32)
+    check(eng.coo_to_csr(rows, cols, r, c, v).to_host(), rows, r, c, v)
+
+
 def write_mtx(path, rows, cols, r, c, v, kind="real general"):
     with open(path, "w") as f:
         f.write(f"%%MatrixMarket matrix coordinate {kind}\n% generated\n{rows} {cols} {len(r)}\n")
