@@ -293,9 +293,9 @@ struct Pipeline {
     return SPG_OK;
   }
 
-  void bin(const int64_t* key, int mode) {
+  void bin(const int64_t* key, int mode, const EscArgs& esc = EscArgs{}) {
     launch_binning(key, rows, cols, mode, bp, bin_of_row.as<uint8_t>(), counts(), offsets(), cursors(),
-                   lists.as<int32_t>(), lc);
+                   lists.as<int32_t>(), lc, esc);
     ctx->launches += 3;
   }
 
@@ -443,6 +443,12 @@ struct Pipeline {
                       wpb, esc);
       ++ctx->launches;
     }
+    for (int b = kBinEsc; b < kBinEsc + kNumEscBins; ++b) {
+      if (bin_size(b) == 0) continue;
+      launch_num_esc(b, A.view, B.view, bin_rows(b), bin_size(b), row_prod, c_rp, c_col, c_val, nullptr, nullptr,
+                     nullptr, nullptr, ctx->d_flags, lc, wpb);
+      ++ctx->launches;
+    }
     // rows above the efficient warp tables: CTA-wide hash tables
     for (int b : {kBinBlock, kBinDense}) {
       if (bin_size(b) == 0) continue;
@@ -547,7 +553,7 @@ spg_status multiply_plain(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opts&
   tm.mark(SPG_STAGE_SYMBOLIC);
   SPG_TRY(P.symbolic(P.prod.as<int64_t>()));
   tm.mark(SPG_STAGE_BINNING);
-  P.bin(P.nnz.as<int64_t>(), kBinNumeric);
+  P.bin(P.nnz.as<int64_t>(), kBinNumeric, P.esc_args(P.prod.as<int64_t>()));
   tm.mark(SPG_STAGE_SCAN);
   launch_excl_scan(P.nnz.as<int64_t>(), P.rows, P.nnz.as<int64_t>(), P.scan_tmp.as<int64_t>(), lc);
   ctx->launches += 4;
@@ -600,7 +606,7 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
     BinParams lbp = P.bp;
     lbp.max_load = std::min(0.9f, std::max(0.1f, P.tune.learned_load > 0.f ? P.tune.learned_load : P.bp.max_load));
     launch_binning(cap.as<int64_t>(), rows, P.cols, kBinLearned, lbp, P.bin_of_row.as<uint8_t>(), P.counts(),
-                   P.offsets(), P.cursors(), P.lists.as<int32_t>(), lc);
+                   P.offsets(), P.cursors(), P.lists.as<int32_t>(), lc, P.esc_args(P.prod.as<int64_t>()));
     ctx->launches += 3;
   }
   launch_excl_scan(cap.as<int64_t>(), rows, slab_off.as<int64_t>(), P.scan_tmp.as<int64_t>(), lc);
@@ -610,10 +616,10 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
   SPG_TRY(stage_read(ctx, ctx->h_stage + kExactSlot, ctx->d_counter + 3, 8));
   SPG_TRY(P.fetch_offsets(slab_off.as<int64_t>() + rows, &slab_total, 1));
   const int64_t n_exact = ctx->h_stage[kExactSlot];
-  // predicted-light rows: the warp bins and the CTA bins, the first
+  // predicted-light rows: the warp, CTA and expand-sort-fold bins, the first
   // entries of the binning's lists
   int64_t light = 0;
-  for (int b = 0; b <= kBinDense; ++b) light += P.bin_size(b);
+  for (int b = 0; b < kBinHeavy; ++b) light += P.bin_size(b);
   if (rep) rep->rows_predicted = light;
   // single numeric pass for the predicted-light rows
   DevBuf slab_col, slab_val, retry;
@@ -627,6 +633,13 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
                             slab_off.as<int64_t>(), slab_col.as<int32_t>(), slab_val.as<float>(), P.nnz.as<int64_t>(),
                             retry.as<int32_t>(), ctx->d_counter + 2, ctx->d_flags, lc, P.wpb,
                             P.esc_args(P.prod.as<int64_t>()));
+    ++ctx->launches;
+  }
+  for (int b = kBinEsc; b < kBinEsc + kNumEscBins; ++b) {
+    if (P.bin_size(b) == 0) continue;
+    launch_num_esc(b, P.A.view, P.B.view, P.bin_rows(b), P.bin_size(b), P.prod.as<int64_t>(), slab_off.as<int64_t>(),
+                   slab_col.as<int32_t>(), slab_val.as<float>(), cap.as<int64_t>(), P.nnz.as<int64_t>(),
+                   retry.as<int32_t>(), ctx->d_counter + 2, ctx->d_flags, lc, P.wpb);
     ++ctx->launches;
   }
   for (int b : {kBinBlock, kBinDense}) {
@@ -680,7 +693,7 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
     ctx->launches += 2;
     SPG_TRY(P.symbolic(key.as<int64_t>()));
     launch_mask_key(P.nnz.as<int64_t>(), need.as<uint8_t>(), rows, key.as<int64_t>(), lc);
-    P.bin(key.as<int64_t>(), kBinNumeric);
+    P.bin(key.as<int64_t>(), kBinNumeric, P.esc_args(P.prod.as<int64_t>()));
     ctx->launches += 1;
   }
   if (exact_needed) {

@@ -101,7 +101,11 @@ __device__ __forceinline__ int ceil_log2_i64(int64_t v) {
 //  mode kBinSymbolic: key = products; bound u = min(key, cols).
 //  mode kBinNumeric:  key = exact nnz.
 //  mode kBinLearned:  key = predicted capacity (already capped by the bound).
-__device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const BinParams& bp) {
+// prod > 0 (numeric, learned): the row's products, of which esc_min or more
+// with half of them distinct send it to the expand-sort-fold bins when a word
+// holds any column and position of it.
+__device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const BinParams& bp, int64_t prod,
+                                      int esc_min) {
   if (mode == kBinSymbolic) {
     int64_t u = key < cols ? key : cols;
     if (u <= 0) return kBinEmpty;
@@ -120,6 +124,12 @@ __device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const
   }
   if (key <= 0) return kBinEmpty;
   const bool warp_ok = key <= bp.warp_cap;
+  if (warp_ok && key <= bp.block_min && esc_wanted(prod, key, esc_min, esc_bin_products(kNumEscBins - 1)) &&
+      ceil_log2_i64(cols) + ceil_log2_i64(prod) <= 31) {
+    int b = 0;
+    while (prod > esc_bin_products(b)) ++b;
+    return kBinEsc + b;
+  }
   if (!(warp_ok && key <= bp.block_min)) {
     // the CTA-wide hash bins
     if (key <= bp.blk_small_cap) return kBinBlock;
@@ -140,12 +150,12 @@ __device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const
 // atomic per (block, bin) -- rows of one matrix mostly share a bin, so
 // per-warp global atomics would queue on one address.
 __global__ void k_bin_count(const int64_t* key, int64_t rows, int64_t cols, int mode, BinParams bp,
-                            uint8_t* bin_of_row, int64_t* counts) {
+                            uint8_t* bin_of_row, int64_t* counts, const int64_t* prod, int esc_min) {
   __shared__ unsigned sh_cnt[kNumBins];
   if (threadIdx.x < kNumBins) sh_cnt[threadIdx.x] = 0;
   __syncthreads();
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
-    const int b = bin_of(key[r], cols, mode, bp);
+    const int b = bin_of(key[r], cols, mode, bp, prod ? prod[r] : 0, esc_min);
     bin_of_row[r] = (uint8_t)b;
     atomicAdd(&sh_cnt[b], 1u);
   }
@@ -639,6 +649,38 @@ __global__ void __maxnreg__(56) k_num_warp_learned(DCsr A, DCsr B, const int32_t
       if (lane == 0) nnz_out[row] = n;
     }
     next_row<LOGT>(keys, epoch);
+  }
+}
+
+// Expand-sort-fold rows of one bin, a warp a row, `words` words of shared
+// memory each (esc_capacity(words) >= the bin's products).
+//
+// Bound: latency and issue of the shared-memory passes over the row's products
+// (expand, count, scatter, rank, fold), so the memory a row needs decides the
+// warps at work: in the tables of its output's size a row of 1,024 products
+// took 48 KB and four warps an SM, by its products 15 KB and fifteen.
+template <bool R32, bool LEARNED>
+__global__ void __launch_bounds__(256) k_num_esc(DCsr A, DCsr B, const int32_t* rows, int64_t nrows,
+                                                 const int64_t* prod, int words, const int64_t* off, int32_t* out_col,
+                                                 float* out_val, const int64_t* cap, int64_t* nnz, int32_t* retry,
+                                                 unsigned long long* retry_count, int* flags) {
+  extern __shared__ int32_t sm_tab[];
+  int32_t* buf = sm_tab + (size_t)(threadIdx.x >> 5) * words;
+  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t idx = gw; idx < nrows; idx += nw) {
+    const int32_t row = rows[idx];
+    const int64_t o = off[row];
+    const int64_t want = LEARNED ? cap[row] : off[row + 1] - o;
+    const int n = esc_row<R32>(A, B, row, (int)prod[row], buf, want, out_col + o, out_val + o);
+    if (lane_id() == 0) {
+      if (LEARNED) {
+        nnz[row] = n > want ? -1 : n;
+        if (n > want || n < 0) retry[atomicAdd(retry_count, 1ull)] = row;
+      } else if (n != want) {
+        raise_flag(flags, kFlagCountDiff);
+      }
+    }
   }
 }
 
@@ -1426,11 +1468,12 @@ void launch_sum(const int64_t* v, int64_t n, unsigned long long* out, const Laun
 }
 
 void launch_binning(const int64_t* key, int64_t rows, int64_t cols, int mode, const BinParams& bp, uint8_t* bin_of_row,
-                    int64_t* counts, int64_t* offsets, int64_t* cursors, int32_t* lists, const LaunchCtx& lc) {
+                    int64_t* counts, int64_t* offsets, int64_t* cursors, int32_t* lists, const LaunchCtx& lc,
+                    const EscArgs& esc) {
   cudaMemsetAsync(counts, 0, sizeof(int64_t) * kNumBins, lc.stream);
   if (rows > 0)
     k_bin_count<<<grid_for(rows, 256, 1, lc.sms * 8), 256, 0, lc.stream>>>(key, rows, cols, mode, bp, bin_of_row,
-                                                                              counts);
+                                                                              counts, esc.prod, esc.min_prod);
   k_bin_offsets<<<1, 32, 0, lc.stream>>>(counts, offsets, cursors);
   if (rows > 0)
     k_bin_scatter<<<grid_for(rows, 256, 1, lc.sms * 8), 256, 0, lc.stream>>>(bin_of_row, rows, cursors, lists);
@@ -1676,6 +1719,41 @@ void launch_num_warp_learned(int log_t, const DCsr& A, const DCsr& B, const int3
     default: break;
   }
 #undef SPG_NWL
+}
+
+template <bool R32, bool LEARNED>
+static void num_esc_one(int bin, const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows,
+                        const int64_t* prod, const int64_t* off, int32_t* out_col, float* out_val, const int64_t* cap,
+                        int64_t* nnz, int32_t* retry, unsigned long long* retry_count, int* flags,
+                        const LaunchCtx& lc, int wpb) {
+  auto kernel = k_num_esc<R32, LEARNED>;
+  const int words = (3 * esc_bin_products(bin - kBinEsc) + kEscBuckets + 3) / 4 * 4;
+  const size_t per_warp = (size_t)words * 4;
+  const int fit = std::min(8, (int)(200 * 1024 / per_warp));
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  static std::atomic<int> auto_w[kNumEscBins];
+  const int w = std::min(fit, resolve_wpb(wpb, auto_w[bin - kBinEsc], kernel, per_warp, fit));
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, w * 32, w * per_warp);
+  const int blocks = grid_for(nrows, w, 1, lc.sms * std::max(1, per_sm));
+  kernel<<<blocks, w * 32, w * per_warp, lc.stream>>>(A, B, rows, nrows, prod, words, off, out_col, out_val, cap, nnz,
+                                                      retry, retry_count, flags);
+}
+
+void launch_num_esc(int bin, const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, const int64_t* prod,
+                    const int64_t* off, int32_t* out_col, float* out_val, const int64_t* cap, int64_t* nnz,
+                    int32_t* retry, unsigned long long* retry_count, int* flags, const LaunchCtx& lc, int wpb) {
+  if (nrows == 0) return;
+#define SPG_NE(R, K) \
+  num_esc_one<R, K>(bin, A, B, rows, nrows, prod, off, out_col, out_val, cap, nnz, retry, retry_count, flags, lc, wpb)
+  if (B.rp32) {
+    if (cap) SPG_NE(true, true);
+    else SPG_NE(true, false);
+  } else {
+    if (cap) SPG_NE(false, true);
+    else SPG_NE(false, false);
+  }
+#undef SPG_NE
 }
 
 template <int LOGT, bool R32>

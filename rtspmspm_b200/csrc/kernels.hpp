@@ -19,9 +19,14 @@ constexpr int kMaxLogT = 12;
 constexpr int kNumWarpBins = kMaxLogT - kMinLogT + 1;  // 8
 constexpr int kBinBlock = 8;   // symbolic: CTA hash table; numeric: CTA hash of 2^12 slots
 constexpr int kBinDense = 9;   // symbolic: CTA bitmap over the column span; numeric: CTA hash of 2^14 slots
-constexpr int kBinHeavy = 10;  // numeric: column-tiled heavy rows
-constexpr int kBinEmpty = 11;  // no products
-constexpr int kNumBins = 12;
+// Numeric and learned: rows expanded, sorted and folded (esc_row), by products.
+constexpr int kBinEsc = 10;
+constexpr int kNumEscBins = 5;
+// Largest products of bin kBinEsc + i.
+constexpr int esc_bin_products(int i) { return i == 0 ? 320 : i == 1 ? 640 : i == 2 ? 1152 : i == 3 ? 2048 : 4010; }
+constexpr int kBinHeavy = kBinEsc + kNumEscBins;  // numeric: column-tiled heavy rows
+constexpr int kBinEmpty = kBinHeavy + 1;          // no products
+constexpr int kNumBins = kBinEmpty + 1;
 
 // Log2 of the CTA-wide numeric hash tables of kBinBlock / kBinDense.
 constexpr int kBlkLogSmallT = 12;
@@ -101,10 +106,21 @@ void launch_small_count(const DCsr& A, const DCsr& B, int64_t* prod, int64_t* nn
                         int* flags, const LaunchCtx& lc);
 void launch_small_scan(int64_t* nnz, const int64_t* prod, int64_t rows, int32_t* rp32, int32_t* row_list,
                        unsigned long long* stop, int64_t* out, const LaunchCtx& lc);
+// Default smallest product count of an expand-sort-fold row.
+constexpr int kEscMinProd = 128;
+// Expand-sort-fold rows in the warp numeric kernels: the row products
+// (nullptr: off) and the smallest product count that takes the path
+// (0: off).
+struct EscArgs {
+  const int64_t* prod = nullptr;
+  int min_prod = 0;
+};
 void launch_sum(const int64_t* v, int64_t n, unsigned long long* out, const LaunchCtx& lc);
+// Rows into bins by their key; with `esc`, numeric and learned binnings send
+// the rows it wants to the expand-sort-fold bins.
 void launch_binning(const int64_t* key, int64_t rows, int64_t cols, int mode, const BinParams& bp,
                     uint8_t* bin_of_row, int64_t* counts, int64_t* offsets, int64_t* cursors, int32_t* lists,
-                    const LaunchCtx& lc);
+                    const LaunchCtx& lc, const EscArgs& esc = EscArgs{});
 int64_t scan_temp_elems(int64_t n);
 void launch_excl_scan(const int64_t* in, int64_t n, int64_t* out, int64_t* tmp, const LaunchCtx& lc);
 
@@ -116,15 +132,6 @@ void launch_sym_block(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t
 void launch_sym_dense(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, int64_t slot_base,
                       int64_t* nnz, int32_t* big_slot, int32_t* tile_cnt, int ntiles, uint32_t* bitmap, int* flags,
                       const LaunchCtx& lc);
-// Default smallest product count of an expand-sort-fold row.
-constexpr int kEscMinProd = 128;
-// Expand-sort-fold rows in the warp numeric kernels: the row products
-// (nullptr: off) and the smallest product count that takes the path
-// (0: off).
-struct EscArgs {
-  const int64_t* prod = nullptr;
-  int min_prod = 0;
-};
 void launch_num_warp(int log_t, const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows,
                      const int64_t* c_rp, int32_t* c_col, float* c_val, int* flags, const LaunchCtx& lc, int wpb,
                      const EscArgs& esc = EscArgs{});
@@ -132,6 +139,12 @@ void launch_num_warp_learned(int log_t, const DCsr& A, const DCsr& B, const int3
                              const int64_t* cap, const int64_t* slab_off, int32_t* slab_col, float* slab_val,
                              int64_t* nnz_out, int32_t* retry_rows, unsigned long long* retry_count, int* flags,
                              const LaunchCtx& lc, int wpb, const EscArgs& esc = EscArgs{});
+// Expand-sort-fold pass over the rows of bin kBinEsc + i: into C (off = its
+// row pointers, cap = null; the counts are checked) or into the slab (off = its
+// offsets; rows of more than cap[row] entries to `retry`, nnz -1).
+void launch_num_esc(int bin, const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, const int64_t* prod,
+                    const int64_t* off, int32_t* out_col, float* out_val, const int64_t* cap, int64_t* nnz,
+                    int32_t* retry, unsigned long long* retry_count, int* flags, const LaunchCtx& lc, int wpb);
 // CTA-wide hash numeric pass over the rows of bin kBinBlock (2^12-slot
 // tables) or kBinDense (2^14) of a numeric / learned binning.
 void launch_num_block(int bin, const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, const int64_t* c_rp,

@@ -476,16 +476,24 @@ __device__ __forceinline__ void next_row(int32_t* keys, int& epoch) {
 // For rows whose products mostly land on distinct columns the hash table
 // costs more than it saves: the row's P products are written in canonical
 // order (columns and values), turned into words ((column - lo) << b) |
-// position (b = the bits of P - 1), radix sorted (stable, LSD) on the column
-// bits, and folded left
-// to right, each column's sum starting from 0 and adding its products in
-// canonical order, as the hash accumulators do (the same bits).  Measured on
-// Erdos-Renyi 2^18 rows of 17 entries (289 products, 286 outputs per row):
-// numeric 3.85 -> 2.31 ms; rows of 64 products stay hashed (0.55 against
-// 0.81 ms).
+// position (b = the bits of P - 1), sorted, and folded left to right, each
+// column's sum starting from 0 and adding its products in canonical order, as
+// the hash accumulators do (the same bits).  Measured on Erdos-Renyi 2^18 rows
+// of 17 entries (289 products, 286 outputs per row): numeric 3.85 -> 2.31 ms;
+// rows of 64 products stay hashed (0.55 against 0.81 ms).
+//
+// The words differ in their positions, so the sort need not be stable: one
+// scatter into kEscBuckets ranges of columns (the order inside a bucket does
+// not matter) and then every word counts the smaller ones of its bucket, a
+// few words.  A stable radix sort ranks every word of every pass with
+// __match_any_sync, which takes an SM about 70 cycles for 30 distinct digits.
+constexpr int kEscBuckets = 256;
+// A fuller bucket than this sends the row to a bitonic sort (columns crowded
+// into few of the ranges).
+constexpr int kEscCrowd = 64;
 // Largest P that `words` 32-bit words of a warp's shared memory hold: two
-// word buffers, the values and 256 bucket counts.
-__host__ __device__ __forceinline__ int esc_capacity(int words) { return (words - 256) / 3; }
+// word buffers, the values and the bucket counts.
+__host__ __device__ __forceinline__ int esc_capacity(int words) { return (words - kEscBuckets) / 3; }
 
 // True when a row of `prod` products and at least `out` output entries
 // (its exact count, or the learned capacity) takes the expand-sort-fold
@@ -513,7 +521,7 @@ __device__ __forceinline__ int esc_row(const DCsr& A, const DCsr& B, int32_t row
   // expand in canonical order: columns into wa, products into vals
   const int64_t s = A.rp[row], e = A.rp[row + 1];
   int base = 0;
-  int lo = 0x7fffffff, hi = -1;
+  int lo = 0x7fffffff, hi = 0;  // a lane without products leaves both alone
   for (int64_t c0 = s; c0 < e; c0 += 32) {
     const int64_t q = c0 + lane;
     Off bs = 0;
@@ -557,47 +565,52 @@ __device__ __forceinline__ int esc_row(const DCsr& A, const DCsr& B, int32_t row
     return -1;
   }
   __syncwarp();
-  for (int i = lane; i < P; i += 32) wa[i] = ((wa[i] - (uint32_t)lo) << ib) | (uint32_t)i;
+  // bucket of a column: its share of the span, in order
+  const uint32_t mult = span >= kEscBuckets ? (uint32_t)(((uint64_t)kEscBuckets << 32) / ((uint64_t)span + 1u)) : 0u;
+  auto bucket = [&](uint32_t off) { return mult ? __umulhi(off, mult) : off; };
+  for (int b = lane; b < kEscBuckets; b += 32) hist[b] = 0;
   __syncwarp();
-  // stable LSD radix sort on the column bits, 8-bit digits
-  uint32_t* src = wa;
-  uint32_t* dst = wb;
-  for (int shift = ib; shift < ib + span_bits; shift += 8) {
-    for (int b = lane; b < 256; b += 32) hist[b] = 0;
-    __syncwarp();
-    for (int i = lane; i < P; i += 32) atomicAdd(&hist[(src[i] >> shift) & 255u], 1);
-    __syncwarp();
-    int loc[8];
-    int sum = 0;
+  for (int i = lane; i < P; i += 32) atomicAdd(&hist[bucket(wa[i] - (uint32_t)lo)], 1);
+  __syncwarp();
+  constexpr int kPer = kEscBuckets / 32;
+  int loc[kPer];
+  int sum = 0, most = 0;
 #pragma unroll
-    for (int x = 0; x < 8; ++x) {
-      loc[x] = hist[lane * 8 + x];
-      sum += loc[x];
-    }
-    int run = warp_incl_scan(sum) - sum;
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {
-      hist[lane * 8 + x] = run;
-      run += loc[x];
-    }
-    __syncwarp();
-    for (int i0 = 0; i0 < P; i0 += 32) {
-      const int i = i0 + lane;
-      const bool act = i < P;
-      const uint32_t v = act ? src[i] : 0u;
-      const int dig = act ? (int)((v >> shift) & 255u) : -1 - lane;
-      const unsigned grp = __match_any_sync(kFull, dig);
-      const int leader = __ffs(grp) - 1;
-      int at = 0;
-      if (act && lane == leader) at = atomicAdd(&hist[dig], __popc(grp));
-      at = __shfl_sync(kFull, at, leader);
-      if (act) dst[at + __popc(grp & lt)] = v;
-    }
-    __syncwarp();
-    uint32_t* t = src;
-    src = dst;
-    dst = t;
+  for (int x = 0; x < kPer; ++x) {
+    loc[x] = hist[lane * kPer + x];
+    sum += loc[x];
+    most = max(most, loc[x]);
   }
+  int run = warp_incl_scan(sum) - sum;
+#pragma unroll
+  for (int x = 0; x < kPer; ++x) {
+    hist[lane * kPer + x] = run;
+    run += loc[x];
+  }
+  most = __reduce_max_sync(kFull, most);
+  __syncwarp();
+  const uint32_t* src = wa;
+  if (most <= kEscCrowd) {
+    for (int i = lane; i < P; i += 32) {
+      const uint32_t off = wa[i] - (uint32_t)lo;
+      wb[atomicAdd(&hist[bucket(off)], 1)] = (off << ib) | (uint32_t)i;
+    }
+    __syncwarp();
+    // hist[b] is now the end of bucket b
+    for (int i = lane; i < P; i += 32) {
+      const uint32_t w = wb[i];
+      const uint32_t b = bucket(w >> ib);
+      const int b0 = b ? hist[b - 1] : 0, b1 = hist[b];
+      int at = b0;
+      for (int j = b0; j < b1; ++j) at += wb[j] < w;
+      wa[at] = w;
+    }
+  } else {
+    for (int i = lane; i < P; i += 32) wa[i] = ((wa[i] - (uint32_t)lo) << ib) | (uint32_t)i;
+    __syncwarp();
+    warp_sort_keys(reinterpret_cast<int32_t*>(wa), P, 2 * P);  // the padding reaches into wb
+  }
+  __syncwarp();
   // fold runs of equal columns left to right; run heads write the entries
   int count = 0;
   for (int i0 = 0; i0 < P; i0 += 32) {
