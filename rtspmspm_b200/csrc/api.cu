@@ -264,6 +264,7 @@ struct Pipeline {
   DevBuf binmeta;     // int64: counts[12] offsets[13] cursors[12]
   DevBuf lists;       // int32 rows
   DevBuf big_slot;    // int32 rows
+  DevBuf span;        // int32 rows: span words (plain method)
   DevBuf tile_cnt;    // int32 nbig * ntiles
   DevBuf tile_off;    // int32 nbig * ntiles
   DevBuf bitmap;      // uint32 nbig * bitmap_stride(), or empty
@@ -293,9 +294,17 @@ struct Pipeline {
     return SPG_OK;
   }
 
+  // Products of every row and, for the symbolic binning, their span words.
+  spg_status products() {
+    SPG_TRY(span.alloc(ctx, (size_t)std::max<int64_t>(rows, 1) * 4));
+    launch_row_products(A.view, B.view, prod.as<int64_t>(), lc, span.as<int32_t>());
+    ++ctx->launches;
+    return SPG_OK;
+  }
+
   void bin(const int64_t* key, int mode, const EscArgs& esc = EscArgs{}) {
     launch_binning(key, rows, cols, mode, bp, bin_of_row.as<uint8_t>(), counts(), offsets(), cursors(),
-                   lists.as<int32_t>(), lc, esc);
+                   lists.as<int32_t>(), lc, esc, span.as<int32_t>());
     ctx->launches += 3;
   }
 
@@ -320,6 +329,11 @@ struct Pipeline {
   spg_status symbolic(const int64_t* key) {
     bin(key, kBinSymbolic);
     SPG_TRY(fetch_offsets());
+    for (int b = kBinSpan; b < kBinSpan + kNumSpanBins; ++b) {
+      if (bin_size(b) == 0) continue;
+      launch_sym_span(b, A.view, B.view, bin_rows(b), bin_size(b), nnz.as<int64_t>(), ctx->d_flags, lc);
+      ++ctx->launches;
+    }
     for (int b = 0; b < kNumWarpBins; ++b) {
       if (bin_size(b) == 0) continue;
       launch_sym_warp(kMinLogT + b, A.view, B.view, bin_rows(b), bin_size(b), nnz.as<int64_t>(), ctx->d_flags, lc,
@@ -546,10 +560,10 @@ spg_status multiply_plain(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opts&
                           StageTimer& tm) {
   const LaunchCtx lc = P.lc;
   tm.mark(SPG_STAGE_PRODUCTS);
-  launch_row_products(P.A.view, P.B.view, P.prod.as<int64_t>(), lc);
+  SPG_TRY(P.products());
   SPG_CUDA(ctx, cudaMemsetAsync(ctx->d_counter + 1, 0, 8, ctx->stream));
   launch_sum(P.prod.as<int64_t>(), P.rows, ctx->d_counter + 1, lc);
-  ctx->launches += 2;
+  ++ctx->launches;
   tm.mark(SPG_STAGE_SYMBOLIC);
   SPG_TRY(P.symbolic(P.prod.as<int64_t>()));
   tm.mark(SPG_STAGE_BINNING);
@@ -616,7 +630,7 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
   SPG_TRY(stage_read(ctx, ctx->h_stage + kExactSlot, ctx->d_counter + 3, 8));
   SPG_TRY(P.fetch_offsets(slab_off.as<int64_t>() + rows, &slab_total, 1));
   const int64_t n_exact = ctx->h_stage[kExactSlot];
-  // predicted-light rows: the warp, CTA and expand-sort-fold bins, the first
+  // predicted-light rows: the warp, CTA, and expand-sort-fold bins, the first
   // entries of the binning's lists
   int64_t light = 0;
   for (int b = 0; b < kBinHeavy; ++b) light += P.bin_size(b);
@@ -883,7 +897,7 @@ spg_status multiply_reuse_device(spg_ctx* ctx, const DevMat& A, const DevMat& B,
 spg_status row_nnz_device(spg_ctx* ctx, const DevMat& A, const DevMat& B, int64_t* d_nnz) {
   Pipeline P(ctx, A, B, ctx->tuning);
   SPG_TRY(P.init());
-  launch_row_products(A.view, B.view, P.prod.as<int64_t>(), P.lc);
+  SPG_TRY(P.products());
   SPG_TRY(P.symbolic(P.prod.as<int64_t>()));
   if (P.rows)
     SPG_CUDA(ctx, cudaMemcpyAsync(d_nnz, P.nnz.get(), (size_t)P.rows * 8, cudaMemcpyDeviceToDevice, ctx->stream));

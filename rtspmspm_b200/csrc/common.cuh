@@ -202,6 +202,9 @@ __device__ __forceinline__ int hash_find(const int32_t* keys, int log_t, int32_t
   return -1;
 }
 
+// 32-column words from the word of column lo to that of column hi.
+__device__ __forceinline__ int span_words(int32_t lo, int32_t hi) { return (hi >> 5) - (lo >> 5) + 1; }
+
 // B-row segments shorter than this are packed several to a warp step; longer
 // ones are read by the whole warp, one segment at a time.
 constexpr int kPackBelow = 16;

@@ -62,20 +62,37 @@ __global__ void k_validate(DCsr M, int64_t nnz, int* flags) {
 }
 
 // Intermediate products per row (sum of |B_k| over k in A_i) and the upper
-// bound min(products, cols of B) of its output nnz.  One warp per row.
-__global__ void k_row_products(DCsr A, DCsr B, int64_t* prod) {
+// bound min(products, cols of B) of its output nnz.  One warp per row.  SPAN:
+// the words of the bitmap over the row's columns too (0 when its rows of B
+// hold fewer than kPackBelow entries on average: packing them costs as much as
+// hashing them).
+template <bool SPAN>
+__global__ void k_row_products(DCsr A, DCsr B, int64_t* prod, int32_t* span) {
   const int lane = lane_id();
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t r = gw; r < A.rows; r += nw) {
     const int64_t s = A.rp[r], e = A.rp[r + 1];
     int64_t sum = 0;
+    unsigned lo = 0x7fffffffu, hi = 0u;
     for (int64_t p = s + lane; p < e; p += 32) {
-      int32_t k = A.col[p];
-      sum += B.rp[k + 1] - B.rp[k];
+      const int32_t k = A.col[p];
+      const int64_t bs = B.rp[k], be = B.rp[k + 1];
+      sum += be - bs;
+      if (SPAN && be > bs) {
+        lo = min(lo, (unsigned)B.col[bs]);
+        hi = max(hi, (unsigned)B.col[be - 1]);
+      }
     }
     sum = warp_sum(sum);
-    if (lane == 0) prod[r] = sum;
+    if (SPAN) {
+      lo = __reduce_min_sync(kFull, lo);
+      hi = __reduce_max_sync(kFull, hi);
+    }
+    if (lane == 0) {
+      prod[r] = sum;
+      if (SPAN) span[r] = sum >= (e - s) * kPackBelow && sum > 0 ? span_words((int32_t)lo, (int32_t)hi) : 0;
+    }
   }
 }
 
@@ -105,10 +122,16 @@ __device__ __forceinline__ int ceil_log2_i64(int64_t v) {
 // with half of them distinct send it to the expand-sort-fold bins when a word
 // holds any column and position of it.
 __device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const BinParams& bp, int64_t prod,
-                                      int esc_min) {
+                                      int esc_min, int span) {
   if (mode == kBinSymbolic) {
     int64_t u = key < cols ? key : cols;
     if (u <= 0) return kBinEmpty;
+    // counting and clearing a span's words (a quarter instruction each) must
+    // not outweigh the products (60 a hash step of 32 saved); small tunings of
+    // the tables keep their rows
+    if (span > 0 && span <= span_bin_words(kNumSpanBins - 1) && bp.warp_log_max >= 9 && key >= 64 &&
+        u <= bp.warp_cap && span <= 4 * key)
+      return kBinSpan + (span > span_bin_words(0)) + (span > span_bin_words(1));
     if (u <= bp.warp_cap) {
       // a row has at most u distinct columns, so a table of 1.25 u slots
       // stays at most 4/5 full, and usually far below (125 columns from
@@ -150,12 +173,13 @@ __device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const
 // atomic per (block, bin) -- rows of one matrix mostly share a bin, so
 // per-warp global atomics would queue on one address.
 __global__ void k_bin_count(const int64_t* key, int64_t rows, int64_t cols, int mode, BinParams bp,
-                            uint8_t* bin_of_row, int64_t* counts, const int64_t* prod, int esc_min) {
+                            uint8_t* bin_of_row, int64_t* counts, const int64_t* prod, int esc_min,
+                            const int32_t* span) {
   __shared__ unsigned sh_cnt[kNumBins];
   if (threadIdx.x < kNumBins) sh_cnt[threadIdx.x] = 0;
   __syncthreads();
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
-    const int b = bin_of(key[r], cols, mode, bp, prod ? prod[r] : 0, esc_min);
+    const int b = bin_of(key[r], cols, mode, bp, prod ? prod[r] : 0, esc_min, span ? span[r] : 0);
     bin_of_row[r] = (uint8_t)b;
     atomicAdd(&sh_cnt[b], 1u);
   }
@@ -1440,9 +1464,11 @@ void launch_validate(const DCsr& M, int64_t nnz, int* flags, const LaunchCtx& lc
   k_validate<<<grid_for(M.rows, 256, 32, lc.sms * 16), 256, 0, lc.stream>>>(M, nnz, flags);
 }
 
-void launch_row_products(const DCsr& A, const DCsr& B, int64_t* prod, const LaunchCtx& lc) {
+void launch_row_products(const DCsr& A, const DCsr& B, int64_t* prod, const LaunchCtx& lc, int32_t* span) {
   if (A.rows == 0) return;
-  k_row_products<<<grid_for(A.rows, 256, 32, lc.sms * 16), 256, 0, lc.stream>>>(A, B, prod);
+  const int blocks = grid_for(A.rows, 256, 32, lc.sms * 16);
+  if (span) k_row_products<true><<<blocks, 256, 0, lc.stream>>>(A, B, prod, span);
+  else k_row_products<false><<<blocks, 256, 0, lc.stream>>>(A, B, prod, nullptr);
 }
 
 void launch_small_count(const DCsr& A, const DCsr& B, int64_t* prod, int64_t* nnz, unsigned long long* stop,
@@ -1469,11 +1495,11 @@ void launch_sum(const int64_t* v, int64_t n, unsigned long long* out, const Laun
 
 void launch_binning(const int64_t* key, int64_t rows, int64_t cols, int mode, const BinParams& bp, uint8_t* bin_of_row,
                     int64_t* counts, int64_t* offsets, int64_t* cursors, int32_t* lists, const LaunchCtx& lc,
-                    const EscArgs& esc) {
+                    const EscArgs& esc, const int32_t* span) {
   cudaMemsetAsync(counts, 0, sizeof(int64_t) * kNumBins, lc.stream);
   if (rows > 0)
     k_bin_count<<<grid_for(rows, 256, 1, lc.sms * 8), 256, 0, lc.stream>>>(key, rows, cols, mode, bp, bin_of_row,
-                                                                              counts, esc.prod, esc.min_prod);
+                                                                              counts, esc.prod, esc.min_prod, span);
   k_bin_offsets<<<1, 32, 0, lc.stream>>>(counts, offsets, cursors);
   if (rows > 0)
     k_bin_scatter<<<grid_for(rows, 256, 1, lc.sms * 8), 256, 0, lc.stream>>>(bin_of_row, rows, cursors, lists);

@@ -24,6 +24,10 @@ constexpr int kBinEsc = 10;
 constexpr int kNumEscBins = 5;
 // Largest products of bin kBinEsc + i.
 constexpr int esc_bin_products(int i) { return i == 0 ? 320 : i == 1 ? 640 : i == 2 ? 1152 : i == 3 ? 2048 : 4010; }
+// Symbolic: rows with a bitmap of their column span (span.cu), by its words.
+constexpr int kBinSpan = kBinEsc;
+constexpr int kNumSpanBins = 3;
+constexpr int span_bin_words(int i) { return i == 0 ? 576 : i == 1 ? 1216 : 2048; }
 constexpr int kBinHeavy = kBinEsc + kNumEscBins;  // numeric: column-tiled heavy rows
 constexpr int kBinEmpty = kBinHeavy + 1;          // no products
 constexpr int kNumBins = kBinEmpty + 1;
@@ -85,7 +89,9 @@ struct LaunchCtx {
 void launch_widen_rp(const int32_t* in, int64_t n, int64_t* out, const LaunchCtx& lc);
 void launch_narrow_rp(const int64_t* in, int64_t n, int32_t* out, const LaunchCtx& lc);
 void launch_validate(const DCsr& M, int64_t nnz, int* flags, const LaunchCtx& lc);
-void launch_row_products(const DCsr& A, const DCsr& B, int64_t* prod, const LaunchCtx& lc);
+// Products of every row and, when `span` is given, the words of its column
+// span's bitmap (span_words; 0: none).
+void launch_row_products(const DCsr& A, const DCsr& B, int64_t* prod, const LaunchCtx& lc, int32_t* span = nullptr);
 
 // Small products (at most kSmallMaxRows rows of A, every row of at most
 // 2^kSmallLogT products): products and exact counts per row in one launch
@@ -117,10 +123,11 @@ struct EscArgs {
 };
 void launch_sum(const int64_t* v, int64_t n, unsigned long long* out, const LaunchCtx& lc);
 // Rows into bins by their key; with `esc`, numeric and learned binnings send
-// the rows it wants to the expand-sort-fold bins.
+// the rows it wants to the expand-sort-fold bins, with `span`, symbolic ones
+// the rows of few span words to the span bins.
 void launch_binning(const int64_t* key, int64_t rows, int64_t cols, int mode, const BinParams& bp,
                     uint8_t* bin_of_row, int64_t* counts, int64_t* offsets, int64_t* cursors, int32_t* lists,
-                    const LaunchCtx& lc, const EscArgs& esc = EscArgs{});
+                    const LaunchCtx& lc, const EscArgs& esc = EscArgs{}, const int32_t* span = nullptr);
 int64_t scan_temp_elems(int64_t n);
 void launch_excl_scan(const int64_t* in, int64_t n, int64_t* out, int64_t* tmp, const LaunchCtx& lc);
 
@@ -139,6 +146,9 @@ void launch_num_warp_learned(int log_t, const DCsr& A, const DCsr& B, const int3
                              const int64_t* cap, const int64_t* slab_off, int32_t* slab_col, float* slab_val,
                              int64_t* nnz_out, int32_t* retry_rows, unsigned long long* retry_count, int* flags,
                              const LaunchCtx& lc, int wpb, const EscArgs& esc = EscArgs{});
+// Span bitmaps: exact counts of the rows of a symbolic bin.
+void launch_sym_span(int bin, const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, int64_t* nnz,
+                     int* flags, const LaunchCtx& lc);
 // Expand-sort-fold pass over the rows of bin kBinEsc + i: into C (off = its
 // row pointers, cap = null; the counts are checked) or into the slab (off = its
 // offsets; rows of more than cap[row] entries to `retry`, nnz -1).
