@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <mutex>
 
 #include "context.hpp"
 
@@ -42,17 +43,75 @@ spg_status cuda_status(spg_ctx* ctx, cudaError_t e, const char* what) {
   return fail(ctx, st, "%s: %s", what, cudaGetErrorString(e));
 }
 
-spg_status DevBuf::alloc(spg_ctx* ctx, size_t bytes) {
+spg_status DevBuf::alloc_from(spg_ctx* ctx, size_t bytes, cudaMemPool_t pool) {
   reset();
   ctx_ = ctx;
   if (bytes == 0) return SPG_OK;
-  cudaError_t e = cudaMallocAsync(&ptr_, bytes, ctx->stream);
+  cudaError_t e = cudaMallocFromPoolAsync(&ptr_, bytes, pool, ctx->stream);
+  if (e == cudaErrorMemoryAllocation) {
+    // what either pool holds in reserve may be what the other lacks
+    (void)cudaGetLastError();
+    cudaStreamSynchronize(ctx->stream);
+    cudaMemPoolTrimTo(ctx->scratch, 0);
+    cudaMemPoolTrimTo(ctx->pool, 0);
+    e = cudaMallocFromPoolAsync(&ptr_, bytes, pool, ctx->stream);
+  }
   if (e != cudaSuccess) {
     ptr_ = nullptr;
-    return cuda_status(ctx, e, "cudaMallocAsync");
+    return cuda_status(ctx, e, "cudaMallocFromPoolAsync");
   }
   return SPG_OK;
 }
+
+namespace {
+
+// One scratch pool a device, shared by its contexts, kept while any of them
+// lives.  It keeps up to kScratchKeep bytes between calls (an R-MAT scale 18
+// product works in 3.5 GB, scale 20 in 9 GB); more goes back to the device at
+// the next synchronisation.
+constexpr int kMaxDevices = 64;
+constexpr uint64_t kScratchKeep = uint64_t(12) << 30;
+struct ScratchPool {
+  cudaMemPool_t pool = nullptr;
+  int contexts = 0;
+};
+std::mutex g_scratch_mutex;
+ScratchPool g_scratch[kMaxDevices];
+
+cudaError_t scratch_acquire(int device, cudaMemPool_t* out) {
+  if (device >= kMaxDevices) return cudaDeviceGetDefaultMemPool(out, device);
+  std::lock_guard<std::mutex> hold(g_scratch_mutex);
+  ScratchPool& s = g_scratch[device];
+  if (s.contexts == 0) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaError_t e = cudaMemPoolCreate(&s.pool, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = kScratchKeep;
+    e = cudaMemPoolSetAttribute(s.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(s.pool);
+      return e;
+    }
+  }
+  ++s.contexts;
+  *out = s.pool;
+  return cudaSuccess;
+}
+
+void scratch_release(int device) {
+  if (device >= kMaxDevices) return;
+  std::lock_guard<std::mutex> hold(g_scratch_mutex);
+  ScratchPool& s = g_scratch[device];
+  if (--s.contexts == 0) {
+    cudaMemPoolDestroy(s.pool);
+    s.pool = nullptr;
+  }
+}
+
+}  // namespace
 
 void DevBuf::reset() {
   if (ptr_ && ctx_) cudaFreeAsync(ptr_, ctx_->stream);
@@ -195,15 +254,11 @@ spg_status prepare_matrix(spg_ctx* ctx, const spg_csr* m, DevMat& out, bool vali
 }
 
 StageTimer::StageTimer(spg_ctx* ctx, bool enabled) : ctx_(ctx), on_(enabled) {
-  cudaEventCreate(&start_);
-  cudaEventCreate(&end_);
-  cudaEventRecord(start_, ctx->stream);
+  cudaEventRecord(ctx->ev_start, ctx->stream);
 }
 
 StageTimer::~StageTimer() {
   for (auto& m : marks_) cudaEventDestroy(m.second);
-  cudaEventDestroy(start_);
-  cudaEventDestroy(end_);
 }
 
 void StageTimer::mark(int stage) {
@@ -215,6 +270,7 @@ void StageTimer::mark(int stage) {
 }
 
 void StageTimer::finish(spg_report* rep) {
+  const cudaEvent_t start_ = ctx_->ev_start, end_ = ctx_->ev_end;
   cudaEventRecord(end_, ctx_->stream);
   cudaEventSynchronize(end_);
   if (!rep) return;
@@ -258,17 +314,18 @@ struct Pipeline {
   int ntiles;
   int wpb;
 
-  DevBuf prod;        // int64 rows
+  DevBuf block;         // holds the slices below
+  DevSlice prod;        // int64 rows
+  DevSlice bin_of_row;  // uint8 rows
+  DevSlice binmeta;     // int64: counts, offsets (one more) and cursors of the bins
+  DevSlice lists;       // int32 rows
+  DevSlice big_slot;    // int32 rows
+  DevSlice scan_tmp;    // int64
   DevBuf nnz;         // int64 rows+1 (becomes C's row pointers)
-  DevBuf bin_of_row;  // uint8 rows
-  DevBuf binmeta;     // int64: counts[12] offsets[13] cursors[12]
-  DevBuf lists;       // int32 rows
-  DevBuf big_slot;    // int32 rows
   DevBuf span;        // int32 rows: span words (plain method)
   DevBuf tile_cnt;    // int32 nbig * ntiles
   DevBuf tile_off;    // int32 nbig * ntiles
   DevBuf bitmap;      // uint32 nbig * bitmap_stride(), or empty
-  DevBuf scan_tmp;    // int64
   int64_t h_off[kNumBins + 1] = {};
   int64_t nbig = 0;
 
@@ -283,13 +340,16 @@ struct Pipeline {
   int64_t* cursors() { return binmeta.as<int64_t>() + 2 * kNumBins + 1; }
 
   spg_status init() {
-    SPG_TRY(prod.alloc(ctx, (size_t)std::max<int64_t>(rows, 1) * 8));
-    SPG_TRY(nnz.alloc(ctx, (size_t)(rows + 1) * 8));
-    SPG_TRY(bin_of_row.alloc(ctx, (size_t)std::max<int64_t>(rows, 1)));
-    SPG_TRY(binmeta.alloc(ctx, (size_t)(3 * kNumBins + 1) * 8));
-    SPG_TRY(lists.alloc(ctx, (size_t)std::max<int64_t>(rows, 1) * 4));
-    SPG_TRY(big_slot.alloc(ctx, (size_t)std::max<int64_t>(rows, 1) * 4));
-    SPG_TRY(scan_tmp.alloc(ctx, (size_t)scan_temp_elems(rows + 1) * 8));
+    const size_t r = (size_t)std::max<int64_t>(rows, 1);
+    DevLayout l;
+    l.add(&prod, r * 8);
+    l.add(&bin_of_row, r);
+    l.add(&binmeta, (size_t)(3 * kNumBins + 1) * 8);
+    l.add(&lists, r * 4);
+    l.add(&big_slot, r * 4);
+    l.add(&scan_tmp, (size_t)scan_temp_elems(rows + 1) * 8);
+    SPG_TRY(l.alloc(ctx, block));
+    SPG_TRY(nnz.alloc_result(ctx, (size_t)(rows + 1) * 8));
     SPG_CUDA(ctx, cudaMemsetAsync(nnz.get(), 0, (size_t)(rows + 1) * 8, ctx->stream));
     return SPG_OK;
   }
@@ -381,8 +441,8 @@ struct Pipeline {
   spg_status alloc_entries(int64_t total, DevBuf& c_col, DevBuf& c_val) {
     spg_status st = SPG_OK;
     for (int pass = 0; pass < 2; ++pass) {
-      st = c_col.alloc(ctx, (size_t)total * 4);
-      if (st == SPG_OK) st = c_val.alloc(ctx, (size_t)total * 4);
+      st = c_col.alloc_result(ctx, (size_t)total * 4);
+      if (st == SPG_OK) st = c_val.alloc_result(ctx, (size_t)total * 4);
       if (st != SPG_ERR_OUT_OF_MEMORY || !bitmap.get()) break;
       c_col.reset();
       bitmap.reset();
@@ -521,7 +581,7 @@ spg_status finish_output(spg_ctx* ctx, Pipeline& P, int64_t total, const spg_opt
     rp = P.nnz.release();
   } else {
     DevBuf rp32;
-    SPG_TRY(rp32.alloc(ctx, (size_t)(P.rows + 1) * 4));
+    SPG_TRY(rp32.alloc_result(ctx, (size_t)(P.rows + 1) * 4));
     launch_narrow_rp(P.nnz.as<int64_t>(), P.rows + 1, rp32.as<int32_t>(), lc);
     ++ctx->launches;
     rp = rp32.release();
@@ -598,11 +658,18 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
   const LaunchCtx lc = P.lc;
   SPG_TRY(ensure_mlp(ctx));
   const int64_t rows = P.rows;
-  DevBuf cap, need, slab_off, key;
-  SPG_TRY(cap.alloc(ctx, (size_t)(rows + 1) * 8));
-  SPG_TRY(need.alloc(ctx, (size_t)std::max<int64_t>(rows, 1)));
-  SPG_TRY(slab_off.alloc(ctx, (size_t)(rows + 1) * 8));
-  SPG_TRY(key.alloc(ctx, (size_t)std::max<int64_t>(rows, 1) * 8));
+  DevBuf learned_block;
+  DevSlice cap, need, slab_off, key, retry;
+  {
+    const size_t r = (size_t)std::max<int64_t>(rows, 1);
+    DevLayout l;
+    l.add(&cap, (size_t)(rows + 1) * 8);
+    l.add(&need, r);
+    l.add(&slab_off, (size_t)(rows + 1) * 8);
+    l.add(&key, r * 8);
+    l.add(&retry, r * 4);
+    SPG_TRY(l.alloc(ctx, learned_block));
+  }
   // products, features and the tensor-core MLP in one pass over A
   tm.mark(SPG_STAGE_MLP);
   // d_counter: [1] products, [2] overflowed rows, [3] rows predicted heavy
@@ -636,10 +703,9 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
   for (int b = 0; b < kBinHeavy; ++b) light += P.bin_size(b);
   if (rep) rep->rows_predicted = light;
   // single numeric pass for the predicted-light rows
-  DevBuf slab_col, slab_val, retry;
+  DevBuf slab_col, slab_val;
   SPG_TRY(slab_col.alloc(ctx, (size_t)slab_total * 4));
   SPG_TRY(slab_val.alloc(ctx, (size_t)slab_total * 4));
-  SPG_TRY(retry.alloc(ctx, (size_t)std::max<int64_t>(light, 1) * 4));
   tm.mark(SPG_STAGE_NUMERIC);
   for (int b = 0; b < kNumWarpBins; ++b) {
     if (P.bin_size(b) == 0) continue;
@@ -764,7 +830,7 @@ spg_status multiply_small(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opts&
   const int bits = o.out_index_bits;
   if (bits != 0 && bits != 32 && bits != 64) return fail(ctx, SPG_ERR_INVALID_ARG, "out_index_bits must be 0, 32 or 64");
   DevBuf rp32;
-  if (bits != 64) SPG_TRY(rp32.alloc(ctx, (size_t)(rows + 1) * 4));
+  if (bits != 64) SPG_TRY(rp32.alloc_result(ctx, (size_t)(rows + 1) * 4));
   tm.mark(SPG_STAGE_SYMBOLIC);
   // d_counter[6]: the counting launch's stop word (zero between calls)
   launch_small_count(P.A.view, P.B.view, P.prod.as<int64_t>(), P.nnz.as<int64_t>(), ctx->d_counter + 6, ctx->d_flags,
@@ -789,8 +855,7 @@ spg_status multiply_small(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opts&
   if (bits == 32 && total >= INT32_MAX)
     return fail(ctx, SPG_ERR_INVALID_ARG, "nnz(C)=%lld does not fit int32 row pointers", (long long)total);
   DevBuf c_col, c_val;
-  SPG_TRY(c_col.alloc(ctx, (size_t)total * 4));
-  SPG_TRY(c_val.alloc(ctx, (size_t)total * 4));
+  SPG_TRY(P.alloc_entries(total, c_col, c_val));
   tm.mark(SPG_STAGE_NUMERIC);
   if (total > 0) {
     launch_num_warp(log_t, P.A.view, P.B.view, P.lists.as<int32_t>(), rows, P.nnz.as<int64_t>(), c_col.as<int32_t>(),
@@ -951,6 +1016,8 @@ spg_status spg_create(spg_ctx** out, int32_t device) {
   SPG_CUDA(ctx.get(), cudaDeviceGetDefaultMemPool(&ctx->pool, device));
   uint64_t thr = UINT64_MAX;
   SPG_CUDA(ctx.get(), cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &thr));
+  SPG_CUDA(ctx.get(), cudaEventCreate(&ctx->ev_start));
+  SPG_CUDA(ctx.get(), cudaEventCreate(&ctx->ev_end));
   SPG_CUDA(ctx.get(), cudaMalloc(&ctx->d_flags, 64));
   SPG_CUDA(ctx.get(), cudaMemset(ctx->d_flags, 0, 64));
   SPG_CUDA(ctx.get(), cudaMalloc(&ctx->d_counter, 16 * sizeof(unsigned long long)));
@@ -959,6 +1026,7 @@ spg_status spg_create(spg_ctx** out, int32_t device) {
   SPG_CUDA(ctx.get(), cudaHostAlloc((void**)&ctx->h_stage, 64 * sizeof(int64_t), cudaHostAllocMapped));
   SPG_CUDA(ctx.get(), cudaHostGetDevicePointer((void**)&ctx->h_stage_dev, ctx->h_stage, 0));
   ctx->tuning = default_tuning();
+  SPG_CUDA(ctx.get(), scratch_acquire(device, &ctx->scratch));
   *out = ctx.release();
   return SPG_OK;
 }
@@ -981,7 +1049,10 @@ spg_status spg_destroy(spg_ctx* ctx) {
     cudaStreamSynchronize(ctx->copy_stream);
     cudaStreamDestroy(ctx->copy_stream);
   }
+  cudaEventDestroy(ctx->ev_start);
+  cudaEventDestroy(ctx->ev_end);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
+  scratch_release(ctx->device);
   delete ctx;
   return SPG_OK;
 }
@@ -1013,7 +1084,6 @@ spg_status spg_multiply(spg_ctx* ctx, const spg_csr* A, const spg_csr* B, spg_cs
     report->rows = A->rows;
   }
   const int launches0 = ctx->launches;
-  StageTimer outer(ctx, false);
   DevMat dA, dB;
   SPG_TRY(prepare_matrix(ctx, A, dA, !o.skip_validation));
   // C = A*A through one descriptor: prepared (uploaded) once
@@ -1040,11 +1110,7 @@ spg_status spg_multiply(spg_ctx* ctx, const spg_csr* A, const spg_csr* B, spg_cs
     *C = dev_c;
   }
   if (report) {
-    outer.finish(nullptr);
     report->kernel_launches = ctx->launches - launches0;
-    // whole-call device time, including uploads and the host copy
-    float ms = 0.f;
-    (void)ms;
   }
   return SPG_OK;
 }
@@ -1330,9 +1396,9 @@ spg_status spg_csr_copy(spg_ctx* ctx, const spg_csr* src, int32_t location, spg_
   } else {
     d.owner = 1;
     DevBuf a, b, c;
-    SPG_TRY(a.alloc(ctx, std::max<size_t>(rpb, 4)));
-    SPG_TRY(b.alloc(ctx, std::max<size_t>(nb, 4)));
-    SPG_TRY(c.alloc(ctx, std::max<size_t>(nb, 4)));
+    SPG_TRY(a.alloc_result(ctx, std::max<size_t>(rpb, 4)));
+    SPG_TRY(b.alloc_result(ctx, std::max<size_t>(nb, 4)));
+    SPG_TRY(c.alloc_result(ctx, std::max<size_t>(nb, 4)));
     d.row_ptr = a.release();
     d.col_idx = (int32_t*)b.release();
     d.val = (float*)c.release();

@@ -21,7 +21,9 @@ struct spg_ctx {
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;  // device-to-host copies overlapped with compute (created on first use)
   cudaStream_t upload_stream = nullptr;  // host-to-device copies of input row chunks (created on first use)
-  cudaMemPool_t pool = nullptr;
+  cudaMemPool_t pool = nullptr;     // results (the device's default pool)
+  cudaMemPool_t scratch = nullptr;  // a call's work memory (shared by the device's contexts)
+  cudaEvent_t ev_start = nullptr, ev_end = nullptr;  // StageTimer's
   std::string last_error;
   std::string gpu_name;
   spg_tuning tuning{};
@@ -60,15 +62,21 @@ spg_status cuda_status(spg_ctx* ctx, cudaError_t e, const char* what);
     if (_s != SPG_OK) return _s;        \
   } while (0)
 
-// Stream-ordered device allocation from the context's pool; released at
-// scope exit (stream-ordered free) unless release() is called.
+// Stream-ordered device allocation; released at scope exit (stream-ordered
+// free) unless release() is called.  alloc: work memory, from the scratch
+// pool; alloc_result: memory that a caller may keep, from the device's default
+// pool.  Apart, each call finds the blocks the last one freed: in one pool the
+// scratch of a call was cut from the results' blocks and the driver remapped
+// gigabytes to make room for the next result (R-MAT 18, 10 GB of C: calls of
+// 36 ms took 45 to 3,000 ms).
 class DevBuf {
  public:
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { reset(); }
-  spg_status alloc(spg_ctx* ctx, size_t bytes);
+  spg_status alloc(spg_ctx* ctx, size_t bytes) { return alloc_from(ctx, bytes, ctx->scratch); }
+  spg_status alloc_result(spg_ctx* ctx, size_t bytes) { return alloc_from(ctx, bytes, ctx->pool); }
   void reset();
   void* release() {
     void* p = ptr_;
@@ -82,11 +90,45 @@ class DevBuf {
   void* get() const { return ptr_; }
 
  private:
+  spg_status alloc_from(spg_ctx* ctx, size_t bytes, cudaMemPool_t pool);
   spg_ctx* ctx_ = nullptr;
   void* ptr_ = nullptr;
 };
 
-inline LaunchCtx launch_ctx(const spg_ctx* ctx) { return LaunchCtx{ctx->stream, ctx->sms}; }
+// Part of a DevBuf; several arrays of one call share an allocation.
+struct DevSlice {
+  void* ptr = nullptr;
+  template <typename T>
+  T* as() const {
+    return static_cast<T*>(ptr);
+  }
+  void* get() const { return ptr; }
+};
+
+// Lays arrays out behind one another, each 256-byte aligned; then one
+// allocation holds them all.
+class DevLayout {
+ public:
+  void add(DevSlice* s, size_t bytes) {
+    parts_[n_] = s;
+    at_[n_++] = size_;
+    size_ += (bytes + 255) / 256 * 256;
+  }
+  spg_status alloc(spg_ctx* ctx, DevBuf& buf) {
+    const spg_status st = buf.alloc(ctx, size_);
+    if (st == SPG_OK)
+      for (int i = 0; i < n_; ++i) parts_[i]->ptr = buf.as<char>() + at_[i];
+    return st;
+  }
+
+ private:
+  static constexpr int kMax = 8;
+  DevSlice* parts_[kMax];
+  size_t at_[kMax], size_ = 0;
+  int n_ = 0;
+};
+
+inline LaunchCtx launch_ctx(const spg_ctx* ctx) { return LaunchCtx{ctx->stream, ctx->sms, ctx->device}; }
 
 // Enqueues a copy of `bytes` (a multiple of 4) device bytes into the mapped
 // staging words at host_dst (inside ctx->h_stage); valid after the next
@@ -149,8 +191,6 @@ class StageTimer {
  private:
   spg_ctx* ctx_;
   bool on_;
-  cudaEvent_t start_ = nullptr;
-  cudaEvent_t end_ = nullptr;
   std::vector<std::pair<int, cudaEvent_t>> marks_;
 };
 

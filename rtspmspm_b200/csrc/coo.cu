@@ -307,9 +307,9 @@ spg_status coo_to_csr_device(spg_ctx* ctx, int64_t rows, int64_t cols, int64_t n
     if (f & kFlagBadIndex) return fail(ctx, SPG_ERR_INVALID_ARG, "COO entry outside [0, rows) x [0, cols)");
   }
   DevBuf col, val, rp;
-  SPG_TRY(col.alloc(ctx, (size_t)m * 4));
-  SPG_TRY(val.alloc(ctx, (size_t)m * 4));
-  SPG_TRY(rp.alloc(ctx, (size_t)(rows + 1) * 8));
+  SPG_TRY(col.alloc_result(ctx, (size_t)m * 4));
+  SPG_TRY(val.alloc_result(ctx, (size_t)m * 4));
+  SPG_TRY(rp.alloc_result(ctx, (size_t)(rows + 1) * 8));
   if (n > 0)
     k_fold_runs<<<(unsigned)nfold, kFoldThreads, 0, lc.stream>>>(kin, vin, n, runs.as<int64_t>(), m, rows,
                                                                  col.as<int32_t>(), val.as<float>(), rp.as<int64_t>());

@@ -50,7 +50,7 @@ spg_status multiply_cusparse(spg_ctx* ctx, const DevMat& A, const DevMat& B, spg
   DevBuf arp, brp, crp;
   SPG_TRY(arp.alloc(ctx, (size_t)(A.view.rows + 1) * 4));
   SPG_TRY(brp.alloc(ctx, (size_t)(B.view.rows + 1) * 4));
-  SPG_TRY(crp.alloc(ctx, (size_t)(A.view.rows + 1) * 4));
+  SPG_TRY(crp.alloc_result(ctx, (size_t)(A.view.rows + 1) * 4));
   launch_narrow_rp(A.view.rp, A.view.rows + 1, arp.as<int32_t>(), lc);
   launch_narrow_rp(B.view.rp, B.view.rows + 1, brp.as<int32_t>(), lc);
   SpHandle H;
@@ -101,8 +101,8 @@ spg_status multiply_cusparse(spg_ctx* ctx, const DevMat& A, const DevMat& B, spg
   int64_t cr = 0, cc = 0, cn = 0;
   SPG_SPARSE(ctx, cusparseSpMatGetSize(H.c, &cr, &cc, &cn));
   DevBuf ccol, cval;
-  SPG_TRY(ccol.alloc(ctx, (size_t)cn * 4));
-  SPG_TRY(cval.alloc(ctx, (size_t)cn * 4));
+  SPG_TRY(ccol.alloc_result(ctx, (size_t)cn * 4));
+  SPG_TRY(cval.alloc_result(ctx, (size_t)cn * 4));
   SPG_SPARSE(ctx, cusparseCsrSetPointers(H.c, crp.get(), ccol.get(), cval.get()));
   SPG_SPARSE(ctx, cusparseSpGEMM_copy(H.h, op, op, &alpha, H.a, H.b, &beta, H.c, CUDA_R_32F, alg, H.g));
   std::memset(C, 0, sizeof *C);

@@ -1451,6 +1451,63 @@ static int grid_for(int64_t work, int threads, int per_thread, int max_blocks) {
   return (int)b;
 }
 
+// CTA size (warps, 1..max_w) giving a kernel the most resident warps per SM
+// for `smem_per_warp` bytes of dynamic shared memory per warp; ties go to
+// the larger CTA.  Register and shared-memory granularity make this differ
+// by table size: 2^9-slot numeric tables (6 KB a warp) reach 36 warps with
+// 6-warp CTAs but 32 with 8-warp ones; 2^11-slot symbolic tables (8 KB) fit
+// 28 warps with 7-warp CTAs and 24 with 8-warp ones.
+template <typename Kernel>
+static int auto_wpb(Kernel kernel, size_t smem_per_warp, int max_w) {
+  int best_w = 1, best = -1;
+  for (int w = 1; w <= max_w; ++w) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, w * 32, (size_t)w * smem_per_warp) !=
+        cudaSuccess)
+      continue;
+    if (per_sm * w >= best) {
+      best = per_sm * w;
+      best_w = w;
+    }
+  }
+  return best_w;
+}
+
+// Warps a CTA and CTAs an SM of a launch.
+struct LaunchShape {
+  int wpb, per_sm;
+};
+
+// The shape of a kernel instantiation and the shared memory it may ask for.
+// wpb <= 0 selects auto_wpb; its answer is computed once (the first device
+// that launches the kernel decides; all devices here are alike) and the
+// shared-memory limit is raised once a device, since the driver calls behind
+// both cost a small product as much as its launches.
+class LaunchCache {
+ public:
+  template <typename Kernel>
+  LaunchShape get(Kernel kernel, int wpb, size_t smem_per_warp, int max_w, int device) {
+    const uint64_t bit = device < 64 ? uint64_t(1) << device : 0;
+    if (!(raised_.load(std::memory_order_acquire) & bit)) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess)
+        raised_.fetch_or(bit, std::memory_order_release);
+    }
+    int packed = wpb > 0 ? 0 : shape_.load(std::memory_order_relaxed);
+    if (packed == 0) {
+      const int w = wpb > 0 ? std::min(wpb, max_w) : auto_wpb(kernel, smem_per_warp, max_w);
+      int per_sm = 0;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, w * 32, (size_t)w * smem_per_warp);
+      packed = w | (std::max(1, per_sm) << 8);
+      if (wpb <= 0) shape_.store(packed, std::memory_order_relaxed);
+    }
+    return LaunchShape{packed & 0xff, packed >> 8};
+  }
+
+ private:
+  std::atomic<uint64_t> raised_{0};
+  std::atomic<int> shape_{0};
+};
+
 void launch_widen_rp(const int32_t* in, int64_t n, int64_t* out, const LaunchCtx& lc) {
   k_widen_rp<<<grid_for(n, 256, 1, lc.sms * 8), 256, 0, lc.stream>>>(in, n, out);
 }
@@ -1474,13 +1531,15 @@ void launch_row_products(const DCsr& A, const DCsr& B, int64_t* prod, const Laun
 void launch_small_count(const DCsr& A, const DCsr& B, int64_t* prod, int64_t* nnz, unsigned long long* stop,
                         int* flags, const LaunchCtx& lc) {
   if (A.rows == 0) return;
-  const size_t smem = (size_t)kSmallCountWarps * (1u << kSmallLogT) * 4;
-  int per_sm = 0;
-  if (B.rp32) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small_count<true>, kSmallCountWarps * 32, smem);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small_count<false>, kSmallCountWarps * 32, smem);
-  const int blocks = grid_for(A.rows, kSmallCountWarps, 1, lc.sms * (per_sm < 1 ? 1 : per_sm));
-  if (B.rp32) k_small_count<true><<<blocks, kSmallCountWarps * 32, smem, lc.stream>>>(A, B, prod, nnz, stop, flags);
-  else k_small_count<false><<<blocks, kSmallCountWarps * 32, smem, lc.stream>>>(A, B, prod, nnz, stop, flags);
+  const size_t per_warp = (size_t)(1u << kSmallLogT) * 4;
+  static LaunchCache cache[2];
+  const LaunchShape sh = B.rp32
+                             ? cache[1].get(k_small_count<true>, 0, per_warp, kSmallCountWarps, lc.device)
+                             : cache[0].get(k_small_count<false>, 0, per_warp, kSmallCountWarps, lc.device);
+  const int blocks = grid_for(A.rows, sh.wpb, 1, lc.sms * sh.per_sm);
+  const size_t smem = sh.wpb * per_warp;
+  if (B.rp32) k_small_count<true><<<blocks, sh.wpb * 32, smem, lc.stream>>>(A, B, prod, nnz, stop, flags);
+  else k_small_count<false><<<blocks, sh.wpb * 32, smem, lc.stream>>>(A, B, prod, nnz, stop, flags);
 }
 
 void launch_small_scan(int64_t* nnz, const int64_t* prod, int64_t rows, int32_t* rp32, int32_t* row_list,
@@ -1551,53 +1610,14 @@ static int wpb_for(int log_t, int wpb) {
   return std::max(1, std::min(wpb, lim));
 }
 
-// CTA size (warps, 1..max_w) giving a kernel the most resident warps per SM
-// for `smem_per_warp` bytes of dynamic shared memory per warp; ties go to
-// the larger CTA.  Register and shared-memory granularity make this differ
-// by table size: 2^9-slot numeric tables (6 KB a warp) reach 36 warps with
-// 6-warp CTAs but 32 with 8-warp ones; 2^11-slot symbolic tables (8 KB) fit
-// 28 warps with 7-warp CTAs and 24 with 8-warp ones.
-template <typename Kernel>
-static int auto_wpb(Kernel kernel, size_t smem_per_warp, int max_w) {
-  int best_w = 1, best = -1;
-  for (int w = 1; w <= max_w; ++w) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, w * 32, (size_t)w * smem_per_warp) !=
-        cudaSuccess)
-      continue;
-    if (per_sm * w >= best) {
-      best = per_sm * w;
-      best_w = w;
-    }
-  }
-  return best_w;
-}
-
-// wpb <= 0 selects auto_wpb, computed once per kernel instantiation (the
-// first device that launches it decides; all devices here are alike).
-template <typename Kernel>
-static int resolve_wpb(int wpb, std::atomic<int>& cache, Kernel kernel, size_t smem_per_warp, int max_w) {
-  if (wpb > 0) return wpb;
-  int w = cache.load(std::memory_order_relaxed);
-  if (w <= 0) {
-    w = auto_wpb(kernel, smem_per_warp, max_w);
-    cache.store(w, std::memory_order_relaxed);
-  }
-  return w;
-}
-
 template <int LOGT, bool R32>
 static void sym_warp_one(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, int64_t* nnz, int* flags,
                          const LaunchCtx& lc, int wpb) {
-  cudaFuncSetAttribute(k_sym_warp<LOGT, R32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  static std::atomic<int> auto_w{0};
-  wpb = resolve_wpb(wpb, auto_w, k_sym_warp<LOGT, R32>, (size_t)(1 << LOGT) * sizeof(int32_t), 8);
-  const size_t smem = (size_t)wpb * (1 << LOGT) * sizeof(int32_t);
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sym_warp<LOGT, R32>, wpb * 32, smem);
-  if (per_sm < 1) per_sm = 1;
-  const int blocks = grid_for(nrows, wpb, 1, lc.sms * per_sm);
-  k_sym_warp<LOGT, R32><<<blocks, wpb * 32, smem, lc.stream>>>(A, B, rows, nrows, nnz, flags);
+  static LaunchCache cache;
+  const size_t per_warp = (size_t)(1 << LOGT) * sizeof(int32_t);
+  const LaunchShape sh = cache.get(k_sym_warp<LOGT, R32>, wpb, per_warp, wpb > 0 ? 16 : 8, lc.device);
+  const int blocks = grid_for(nrows, sh.wpb, 1, lc.sms * sh.per_sm);
+  k_sym_warp<LOGT, R32><<<blocks, sh.wpb * 32, sh.wpb * per_warp, lc.stream>>>(A, B, rows, nrows, nnz, flags);
 }
 
 void launch_sym_warp(int log_t, const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, int64_t* nnz,
@@ -1677,15 +1697,11 @@ void launch_sym_dense(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t
 template <int LOGT, bool R32>
 static void num_warp_one(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, const int64_t* c_rp,
                          int32_t* c_col, float* c_val, int* flags, const LaunchCtx& lc, int wpb, const EscArgs& esc) {
-  cudaFuncSetAttribute(k_num_warp<LOGT, R32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  static std::atomic<int> auto_w{0};
-  wpb = resolve_wpb(wpb, auto_w, k_num_warp<LOGT, R32>, (size_t)numeric_words<LOGT>() * 4, wpb_for(LOGT, 8));
-  const size_t smem = (size_t)wpb * numeric_words<LOGT>() * 4;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_num_warp<LOGT, R32>, wpb * 32, smem);
-  if (per_sm < 1) per_sm = 1;
-  const int blocks = grid_for(nrows, wpb, 1, lc.sms * per_sm);
-  k_num_warp<LOGT, R32><<<blocks, wpb * 32, smem, lc.stream>>>(A, B, rows, nrows, c_rp, c_col, c_val, esc.prod,
+  static LaunchCache cache;
+  const size_t per_warp = (size_t)numeric_words<LOGT>() * 4;
+  const LaunchShape sh = cache.get(k_num_warp<LOGT, R32>, wpb, per_warp, wpb_for(LOGT, wpb > 0 ? 16 : 8), lc.device);
+  const int blocks = grid_for(nrows, sh.wpb, 1, lc.sms * sh.per_sm);
+  k_num_warp<LOGT, R32><<<blocks, sh.wpb * 32, sh.wpb * per_warp, lc.stream>>>(A, B, rows, nrows, c_rp, c_col, c_val, esc.prod,
                                                                 esc.min_prod, flags);
 }
 
@@ -1711,16 +1727,12 @@ static void num_warp_learned_one(const DCsr& A, const DCsr& B, const int32_t* ro
                                  const int64_t* cap, const int64_t* slab_off, int32_t* slab_col, float* slab_val,
                                  int64_t* nnz_out, int32_t* retry_rows, unsigned long long* retry_count, int* flags,
                                  const LaunchCtx& lc, int wpb, const EscArgs& esc) {
-  cudaFuncSetAttribute(k_num_warp_learned<LOGT, R32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  static std::atomic<int> auto_w{0};
-  wpb = resolve_wpb(wpb, auto_w, k_num_warp_learned<LOGT, R32>, (size_t)numeric_words<LOGT>() * 4,
-                    wpb_for(LOGT, 8));
-  const size_t smem = (size_t)wpb * numeric_words<LOGT>() * 4;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_num_warp_learned<LOGT, R32>, wpb * 32, smem);
-  if (per_sm < 1) per_sm = 1;
-  const int blocks = grid_for(nrows, wpb, 1, lc.sms * per_sm);
-  k_num_warp_learned<LOGT, R32><<<blocks, wpb * 32, smem, lc.stream>>>(A, B, rows, nrows, cap, slab_off, slab_col,
+  static LaunchCache cache;
+  const size_t per_warp = (size_t)numeric_words<LOGT>() * 4;
+  const LaunchShape sh =
+      cache.get(k_num_warp_learned<LOGT, R32>, wpb, per_warp, wpb_for(LOGT, wpb > 0 ? 16 : 8), lc.device);
+  const int blocks = grid_for(nrows, sh.wpb, 1, lc.sms * sh.per_sm);
+  k_num_warp_learned<LOGT, R32><<<blocks, sh.wpb * 32, sh.wpb * per_warp, lc.stream>>>(A, B, rows, nrows, cap, slab_off, slab_col,
                                                                         slab_val, nnz_out, retry_rows, retry_count,
                                                                         esc.prod, esc.min_prod, flags);
 }
@@ -1756,13 +1768,10 @@ static void num_esc_one(int bin, const DCsr& A, const DCsr& B, const int32_t* ro
   const int words = (3 * esc_bin_products(bin - kBinEsc) + kEscBuckets + 3) / 4 * 4;
   const size_t per_warp = (size_t)words * 4;
   const int fit = std::min(8, (int)(200 * 1024 / per_warp));
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  static std::atomic<int> auto_w[kNumEscBins];
-  const int w = std::min(fit, resolve_wpb(wpb, auto_w[bin - kBinEsc], kernel, per_warp, fit));
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, w * 32, w * per_warp);
-  const int blocks = grid_for(nrows, w, 1, lc.sms * std::max(1, per_sm));
-  kernel<<<blocks, w * 32, w * per_warp, lc.stream>>>(A, B, rows, nrows, prod, words, off, out_col, out_val, cap, nnz,
+  static LaunchCache cache[kNumEscBins];
+  const LaunchShape sh = cache[bin - kBinEsc].get(kernel, wpb, per_warp, fit, lc.device);
+  const int blocks = grid_for(nrows, sh.wpb, 1, lc.sms * sh.per_sm);
+  kernel<<<blocks, sh.wpb * 32, sh.wpb * per_warp, lc.stream>>>(A, B, rows, nrows, prod, words, off, out_col, out_val, cap, nnz,
                                                       retry, retry_count, flags);
 }
 

@@ -84,6 +84,7 @@ inline BinParams without_block_bins(BinParams bp) {
 struct LaunchCtx {
   cudaStream_t stream;
   int sms;
+  int device;
 };
 
 void launch_widen_rp(const int32_t* in, int64_t n, int64_t* out, const LaunchCtx& lc);
