@@ -159,6 +159,7 @@ BinParams bin_params(const spg_tuning& t) {
   bp.block_min = (int64_t)t.block_min_nnz;
   bp.blk_small_cap = ((int64_t)1 << kBlkLogSmallT) / 2;
   bp.blk_large_cap = ((int64_t)1 << kBlkLogLargeT) / 2;
+  bp.esc_cap = std::min(bp.warp_cap, bp.block_min);
   return bp;
 }
 

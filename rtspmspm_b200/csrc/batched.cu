@@ -317,6 +317,41 @@ __global__ void __launch_bounds__(kBlkThreads, MINB) k_batch_queue(const BatchMa
   }
 }
 
+// Expand-sort-fold rows of one bin of all products, a warp a row, `words` words
+// of shared memory each.  Rows of mostly distinct products: in the queues they
+// took the slots of their output's tables (12 KB at 938 products, a whole CTA
+// and its barriers above), here 3 words a product.
+template <bool LEARNED>
+__global__ void __launch_bounds__(kBlkThreads) k_batch_esc(const BatchMat* mats, const int32_t* row_mat,
+                                                           const int32_t* lists, const int64_t* bin_off, int bin,
+                                                           int words, const int64_t* prod, int64_t* nnz,
+                                                           const int64_t* gscan, int32_t* c_col, float* c_val,
+                                                           LearnedOut lo, int* flags) {
+  extern __shared__ int32_t sm_q[];
+  int32_t* buf = sm_q + (size_t)(threadIdx.x >> 5) * words;
+  const int64_t last = bin_off[bin + 1];
+  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t i = bin_off[bin] + gw; i < last; i += nw) {
+    const int64_t g = lists[i];
+    const BatchMat& M = mats[row_mat[g]];
+    const int32_t r = (int32_t)(g - M.row_start);
+    const int64_t off = LEARNED ? lo.slab_off[g] : M.c_base + (gscan[g] - gscan[M.row_start]);
+    const int64_t want = LEARNED ? lo.cap[g] : gscan[g + 1] - gscan[g];
+    const int n = esc_row<true>(M.A, M.B, r, (int)prod[g], buf, want, (LEARNED ? lo.slab_col : c_col) + off,
+                                (LEARNED ? lo.slab_val : c_val) + off);
+    if (lane_id() == 0) {
+      if (LEARNED) {
+        const bool over = n < 0 || n > want;
+        nnz[g] = over ? -1 : n;
+        if (over) lo.retry[atomicAdd(lo.retry_count, 1ull)] = (int32_t)g;
+      } else if (n != want) {
+        raise_flag(flags, kFlagCountDiff);
+      }
+    }
+  }
+}
+
 // Per-product row pointers (rebased to 0) and nnz.
 __global__ void k_batch_finalize(const BatchMat* mats, int n, const int32_t* row_mat, int64_t R, const int64_t* gscan,
                                  int64_t* rp_out, int64_t* nnz_m) {
@@ -479,7 +514,14 @@ const void* queue_dispatch(int which, bool learned, const QueueArgs* a, int grid
   }
 }
 
+// Warps a CTA of an expand-sort-fold bin: tens of KB a CTA, so that the last
+// CTA an SM holds leaves little of it unused.
+int esc_warps(int i) { return i <= 1 ? 8 : i == 2 ? 3 : i == 3 ? 2 : 1; }
+size_t esc_smem(int i) { return (size_t)esc_warps(i) * esc_bin_words(esc_bin_products(i)) * 4; }
+
 struct BatchPlan {
+  int64_t max_cols = 1;                 // most columns of a batched product
+  int esc_grid[2][kNumEscBins] = {};    // CTAs of each expand-sort-fold launch (plain, learned form)
   std::vector<uintptr_t> key;
   int n = 0;
   int64_t R = 0;
@@ -613,6 +655,25 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
     queue_dispatch(which, learned, &a, p->grid[learned ? 1 : 0][which], queue_smem(which), lc.stream);
     launches += 2;
   };
+  EscArgs esc;
+  esc.prod = p->prod;
+  esc.min_prod = p->tune.esc_min_prod < 0 ? 0 : (p->tune.esc_min_prod == 0 ? kEscMinProd : p->tune.esc_min_prod);
+  auto run_esc = [&](bool learned) {
+    if (esc.min_prod == 0) return;
+    for (int i = kNumEscBins - 1; i >= 0; --i) {
+      const int threads = esc_warps(i) * 32, grid = p->esc_grid[learned ? 1 : 0][i];
+      const int words = esc_bin_words(esc_bin_products(i));
+      if (learned)
+        k_batch_esc<true><<<grid, threads, esc_smem(i), lc.stream>>>(p->d_mats, p->row_mat, p->lists, offsets,
+                                                                     kBinEsc + i, words, p->prod, p->nnz, p->nnz,
+                                                                     p->c_col, p->c_val, lo, ctx->d_flags);
+      else
+        k_batch_esc<false><<<grid, threads, esc_smem(i), lc.stream>>>(p->d_mats, p->row_mat, p->lists, offsets,
+                                                                      kBinEsc + i, words, p->prod, p->nnz, p->nnz,
+                                                                      p->c_col, p->c_val, lo, ctx->d_flags);
+      ++launches;
+    }
+  };
   auto exact_stages = [&](const int64_t* sym_key) {
     launch_binning(sym_key, R, INT64_MAX, kBinSymbolic, p->bp_sym, p->bin_of_row, counts, offsets, cursors,
                    p->lists, lc);
@@ -622,10 +683,11 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
   };
   if (!p->learned) {
     exact_stages(p->bound);
-    launch_binning(p->nnz, R, INT64_MAX, kBinNumeric, p->bp_num, p->bin_of_row, counts, offsets, cursors, p->lists,
-                   lc);
+    launch_binning(p->nnz, R, p->max_cols, kBinNumeric, p->bp_num, p->bin_of_row, counts, offsets, cursors, p->lists,
+                   lc, esc);
     launch_excl_scan(p->nnz, R, p->nnz, p->scan_tmp, lc);
     launches += 7;
+    run_esc(false);
     run_queue(kQNumLarge, false);
     run_queue(kQNumMid, false);
     run_queue(kQNumSmall, false);
@@ -634,10 +696,11 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
     cudaMemsetAsync(p->need, 0, (size_t)std::max<int64_t>(R, 1), lc.stream);
     launch_learned_plan_batch(p->d_mats, p->row_mat, R, ctx->mlp_w16, p->tune.predict_margin, p->tune.predict_slack,
                               kBatchMaxBound, p->force_overflow, p->prod, p->cap, p->need, p->lcount, lc);
-    launch_binning(p->cap, R, INT64_MAX, kBinLearned, p->bp_lrn, p->bin_of_row, counts, offsets, cursors, p->lists,
-                   lc);
+    launch_binning(p->cap, R, p->max_cols, kBinLearned, p->bp_lrn, p->bin_of_row, counts, offsets, cursors, p->lists,
+                   lc, esc);
     launch_excl_scan(p->cap, R, p->slab_off, p->scan_tmp, lc);
     launches += 8;
+    run_esc(true);
     run_queue(kQNumLarge, true);
     run_queue(kQNumMid, true);
     run_queue(kQNumSmall, true);
@@ -701,6 +764,7 @@ spg_status build_plan(spg_ctx* ctx, int n, const spg_csr* A, const spg_csr* B, c
   bn.block_min = bn.warp_cap;
   bn.blk_small_cap = kBatchMaxBound;
   bn.blk_large_cap = 0;
+  bn.esc_cap = kBatchMaxBound;
   p->bp_num = bn;
   // learned binning: as numeric, at the learned load factor
   BinParams bl = bn;
@@ -793,6 +857,7 @@ spg_status build_plan(spg_ctx* ctx, int n, const spg_csr* A, const spg_csr* B, c
       M.A.rows = 0;
     } else {
       p->batched.push_back(m);
+      p->max_cols = std::max(p->max_cols, M.B.cols);
     }
     M.c_base = cbase;
     M.rp_base = rpbase;
@@ -834,6 +899,13 @@ spg_status build_plan(spg_ctx* ctx, int n, const spg_csr* A, const spg_csr* B, c
       int per_sm = 0;
       SPG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kBlkThreads, smem));
       p->grid[form][w] = ctx->sms * std::max(1, per_sm);
+    }
+    for (int i = 0; i < kNumEscBins; ++i) {
+      const void* k = form == 1 ? (const void*)k_batch_esc<true> : (const void*)k_batch_esc<false>;
+      SPG_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+      int per_sm = 0;
+      SPG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, esc_warps(i) * 32, esc_smem(i)));
+      p->esc_grid[form][i] = ctx->sms * std::max(1, per_sm);
     }
   }
   if (p->learned) {

@@ -147,7 +147,7 @@ __device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const
   }
   if (key <= 0) return kBinEmpty;
   const bool warp_ok = key <= bp.warp_cap;
-  if (warp_ok && key <= bp.block_min && esc_wanted(prod, key, esc_min, esc_bin_products(kNumEscBins - 1)) &&
+  if (key <= bp.esc_cap && esc_wanted(prod, key, esc_min, esc_bin_products(kNumEscBins - 1)) &&
       ceil_log2_i64(cols) + ceil_log2_i64(prod) <= 31) {
     int b = 0;
     while (prod > esc_bin_products(b)) ++b;
@@ -1765,7 +1765,7 @@ static void num_esc_one(int bin, const DCsr& A, const DCsr& B, const int32_t* ro
                         int64_t* nnz, int32_t* retry, unsigned long long* retry_count, int* flags,
                         const LaunchCtx& lc, int wpb) {
   auto kernel = k_num_esc<R32, LEARNED>;
-  const int words = (3 * esc_bin_products(bin - kBinEsc) + kEscBuckets + 3) / 4 * 4;
+  const int words = esc_bin_words(esc_bin_products(bin - kBinEsc));
   const size_t per_warp = (size_t)words * 4;
   const int fit = std::min(8, (int)(200 * 1024 / per_warp));
   static LaunchCache cache[kNumEscBins];

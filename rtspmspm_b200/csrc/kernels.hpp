@@ -23,6 +23,7 @@ constexpr int kBinDense = 9;   // symbolic: CTA bitmap over the column span; num
 constexpr int kBinEsc = 10;
 constexpr int kNumEscBins = 5;
 // Largest products of bin kBinEsc + i.
+// (32-bit words of shared memory a warp of it takes: esc_bin_words, warp_row.cuh)
 constexpr int esc_bin_products(int i) { return i == 0 ? 320 : i == 1 ? 640 : i == 2 ? 1152 : i == 3 ? 2048 : 4010; }
 // Symbolic: rows with a bitmap of their column span (span.cu), by its words.
 constexpr int kBinSpan = kBinEsc;
@@ -70,6 +71,7 @@ struct BinParams {
   int64_t block_min;
   int64_t blk_small_cap;
   int64_t blk_large_cap;
+  int64_t esc_cap;     // most entries of a row in the expand-sort-fold bins
 };
 
 // BinParams with the CTA-wide numeric bins turned off (paths that only
@@ -78,6 +80,7 @@ inline BinParams without_block_bins(BinParams bp) {
   bp.block_min = INT64_MAX;
   bp.blk_small_cap = 0;
   bp.blk_large_cap = 0;
+  bp.esc_cap = bp.warp_cap;
   return bp;
 }
 

@@ -495,6 +495,9 @@ constexpr int kEscCrowd = 64;
 // word buffers, the values and the bucket counts.
 __host__ __device__ __forceinline__ int esc_capacity(int words) { return (words - kEscBuckets) / 3; }
 
+// Words of a warp of an expand-sort-fold bin holding rows of up to P products.
+constexpr int esc_bin_words(int P) { return (3 * P + kEscBuckets + 3) / 4 * 4; }
+
 // True when a row of `prod` products and at least `out` output entries
 // (its exact count, or the learned capacity) takes the expand-sort-fold
 // path: esc_min > 0 (0 turns it off), prod in [esc_min, cap] and at least
