@@ -155,11 +155,16 @@ BinParams bin_params(const spg_tuning& t) {
   // block_min_nnz entries, when set: measured slower than the warp tables
   // and heavy-row tiles they replace on R-MAT scale 17 (plain 29.8 against
   // 21.6 ms) and even on scale 20 (518 against 516 ms), so off by default
-  if (t.block_min_nnz <= 0) return without_block_bins(bp);
+  if (t.block_min_nnz <= 0) {
+    bp = without_block_bins(bp);
+    if (t.heavy_path == 0) bp.heavy_min = std::min(kHeavyMin, bp.warp_cap);
+    return bp;
+  }
   bp.block_min = (int64_t)t.block_min_nnz;
   bp.blk_small_cap = ((int64_t)1 << kBlkLogSmallT) / 2;
   bp.blk_large_cap = ((int64_t)1 << kBlkLogLargeT) / 2;
   bp.esc_cap = std::min(bp.warp_cap, bp.block_min);
+  bp.heavy_min = INT64_MAX;
   return bp;
 }
 
@@ -363,6 +368,24 @@ struct Pipeline {
     return SPG_OK;
   }
 
+  // Big rows of the last symbolic binning, and whether their bitmaps fit the
+  // budget.
+  int64_t big_rows() const { return bin_size(kBinBlock) + bin_size(kBinDense); }
+  bool bitmaps_fit() const {
+    const size_t bytes = (size_t)big_rows() * (size_t)bitmap_stride() * 4;
+    return tune.heavy_path == 0 && bitmap_stride() <= kDenseWindowWords && bytes <= kBitmapMaxBytes && room_for(bytes, 8);
+  }
+
+  // True when `bytes` are less than a part of the device's free memory.  The
+  // driver's answer can take a millisecond, so a few tens of MB are not asked
+  // about.
+  static bool room_for(size_t bytes, size_t part) {
+    if (bytes <= (size_t(64) << 20)) return true;
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    return bytes < free_b / part;
+  }
+
   void bin(const int64_t* key, int mode, const EscArgs& esc = EscArgs{}) {
     launch_binning(key, rows, cols, mode, bp, bin_of_row.as<uint8_t>(), counts(), offsets(), cursors(),
                    lists.as<int32_t>(), lc, esc, span.as<int32_t>());
@@ -390,6 +413,12 @@ struct Pipeline {
   spg_status symbolic(const int64_t* key) {
     bin(key, kBinSymbolic);
     SPG_TRY(fetch_offsets());
+    if (big_rows() > 0 && bp.heavy_min < bp.warp_cap && !bitmaps_fit()) {
+      // only rows with a stored bitmap gain from leaving the warp tables early
+      bp.heavy_min = INT64_MAX;
+      bin(key, kBinSymbolic);
+      SPG_TRY(fetch_offsets());
+    }
     for (int b = kBinSpan; b < kBinSpan + kNumSpanBins; ++b) {
       if (bin_size(b) == 0) continue;
       launch_sym_span(b, A.view, B.view, bin_rows(b), bin_size(b), nnz.as<int64_t>(), ctx->d_flags, lc);
@@ -411,12 +440,7 @@ struct Pipeline {
       // when one bitmap window holds a row and the budget all big rows'
       // bitmaps, every big row takes the bitmap kernel and leaves its bitmap
       // for the units (which else walk their products once more for it)
-      const size_t bitmap_bytes = (size_t)nbig * (size_t)bitmap_stride() * 4;
-      size_t free_b = 0, total_b = 0;
-      cudaMemGetInfo(&free_b, &total_b);
-      if (tune.heavy_path == 0 && bitmap_stride() <= kDenseWindowWords && bitmap_bytes <= kBitmapMaxBytes &&
-          bitmap_bytes < free_b / 8)
-        SPG_TRY(bitmap.alloc(ctx, bitmap_bytes));
+      if (bitmaps_fit()) SPG_TRY(bitmap.alloc(ctx, (size_t)nbig * (size_t)bitmap_stride() * 4));
       if (bitmap.get()) {
         launch_sym_dense(A.view, B.view, bin_rows(kBinBlock), nbig, 0, nnz.as<int64_t>(), big_slot.as<int32_t>(),
                          tile_cnt.as<int32_t>(), ntiles, bitmap.as<uint32_t>(), ctx->d_flags, lc);
@@ -470,15 +494,14 @@ struct Pipeline {
   // scatter over a buffer far larger than L2), and heavy_path 2, tiles that
   // rescan their row with bulk copies of long segments.  *done stays false
   // when the path does not apply (buckets or alignment).
-  spg_status numeric_tiles(const int64_t* c_rp, int32_t* c_col, float* c_val, const int32_t* bidx, size_t free_b,
-                           bool* done) {
+  spg_status numeric_tiles(const int64_t* c_rp, int32_t* c_col, float* c_val, const int32_t* bidx, bool* done) {
     const int64_t nheavy = bin_size(kBinHeavy);
     if (tune.heavy_path == 2 && !bulk_aligned(B.view)) return SPG_OK;
     // the list of non-empty (row, tile) units for the tile kernel, when it
     // fits: rows of wide products touch a small part of their tiles
     const size_t work_bytes = (size_t)nheavy * (size_t)ntiles * 8;
     const bool use_list = tune.heavy_path == 2 && ntiles > 1 && work_bytes <= kWorkListMaxBytes &&
-                          work_bytes < free_b / 4;
+                          room_for(work_bytes, 4);
     DevBuf nz, work;
     if (use_list) SPG_TRY(nz.alloc(ctx, (size_t)(nheavy + 1) * 8));
     launch_tile_offsets(bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles,
@@ -534,20 +557,18 @@ struct Pipeline {
     if (nheavy > 0) {
       // the blocked index reads every row of B
       if (B.complete) SPG_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, B.complete, 0));
-      size_t free_b = 0, total_b = 0;
-      cudaMemGetInfo(&free_b, &total_b);
       // a blocked index of B when it fits the budget (else per-unit binary
       // searches)
       DevBuf bidx;
       const size_t bidx_bytes = (size_t)B.view.rows * (size_t)(ntiles + 1) * 4;
-      const bool use_index = ntiles > 1 && bidx_bytes <= kBlockedIndexMaxBytes && bidx_bytes < free_b / 4;
+      const bool use_index = ntiles > 1 && bidx_bytes <= kBlockedIndexMaxBytes && room_for(bidx_bytes, 4);
       if (use_index) {
         SPG_TRY(bidx.alloc(ctx, bidx_bytes));
         launch_build_blocked_index(B.view, ntiles, bidx.as<int32_t>(), lc);
         ++ctx->launches;
       }
       bool done = false;
-      if (tune.heavy_path != 0) SPG_TRY(numeric_tiles(c_rp, c_col, c_val, bidx.as<int32_t>(), free_b, &done));
+      if (tune.heavy_path != 0) SPG_TRY(numeric_tiles(c_rp, c_col, c_val, bidx.as<int32_t>(), &done));
       if (!done) {
         const int64_t room = heavy_unit_bound(nheavy, ntiles, c_nnz);
         DevBuf units;
@@ -680,7 +701,8 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
   const bool cta_bins = P.bp.blk_large_cap > 0;
   launch_learned_plan(P.A.view, P.B.view, ctx->mlp_w16, P.tune.predict_margin, P.tune.predict_slack,
                       std::max(P.bp.warp_cap, P.bp.blk_large_cap), cta_bins ? 0 : 1, o.force_overflow,
-                      P.prod.as<int64_t>(), cap.as<int64_t>(), need.as<uint8_t>(), ctx->d_counter + 3, lc);
+                      P.prod.as<int64_t>(), cap.as<int64_t>(), need.as<uint8_t>(), ctx->d_counter + 3, lc, P.bp.heavy_min,
+                      P.esc_args(nullptr).min_prod);
   launch_sum(P.prod.as<int64_t>(), rows, ctx->d_counter + 1, lc);
   ctx->launches += 2;
   tm.mark(SPG_STAGE_BINNING);

@@ -118,21 +118,22 @@ __device__ __forceinline__ int ceil_log2_i64(int64_t v) {
 //  mode kBinSymbolic: key = products; bound u = min(key, cols).
 //  mode kBinNumeric:  key = exact nnz.
 //  mode kBinLearned:  key = predicted capacity (already capped by the bound).
-// prod > 0 (numeric, learned): the row's products, of which esc_min or more
+// prod > 0 (numeric, learned; else 0): the row's products, of which esc_min or more
 // with half of them distinct send it to the expand-sort-fold bins when a word
 // holds any column and position of it.
 __device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const BinParams& bp, int64_t prod,
                                       int esc_min, int span) {
+  if (mode == kBinSymbolic) prod = key;
+  const int64_t u = prod <= 0 ? key : prod < cols ? prod : cols;
+  // counting and clearing a span's words (a quarter instruction each) must
+  // not outweigh the products (60 a hash step of 32 saved); small tunings of
+  // the tables keep their rows
+  const bool spanned = span > 0 && span <= span_bin_words(kNumSpanBins - 1) && bp.warp_log_max >= 9 && prod >= 64 &&
+                       u <= bp.warp_cap && span <= 4 * prod;
   if (mode == kBinSymbolic) {
-    int64_t u = key < cols ? key : cols;
     if (u <= 0) return kBinEmpty;
-    // counting and clearing a span's words (a quarter instruction each) must
-    // not outweigh the products (60 a hash step of 32 saved); small tunings of
-    // the tables keep their rows
-    if (span > 0 && span <= span_bin_words(kNumSpanBins - 1) && bp.warp_log_max >= 9 && key >= 64 &&
-        u <= bp.warp_cap && span <= 4 * key)
-      return kBinSpan + (span > span_bin_words(0)) + (span > span_bin_words(1));
-    if (u <= bp.warp_cap) {
+    if (spanned) return kBinSpan + (span > span_bin_words(0)) + (span > span_bin_words(1));
+    if (!big_row(u, cols, bp.warp_cap, bp.heavy_min)) {
       // a row has at most u distinct columns, so a table of 1.25 u slots
       // stays at most 4/5 full, and usually far below (125 columns from
       // 729 products on the stencil: 2^10 slots instead of 2^11 at 2/3)
@@ -147,7 +148,10 @@ __device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const
   }
   if (key <= 0) return kBinEmpty;
   const bool warp_ok = key <= bp.warp_cap;
-  if (key <= bp.esc_cap && esc_wanted(prod, key, esc_min, esc_bin_products(kNumEscBins - 1)) &&
+  // the symbolic pass counted the tiles of the rows it found big
+  const bool heavy = mode == kBinNumeric && key > bp.heavy_min && !spanned &&
+                     big_row(u, cols, bp.warp_cap, bp.heavy_min);
+  if (key <= bp.esc_cap && (!heavy || fold_big(prod, key)) && esc_wanted(prod, key, esc_min, esc_bin_products(kNumEscBins - 1)) &&
       ceil_log2_i64(cols) + ceil_log2_i64(prod) <= 31) {
     int b = 0;
     while (prod > esc_bin_products(b)) ++b;
@@ -158,7 +162,7 @@ __device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const
     if (key <= bp.blk_small_cap) return kBinBlock;
     if (key <= bp.blk_large_cap) return kBinDense;
   }
-  if (warp_ok) {
+  if (warp_ok && !heavy) {
     int64_t need = (int64_t)ceilf((float)key / bp.max_load);
     int lg = ceil_log2_i64(need);
     if (lg < kMinLogT) lg = kMinLogT;

@@ -72,7 +72,35 @@ struct BinParams {
   int64_t blk_small_cap;
   int64_t blk_large_cap;
   int64_t esc_cap;     // most entries of a row in the expand-sort-fold bins
+  int64_t heavy_min;   // rows of more entries may be heavy below warp_cap too (big_row)
 };
+
+// Rows of more entries than this leave the warp tables for the heavy-row units
+// where their bitmap allows (big_row).  A table of 2^11 or 2^12 slots leaves an
+// SM 8 or 4 warps.  Call with R-MAT 16 (4 edges a vertex), 14 and 12, plain:
+// from 2,048 entries 2.31, 2.53 and 1.84 ms, from 1,024 1.86, 1.79 and 1.14,
+// from 512 1.52, 1.53 and 0.80, from 256 1.46, 1.52 and 0.81.
+constexpr int64_t kHeavyMin = 512;
+// A row bounded by u entries goes the way of the heavy rows (symbolic bitmap,
+// units) when it is past the warp tables, or past heavy_min while its columns'
+// bitmap has at most 4 words an entry: clearing and counting it then costs no
+// more than hashing.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool big_row(int64_t u, int64_t cols, int64_t warp_cap, int64_t heavy_min) {
+  return u > warp_cap || (u > heavy_min && cols <= 128 * u);
+}
+
+// Whether such a row (prod products, out entries) is folded all the same: up to
+// 1,152 products, or when nearly all of them are distinct.  The fold's larger
+// bins hold 8 and 4 warps an SM.  From 1,153 products to the units: R-MAT 14
+// and 12 plain 2.59 -> 1.87 and 1.85 -> 1.12 ms; of Erdos-Renyi rows (100,000 x
+// 40, 1,600 products with 1,587 distinct) to the units 4.36 -> 4.87 ms, folded.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool fold_big(int64_t prod, int64_t out) { return prod <= 1152 || 8 * out >= 7 * prod; }
 
 // BinParams with the CTA-wide numeric bins turned off (paths that only
 // launch the warp bins and the heavy tiles).
@@ -81,6 +109,7 @@ inline BinParams without_block_bins(BinParams bp) {
   bp.blk_small_cap = 0;
   bp.blk_large_cap = 0;
   bp.esc_cap = bp.warp_cap;
+  bp.heavy_min = INT64_MAX;
   return bp;
 }
 

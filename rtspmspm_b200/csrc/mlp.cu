@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "mlp.hpp"
+#include "warp_row.cuh"
 
 namespace spg {
 
@@ -287,11 +288,12 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_mlp_predict(const __nv_bflo
 // Capacity from a prediction: cap = min(bound, ceil(margin * (2^o0 - 1)) +
 // slack); a row goes to the exact path (need_exact = 1, cap = 0) when its
 // cap exceeds the largest table of the learned pass (learn_cap) or, with
-// bin_gate, its predicted bin says beyond the warp tables; force_overflow
-// sets cap = 1 (every row then overflows and is re-run).
+// bin_gate, its predicted bin says beyond the warp tables, or when it is past
+// heavy_min and the heavy-row units take it (big_row) but not the fold;
+// force_overflow sets cap = 1 (every row then overflows and is re-run).
 __device__ __forceinline__ void capacity_of(int64_t p, int64_t cols, float o0, float o1, float margin, int slack,
-                                            int64_t learn_cap, int bin_gate, int force_overflow, int64_t& cap,
-                                            uint8_t& ex) {
+                                            int64_t learn_cap, int bin_gate, int force_overflow, int64_t heavy_min,
+                                            int esc_min, int64_t& cap, uint8_t& ex) {
   const int64_t u = p < cols ? p : cols;
   cap = 0;
   ex = 0;
@@ -302,7 +304,9 @@ __device__ __forceinline__ void capacity_of(int64_t p, int64_t cols, float o0, f
   int64_t c = cd >= (double)u ? u : (int64_t)cd;
   if (c < 1) c = 1;
   if (force_overflow) c = 1;
-  if (c > learn_cap || (bin_gate && o1 > (float)kMaxLogT + 0.5f)) {
+  const bool units = c > heavy_min && big_row(c, cols, learn_cap, heavy_min) &&
+                     !(fold_big(p, (int64_t)pred) && esc_wanted(p, c, esc_min, esc_bin_products(kNumEscBins - 1)));
+  if (c > learn_cap || units || (bin_gate && o1 > (float)kMaxLogT + 0.5f)) {
     ex = 1;
     c = 0;
   }
@@ -322,8 +326,8 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_learned_plan(DCsr A, DCsr B
                                                                   const __nv_bfloat16* w, float margin, int slack,
                                                                   int64_t learn_cap, int bin_gate,
                                                                   int force_overflow, int64_t* prod, int64_t* cap,
-                                                                  uint8_t* need_exact,
-                                                                  unsigned long long* n_exact) {
+                                                                  uint8_t* need_exact, unsigned long long* n_exact,
+                                                                  int64_t heavy_min, int esc_min) {
   __shared__ MlpSmem sm;
   __shared__ float tile[kPlanWarps][16 * kMlpIn];
   __shared__ int64_t tprod[kPlanWarps][16];
@@ -371,7 +375,7 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_learned_plan(DCsr A, DCsr B
         int64_t c;
         uint8_t ex;
         capacity_of(tprod[wib][ia], tcols[wib][ia], o[0], o[1], margin, slack, learn_cap, bin_gate, force_overflow,
-                    c, ex);
+                    heavy_min, esc_min, c, ex);
         prod[ra] = tprod[wib][ia];
         cap[ra] = c;
         need_exact[ra] = ex;
@@ -381,7 +385,7 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_learned_plan(DCsr A, DCsr B
         int64_t c;
         uint8_t ex;
         capacity_of(tprod[wib][ib], tcols[wib][ib], o[2], o[3], margin, slack, learn_cap, bin_gate, force_overflow,
-                    c, ex);
+                    heavy_min, esc_min, c, ex);
         prod[rb] = tprod[wib][ib];
         cap[rb] = c;
         need_exact[rb] = ex;
@@ -674,18 +678,18 @@ void launch_mlp_predict(const void* w16, const float* feats, int64_t rows, float
 
 void launch_learned_plan(const DCsr& A, const DCsr& B, const void* w16, float margin, int slack, int64_t learn_cap,
                          int bin_gate, int force_overflow, int64_t* prod, int64_t* cap, uint8_t* need_exact,
-                         unsigned long long* n_exact, const LaunchCtx& lc) {
+                         unsigned long long* n_exact, const LaunchCtx& lc, int64_t heavy_min, int esc_min) {
   if (A.rows == 0) return;
   const int64_t tiles = (A.rows + 15) / 16;
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((tiles + kPlanWarps - 1) / kPlanWarps, lc.sms * 8));
   if (B.rp32)
     k_learned_plan<true, false><<<blocks, kPlanWarps * 32, 0, lc.stream>>>(
         A, B, nullptr, nullptr, A.rows, (const __nv_bfloat16*)w16, margin, slack, learn_cap, bin_gate, force_overflow,
-        prod, cap, need_exact, n_exact);
+        prod, cap, need_exact, n_exact, heavy_min, esc_min);
   else
     k_learned_plan<false, false><<<blocks, kPlanWarps * 32, 0, lc.stream>>>(
         A, B, nullptr, nullptr, A.rows, (const __nv_bfloat16*)w16, margin, slack, learn_cap, bin_gate, force_overflow,
-        prod, cap, need_exact, n_exact);
+        prod, cap, need_exact, n_exact, heavy_min, esc_min);
 }
 
 void launch_learned_plan_batch(const BatchMat* mats, const int32_t* row_mat, int64_t R, const void* w16, float margin,
@@ -698,7 +702,7 @@ void launch_learned_plan_batch(const BatchMat* mats, const int32_t* row_mat, int
   // every product of the batch's queue has 32-bit row offsets of B
   k_learned_plan<true, true><<<blocks, kPlanWarps * 32, 0, lc.stream>>>(
       none, none, mats, row_mat, R, (const __nv_bfloat16*)w16, margin, slack, learn_cap, 0, force_overflow, prod,
-      cap, need_exact, n_exact);
+      cap, need_exact, n_exact, INT64_MAX, 0);
 }
 
 // CTAs of the training step: a tile each, up to two an SM.

@@ -17,10 +17,12 @@ void launch_features(const DCsr& A, const DCsr& B, float* feats, int64_t* prod, 
 void launch_mlp_predict(const void* w16, const float* feats, int64_t rows, float* out, const LaunchCtx& lc);
 // Fused learned plan: per row products, MLP capacity and exact-path mark
 // (capacity above learn_cap, or with bin_gate a predicted bin beyond the
-// warp tables).
+// warp tables).  Rows of more than heavy_min entries that neither the warp
+// tables nor the fold (from esc_min products, 0: off) suit best go to the exact
+// path too.
 void launch_learned_plan(const DCsr& A, const DCsr& B, const void* w16, float margin, int slack, int64_t learn_cap,
                          int bin_gate, int force_overflow, int64_t* prod, int64_t* cap, uint8_t* need_exact,
-                         unsigned long long* n_exact, const LaunchCtx& lc);
+                         unsigned long long* n_exact, const LaunchCtx& lc, int64_t heavy_min, int esc_min);
 // The same over the R global rows of a batch (products with int32 row
 // offsets of B); no bin gate.
 struct BatchMat;

@@ -47,3 +47,27 @@ def test_heavy_units(cols, bits):
         assert rep["rows_heavy"] > 0
         assert_parity(C.to_host(), oracle.spgemm(A2, B))
         C.free()
+
+
+@pytest.mark.parametrize("entries", [9, 12, 20, 36])
+def test_rows_leaving_the_warp_tables_early(entries):
+    """540 to 2,160 products a row over 1,800 columns: 470 to 1,260 output
+    entries, on both sides of the 512 past which rows go to the units and of
+    the products up to which they are folded."""
+    rng = np.random.default_rng(entries)
+    A = gen.coo_to_csr(60, 90, np.repeat(np.arange(60), entries),
+                       np.concatenate([rng.choice(90, entries, replace=False) for _ in range(60)]),
+                       rng.uniform(-1, 1, 60 * entries).astype(np.float32))
+    B = gen.coo_to_csr(90, 1800, np.repeat(np.arange(90), 60),
+                       np.concatenate([rng.choice(1800, 60, replace=False) for _ in range(90)]),
+                       rng.uniform(-1, 1, 90 * 60).astype(np.float32))
+    R = oracle.spgemm(A, B)
+    with Engine(0) as eng:
+        eng.set_tuning(small_rows=-1)
+        for algo in ("plain", "learned"):
+            C, rep = eng.multiply(A, B, algo=algo, use_tuning=True)
+            assert rep["device_flags"] == 0
+            assert_parity(C.to_host(), R)
+        eng.multiply_reuse(A, B, C)
+        assert_parity(C.to_host(), R)
+        C.free()
