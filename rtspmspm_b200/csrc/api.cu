@@ -176,11 +176,18 @@ static int block_table_log(const spg_tuning& t) {
 // the pinned staging words by a one-block kernel through the mapped host
 // address, not by a copy engine: a large device-to-host copy in flight on
 // another stream (spg_multiply_into_host) would otherwise delay them.
-spg_status stage_read(spg_ctx* ctx, void* host_dst, const void* dev_src, size_t bytes) {
-  const size_t at = (size_t)(static_cast<char*>(host_dst) - reinterpret_cast<char*>(ctx->h_stage));
-  if (at + bytes > 64 * sizeof(int64_t) || (bytes & 3)) return fail(ctx, SPG_ERR_INTERNAL, "bad staging read");
-  launch_copy_words(dev_src, reinterpret_cast<char*>(ctx->h_stage_dev) + at, (int64_t)(bytes / 4), launch_ctx(ctx));
-  return cuda_status(ctx, cudaGetLastError(), "stage_read");
+spg_status stage_reads(spg_ctx* ctx, std::initializer_list<StageRead> reads) {
+  StageCopies c{};
+  for (const StageRead& r : reads) {
+    const size_t at = (size_t)(static_cast<char*>(r.host_dst) - reinterpret_cast<char*>(ctx->h_stage));
+    if (at + r.bytes > 64 * sizeof(int64_t) || (r.bytes & 3) || c.n == StageCopies::kMax)
+      return fail(ctx, SPG_ERR_INTERNAL, "bad staging read");
+    c.src[c.n] = static_cast<const uint32_t*>(r.dev_src);
+    c.dst[c.n] = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(ctx->h_stage_dev) + at);
+    c.words[c.n++] = (int)(r.bytes / 4);
+  }
+  launch_copy_words(c, launch_ctx(ctx));
+  return cuda_status(ctx, cudaGetLastError(), "stage_reads");
 }
 
 spg_status read_flags(spg_ctx* ctx, int* flags) {
@@ -392,14 +399,15 @@ struct Pipeline {
     ctx->launches += 3;
   }
 
-  // Offsets of the last binning (and optional extra int64 words) to host.
-  spg_status fetch_offsets(const int64_t* extra = nullptr, int64_t* extra_host = nullptr, int n_extra = 0) {
+  // Offsets of the last binning to host.
+  spg_status fetch_offsets() {
     SPG_TRY(stage_read(ctx, ctx->h_stage, offsets(), sizeof(int64_t) * (kNumBins + 1)));
-    for (int i = 0; i < n_extra; ++i)
-      SPG_TRY(stage_read(ctx, ctx->h_stage + kNumBins + 1 + i, extra + i, sizeof(int64_t)));
+    return wait_offsets();
+  }
+  // Waits for a staged read of the offsets.
+  spg_status wait_offsets() {
     SPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     std::memcpy(h_off, ctx->h_stage, sizeof(int64_t) * (kNumBins + 1));
-    for (int i = 0; i < n_extra; ++i) extra_host[i] = ctx->h_stage[kNumBins + 1 + i];
     return SPG_OK;
   }
 
@@ -656,11 +664,10 @@ spg_status multiply_plain(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opts&
   int64_t extra[2];
   const int64_t* src[2] = {P.nnz.as<int64_t>() + P.rows, reinterpret_cast<const int64_t*>(ctx->d_counter + 1)};
   // fetch offsets + total nnz + products
-  SPG_TRY(stage_read(ctx, ctx->h_stage, P.offsets(), sizeof(int64_t) * (kNumBins + 1)));
-  SPG_TRY(stage_read(ctx, ctx->h_stage + kNumBins + 1, src[0], 8));
-  SPG_TRY(stage_read(ctx, ctx->h_stage + kNumBins + 2, src[1], 8));
-  SPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  std::memcpy(P.h_off, ctx->h_stage, sizeof(int64_t) * (kNumBins + 1));
+  SPG_TRY(stage_reads(ctx, {{ctx->h_stage, P.offsets(), sizeof(int64_t) * (kNumBins + 1)},
+                            {ctx->h_stage + kNumBins + 1, src[0], 8},
+                            {ctx->h_stage + kNumBins + 2, src[1], 8}}));
+  SPG_TRY(P.wait_offsets());
   extra[0] = ctx->h_stage[kNumBins + 1];
   extra[1] = ctx->h_stage[kNumBins + 2];
   const int64_t total = extra[0];
@@ -717,8 +724,11 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
   ctx->launches += 4;
   int64_t slab_total = 0;
   constexpr int kExactSlot = 40;  // h_stage word (64 in all)
-  SPG_TRY(stage_read(ctx, ctx->h_stage + kExactSlot, ctx->d_counter + 3, 8));
-  SPG_TRY(P.fetch_offsets(slab_off.as<int64_t>() + rows, &slab_total, 1));
+  SPG_TRY(stage_reads(ctx, {{ctx->h_stage, P.offsets(), sizeof(int64_t) * (kNumBins + 1)},
+                            {ctx->h_stage + kNumBins + 1, slab_off.as<int64_t>() + rows, 8},
+                            {ctx->h_stage + kExactSlot, ctx->d_counter + 3, 8}}));
+  SPG_TRY(P.wait_offsets());
+  slab_total = ctx->h_stage[kNumBins + 1];
   const int64_t n_exact = ctx->h_stage[kExactSlot];
   // predicted-light rows: the warp, CTA, and expand-sort-fold bins, the first
   // entries of the binning's lists
@@ -763,8 +773,8 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
     tm.mark(SPG_STAGE_SCAN);
     launch_excl_scan(P.nnz.as<int64_t>(), rows, P.nnz.as<int64_t>(), P.scan_tmp.as<int64_t>(), lc);
     ctx->launches += 4;
-    SPG_TRY(stage_read(ctx, ctx->h_stage + kNumBins + 1, P.nnz.as<int64_t>() + rows, 8));
-    SPG_TRY(stage_read(ctx, ctx->h_stage + kNumBins + 2, ctx->d_counter + 1, 16));
+    SPG_TRY(stage_reads(ctx, {{ctx->h_stage + kNumBins + 1, P.nnz.as<int64_t>() + rows, 8},
+                              {ctx->h_stage + kNumBins + 2, ctx->d_counter + 1, 16}}));
     SPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     total = ctx->h_stage[kNumBins + 1];
     if (rep) {
@@ -803,11 +813,10 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
     tm.mark(SPG_STAGE_SCAN);
     launch_excl_scan(P.nnz.as<int64_t>(), rows, P.nnz.as<int64_t>(), P.scan_tmp.as<int64_t>(), lc);
     ctx->launches += 4;
-    SPG_TRY(stage_read(ctx, ctx->h_stage, P.offsets(), sizeof(int64_t) * (kNumBins + 1)));
-    SPG_TRY(stage_read(ctx, ctx->h_stage + kNumBins + 1, P.nnz.as<int64_t>() + rows, 8));
-    SPG_TRY(stage_read(ctx, ctx->h_stage + kNumBins + 2, ctx->d_counter + 1, 16));
-    SPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    std::memcpy(P.h_off, ctx->h_stage, sizeof(int64_t) * (kNumBins + 1));
+    SPG_TRY(stage_reads(ctx, {{ctx->h_stage, P.offsets(), sizeof(int64_t) * (kNumBins + 1)},
+                              {ctx->h_stage + kNumBins + 1, P.nnz.as<int64_t>() + rows, 8},
+                              {ctx->h_stage + kNumBins + 2, ctx->d_counter + 1, 16}}));
+    SPG_TRY(P.wait_offsets());
     total = ctx->h_stage[kNumBins + 1];
     if (rep) {
       rep->products = ctx->h_stage[kNumBins + 2];
@@ -861,7 +870,7 @@ spg_status multiply_small(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opts&
   tm.mark(SPG_STAGE_SCAN);
   constexpr int kSmallSlot = 48;  // h_stage words 48..51
   launch_small_scan(P.nnz.as<int64_t>(), P.prod.as<int64_t>(), rows, bits != 64 ? rp32.as<int32_t>() : nullptr,
-                    P.lists.as<int32_t>(), ctx->d_counter + 6, ctx->h_stage_dev + kSmallSlot, lc);
+                    ctx->d_counter + 6, ctx->h_stage_dev + kSmallSlot, lc);
   ctx->launches += 2;
   SPG_CUDA(ctx, cudaGetLastError());
   SPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -881,7 +890,7 @@ spg_status multiply_small(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opts&
   SPG_TRY(P.alloc_entries(total, c_col, c_val));
   tm.mark(SPG_STAGE_NUMERIC);
   if (total > 0) {
-    launch_num_warp(log_t, P.A.view, P.B.view, P.lists.as<int32_t>(), rows, P.nnz.as<int64_t>(), c_col.as<int32_t>(),
+    launch_num_warp(log_t, P.A.view, P.B.view, nullptr, rows, P.nnz.as<int64_t>(), c_col.as<int32_t>(),
                     c_val.as<float>(), ctx->d_flags, lc, P.wpb, P.esc_args(P.prod.as<int64_t>()));
     ++ctx->launches;
   }

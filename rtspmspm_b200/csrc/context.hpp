@@ -6,6 +6,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -130,10 +131,19 @@ class DevLayout {
 
 inline LaunchCtx launch_ctx(const spg_ctx* ctx) { return LaunchCtx{ctx->stream, ctx->sms, ctx->device}; }
 
-// Enqueues a copy of `bytes` (a multiple of 4) device bytes into the mapped
-// staging words at host_dst (inside ctx->h_stage); valid after the next
-// stream synchronisation.
-spg_status stage_read(spg_ctx* ctx, void* host_dst, const void* dev_src, size_t bytes);
+// Enqueues copies of `bytes` (a multiple of 4) device bytes each into the
+// mapped staging words at host_dst (inside ctx->h_stage), at most
+// StageCopies::kMax in one launch; valid after the next stream
+// synchronisation.
+struct StageRead {
+  void* host_dst;
+  const void* dev_src;
+  size_t bytes;
+};
+spg_status stage_reads(spg_ctx* ctx, std::initializer_list<StageRead> reads);
+inline spg_status stage_read(spg_ctx* ctx, void* host_dst, const void* dev_src, size_t bytes) {
+  return stage_reads(ctx, {{host_dst, dev_src, bytes}});
+}
 
 // Device view of an spg_csr already on the device with int64 row pointers.
 struct DevMat {

@@ -296,9 +296,8 @@ spg_status coo_to_csr_device(spg_ctx* ctx, int64_t rows, int64_t cols, int64_t n
   if (n > 0) k_count_runs<<<(unsigned)nfold, kFoldThreads, 0, lc.stream>>>(kin, n, runs.as<int64_t>());
   launch_excl_scan(runs.as<int64_t>(), nfold, runs.as<int64_t>(), tmp.as<int64_t>(), lc);
   int64_t m = 0;
-  SPG_TRY(stage_read(ctx, ctx->h_stage + 52, runs.as<int64_t>() + nfold, 8));
+  SPG_TRY(stage_reads(ctx, {{ctx->h_stage + 52, runs.as<int64_t>() + nfold, 8}, {ctx->h_stage + 53, ctx->d_flags, 4}}));
   int f = 0;
-  SPG_TRY(stage_read(ctx, ctx->h_stage + 53, ctx->d_flags, 4));
   SPG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   m = ctx->h_stage[52];
   std::memcpy(&f, &ctx->h_stage[53], sizeof f);

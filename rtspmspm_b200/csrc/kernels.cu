@@ -580,7 +580,8 @@ __global__ void __launch_bounds__(kSymDenseThreads, 2048 / kSymDenseThreads) k_s
 // Numeric pass: warp-level hash accumulator
 // --------------------------------------------------------------------------
 
-// Plain numeric pass: exact nnz known, writes straight into C.  With the
+// Plain numeric pass: exact nnz known, writes straight into C (rows == null:
+// rows 0 .. nrows - 1).  With the
 // row products `prod` given, rows that esc_wanted() take esc_row.  56
 // registers (36 resident warps per SM at 2^9-slot tables) also with the
 // expand-sort-fold code inlined, which would take 64 unbounded.
@@ -601,7 +602,7 @@ __global__ void __maxnreg__(56) k_num_warp(DCsr A, DCsr B, const int32_t* rows, 
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int ecap = esc_capacity(numeric_words<LOGT>());
   for (int64_t idx = gw; idx < nrows; idx += nw) {
-    const int32_t row = rows[idx];
+    const int32_t row = rows ? rows[idx] : (int32_t)idx;
     const int64_t off = c_rp[row];
     const int64_t want = c_rp[row + 1] - off;
     if (prod) {
@@ -1378,69 +1379,88 @@ __global__ void __launch_bounds__(kSmallCountWarps * 32) k_small_count(DCsr A, D
 
 // One CTA over the counts of a small product (rows <= kSmallMaxRows): the
 // exclusive scan into C's int64 row pointers in place (nnz[rows] = the
-// total) and, when rp32 is given and the total fits, into int32 row
-// pointers; the identity row list of the numeric launch; and, into the
-// mapped host words out[0..3], the total, the products, the largest count
-// and the number of rows too large to count (any of them sends the call to
-// the binned pipeline).  Thread t owns rows [t * per, (t + 1) * per).
+// total) and, when rp32 is given, into int32 row pointers (the total of so few
+// counts of at most 2^kSmallLogT fits); and, into the mapped host words
+// out[0..3], the total, the products, the largest count and the number of rows
+// too large to count (any of them sends the call to the binned pipeline).
+//
+// Bound: the latency of its loads and barriers.  Warp w owns a run of rows, 32
+// consecutive ones a load; all loads of kSmallScanStep x 32 rows are issued
+// before the first is used.  A thread on a run of its own, row after row with
+// the counts read twice, took 10 us for 4,096 rows.
+constexpr int kSmallScanStep = 8;
 __global__ void __launch_bounds__(kSmallScanThreads) k_small_scan(int64_t* nnz, const int64_t* prod, int64_t rows,
-                                                                  int32_t* rp32, int32_t* row_list,
-                                                                  unsigned long long* stop, volatile int64_t* out) {
+                                                                  int32_t* rp32, unsigned long long* stop,
+                                                                  volatile int64_t* out) {
   constexpr int kW = kSmallScanThreads / 32;
-  __shared__ int64_t wsum[kW], wprod[kW], wmax[kW], wbig[kW];
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  const int64_t per = (rows + kSmallScanThreads - 1) / kSmallScanThreads;
-  const int64_t r0 = min(rows, (int64_t)t * per), r1 = min(rows, r0 + per);
-  int64_t sum = 0, psum = 0, mx = 0, big = 0;
-  for (int64_t r = r0; r < r1; ++r) {
-    const int64_t c = nnz[r];
-    if (c < 0) {
-      ++big;
-    } else {
-      sum += c;
-      mx = max(mx, c);
+  static_assert(kSmallMaxRows <= INT32_MAX >> kSmallLogT, "the counts' total fits 32 bits");
+  __shared__ int wsum[kW], wmax[kW], wbig[kW];
+  __shared__ int64_t wprod[kW];
+  const int lane = lane_id(), w = threadIdx.x >> 5;
+  const int per = ((int)rows + kSmallScanThreads - 1) / kSmallScanThreads;  // 32-row groups a warp
+  const int g0 = w * per * 32;
+  int sum = 0, mx = 0, big = 0;
+  int64_t psum = 0;
+  int c[kSmallScanStep];
+  auto load = [&](int j0) {
+    int64_t p[kSmallScanStep];
+#pragma unroll
+    for (int j = 0; j < kSmallScanStep; ++j) {
+      const int r = g0 + (j0 + j) * 32 + lane;
+      const bool in = j0 + j < per && r < rows;
+      c[j] = in ? (int)nnz[r] : 0;
+      p[j] = in ? prod[r] : 0;
     }
-    psum += prod[r];
-    row_list[r] = (int32_t)r;
-  }
-  const int64_t incl = warp_incl_scan(sum);
-  const int64_t ps = warp_sum(psum), mm = warp_max(mx), bb = warp_sum(big);
-  if (lane == 31) wsum[w] = incl;
+#pragma unroll
+    for (int j = 0; j < kSmallScanStep; ++j) {
+      big += c[j] < 0;
+      c[j] = max(c[j], 0);
+      sum += c[j];
+      mx = max(mx, c[j]);
+      psum += p[j];
+    }
+  };
+  for (int j0 = 0; j0 < per; j0 += kSmallScanStep) load(j0);
+  sum = __reduce_add_sync(kFull, sum);
+  mx = __reduce_max_sync(kFull, mx);
+  big = __reduce_add_sync(kFull, big);
+  psum = warp_sum(psum);
   if (lane == 0) {
-    wprod[w] = ps;
-    wmax[w] = mm;
-    wbig[w] = bb;
+    wsum[w] = sum;
+    wmax[w] = mx;
+    wbig[w] = big;
+    wprod[w] = psum;
   }
   __syncthreads();
-  int64_t wexcl = 0, total = 0;
-  {
-    const int64_t v = lane < kW ? wsum[lane] : 0;
-    const int64_t vi = warp_incl_scan(v);
-    wexcl = __shfl_sync(kFull, vi - v, w);
-    total = __shfl_sync(kFull, vi, 31);
-  }
-  int64_t run = wexcl + incl - sum;
-  const bool narrow = rp32 != nullptr && total < INT32_MAX;
-  for (int64_t r = r0; r < r1; ++r) {
-    const int64_t c = nnz[r];
-    nnz[r] = run;
-    if (narrow) rp32[r] = (int32_t)run;
-    run += c < 0 ? 0 : c;
-  }
-  if (t == 0) {
-    nnz[rows] = total;
-    if (narrow) rp32[rows] = (int32_t)total;
-    int64_t p = 0, m = 0, b = 0;
-    for (int i = 0; i < kW; ++i) {
-      p += wprod[i];
-      m = max(m, wmax[i]);
-      b += wbig[i];
+  const int ws = wsum[lane];
+  const int incl = warp_incl_scan(ws);
+  int run = __shfl_sync(kFull, incl - ws, w);
+  const int total = __shfl_sync(kFull, incl, 31);
+  for (int j0 = 0; j0 < per; j0 += kSmallScanStep) {
+    if (per > kSmallScanStep) load(j0);  // else still in registers
+#pragma unroll
+    for (int j = 0; j < kSmallScanStep; ++j) {
+      const int r = g0 + (j0 + j) * 32 + lane;
+      const int inc = warp_incl_scan(c[j]);
+      if (j0 + j < per && r < rows) {
+        nnz[r] = run + inc - c[j];
+        if (rp32) rp32[r] = run + inc - c[j];
+      }
+      run += __shfl_sync(kFull, inc, 31);
     }
-    out[0] = total;
-    out[1] = p;
-    out[2] = m;
-    out[3] = b;
-    *stop = 0ull;
+  }
+  if (w == 0) {
+    const int64_t p = warp_sum(wprod[lane]);
+    const int m = __reduce_max_sync(kFull, wmax[lane]), b = __reduce_add_sync(kFull, wbig[lane]);
+    if (lane == 0) {
+      nnz[rows] = total;
+      if (rp32) rp32[rows] = total;
+      out[0] = total;
+      out[1] = p;
+      out[2] = m;
+      out[3] = b;
+      *stop = 0ull;
+    }
   }
 }
 
@@ -1546,9 +1566,9 @@ void launch_small_count(const DCsr& A, const DCsr& B, int64_t* prod, int64_t* nn
   else k_small_count<false><<<blocks, sh.wpb * 32, smem, lc.stream>>>(A, B, prod, nnz, stop, flags);
 }
 
-void launch_small_scan(int64_t* nnz, const int64_t* prod, int64_t rows, int32_t* rp32, int32_t* row_list,
-                       unsigned long long* stop, int64_t* out, const LaunchCtx& lc) {
-  k_small_scan<<<1, kSmallScanThreads, 0, lc.stream>>>(nnz, prod, rows, rp32, row_list, stop, out);
+void launch_small_scan(int64_t* nnz, const int64_t* prod, int64_t rows, int32_t* rp32, unsigned long long* stop,
+                       int64_t* out, const LaunchCtx& lc) {
+  k_small_scan<<<1, kSmallScanThreads, 0, lc.stream>>>(nnz, prod, rows, rp32, stop, out);
 }
 
 void launch_sum(const int64_t* v, int64_t n, unsigned long long* out, const LaunchCtx& lc) {
@@ -1855,15 +1875,14 @@ void launch_num_block_learned(int bin, const DCsr& A, const DCsr& B, const int32
 #undef SPG_NBL
 }
 
-// dst[i] = src[i] for n 32-bit words; dst may be mapped pinned host memory.
-__global__ void k_copy_words(const uint32_t* src, uint32_t* dst, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    dst[i] = src[i];
+// Copies a few runs of 32-bit words; dst may be mapped pinned host memory.
+__global__ void k_copy_words(StageCopies c) {
+  for (int k = 0; k < c.n; ++k)
+    for (int i = threadIdx.x; i < c.words[k]; i += blockDim.x) c.dst[k][i] = c.src[k][i];
 }
 
-void launch_copy_words(const void* src, void* dst, int64_t n, const LaunchCtx& lc) {
-  if (n == 0) return;
-  k_copy_words<<<1, 128, 0, lc.stream>>>(static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), n);
+void launch_copy_words(const StageCopies& c, const LaunchCtx& lc) {
+  if (c.n > 0) k_copy_words<<<1, 64, 0, lc.stream>>>(c);
 }
 
 // out[i] = in[i] + off as int32 (out_bits 32) or int64.

@@ -130,9 +130,8 @@ void launch_row_products(const DCsr& A, const DCsr& B, int64_t* prod, const Laun
 // 2^kSmallLogT products): products and exact counts per row in one launch
 // (nnz[row] = -1 for a row of more products), then one CTA scans the counts
 // into C's row pointers (int64 in place, int32 into rp32 when given and the
-// total fits), writes the identity row list and puts the total, the
-// products, the largest count and the too-large rows into out[0..3]
-// (mapped host words).
+// total fits) and puts the total, the products, the largest count and the
+// too-large rows into out[0..3] (mapped host words).
 constexpr int kSmallLogT = 11;
 constexpr int kSmallCountWarps = 4;
 constexpr int kSmallScanThreads = 1024;
@@ -143,8 +142,8 @@ constexpr int kSmallDefaultRows = 8192;
 // the scan clears it.
 void launch_small_count(const DCsr& A, const DCsr& B, int64_t* prod, int64_t* nnz, unsigned long long* stop,
                         int* flags, const LaunchCtx& lc);
-void launch_small_scan(int64_t* nnz, const int64_t* prod, int64_t rows, int32_t* rp32, int32_t* row_list,
-                       unsigned long long* stop, int64_t* out, const LaunchCtx& lc);
+void launch_small_scan(int64_t* nnz, const int64_t* prod, int64_t rows, int32_t* rp32, unsigned long long* stop,
+                       int64_t* out, const LaunchCtx& lc);
 // Default smallest product count of an expand-sort-fold row.  Numeric stage
 // of 200,000-row Erdos-Renyi products with 36 | 64 | 100 | 144 products a row:
 // from 128 products 0.32 | 0.44 | 0.52 | 0.53 ms, from 64 0.30 | 0.33 | 0.37 |
@@ -200,9 +199,16 @@ void launch_num_block_learned(int bin, const DCsr& A, const DCsr& B, const int32
                               const int64_t* cap, const int64_t* slab_off, int32_t* slab_col, float* slab_val,
                               int64_t* nnz_out, int32_t* retry_rows, unsigned long long* retry_count, int* flags,
                               const LaunchCtx& lc);
-// Copies n 32-bit words with one small kernel (dst may be mapped pinned host
-// memory: the read-back then needs no copy engine).
-void launch_copy_words(const void* src, void* dst, int64_t n, const LaunchCtx& lc);
+// Copies a few runs of 32-bit words with one small kernel (dst may be mapped
+// pinned host memory: the read-back then needs no copy engine).
+struct StageCopies {
+  static constexpr int kMax = 4;
+  const uint32_t* src[kMax];
+  uint32_t* dst[kMax];
+  int words[kMax];
+  int n;
+};
+void launch_copy_words(const StageCopies& c, const LaunchCtx& lc);
 // Row pointers shifted by `off` into an int32 (out_bits 32) or int64 array.
 void launch_shift_rp(const int64_t* in, int64_t n, int64_t off, void* out, int out_bits, const LaunchCtx& lc);
 // Value-only recompute: row lengths of C, and heavy-row slots and per-tile
