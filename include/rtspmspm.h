@@ -406,7 +406,7 @@ typedef struct spg_tuning {
                                   warp tables and heavy-row tiles only */
     int32_t esc_min_prod;      /* rows of at least this many products (0: default 32) whose
                                   output keeps half of them or more, and that fit the warp's
-                                  table memory, are expanded, radix sorted on their columns and
+                                  table memory, are expanded, sorted on their columns and
                                   folded instead of hashed; -1: off */
     int32_t small_rows;        /* products whose A has at most this many rows (0: default 8192;
                                   at most 65536), every row of at most 2048 products, take the
