@@ -45,12 +45,15 @@ static_assert(kUnitCost < 65536, "a unit's entries are a 16-bit field");
 // kUnitCost words.  One warp per row, 32 tiles at a time (a scan of their
 // entries and a ballot find the first tile that no longer fits): a sweep to
 // count the units, one atomic for their place in the list, a sweep to write
-// them.  Units of long rows of A fill the list from its front (nunits[0]),
-// the others from its back (nunits[1]).  Unit: {row, first tile, (tiles <<
-// 16) | entries, entries of the row before it}.
+// them.  Units of long rows of A fill the list from its front, the others from
+// its back; *nunits counts them in its low and its high half.  Unit: {row, first
+// tile, (tiles << 16) | entries, entries of the row before it}.  A tile holds at
+// most kTileCols entries and so fits a unit of its own.  The list has room for
+// every unit of rows that hold the entries they were said to; row pointers of
+// C that say otherwise raise a flag.
 __global__ void k_cut_units(const int32_t* heavy_rows, int64_t nheavy, const int32_t* big_slot, const int32_t* tile_cnt,
-                            int ntiles, const int64_t* a_rp, int4* units, int64_t room,
-                            unsigned long long* nunits) {
+                            int ntiles, const int64_t* a_rp, int4* units, int64_t room, unsigned long long* nunits,
+                            int* flags) {
   const int lane = lane_id();
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -92,9 +95,14 @@ __global__ void k_cut_units(const int32_t* heavy_rows, int64_t nheavy, const int
       if (sweep == 0) {
         const bool back = a_rp[row + 1] - a_rp[row] <= kLongRow;
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(nunits + (back ? 1 : 0), (unsigned long long)made);
+        if (lane == 0) base = atomicAdd(nunits, (unsigned long long)made << (back ? 32 : 0));
         base = __shfl_sync(kFull, base, 0);
-        out = back ? units + (room - (int64_t)base - made) : units + base;
+        const int64_t front = (int64_t)(base & 0xffffffffu), behind = (int64_t)(base >> 32);
+        if (front + behind + made > room) {  // the units' kernel sees the count and takes none
+          if (lane == 0) raise_flag(flags, kFlagCountDiff);
+          break;
+        }
+        out = back ? units + (room - behind - made) : units + front;
       }
     }
   }
@@ -203,7 +211,8 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
   __shared__ unsigned long long sh_ticket;
   const int tid = threadIdx.x, lane = lane_id(), wib = tid >> 5;
   uint2* bits = reinterpret_cast<uint2*>(sm_unit);  // {columns, entries before them}
-  const int64_t nfront = (int64_t)nunits[0], total_units = nfront + (int64_t)nunits[1];
+  const int64_t nfront = (int64_t)(*nunits & 0xffffffffu), total_units = nfront + (int64_t)(*nunits >> 32);
+  if (total_units > room) return;
   for (;;) {
     if (tid == 0) sh_ticket = atomicAdd(ticket, 1ull);
     __syncthreads();
@@ -371,7 +380,8 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
 
 int64_t heavy_unit_bound(int64_t nheavy, int ntiles, int64_t entries) {
   // of two consecutive units of a row, the first and the second's first tile
-  // exceed kUnitCost together
+  // exceed kUnitCost together (and the list's two 32-bit counts hold it: at
+  // 16 bytes a unit, 2^31 of them are 32 GB)
   return 2 * (entries + (int64_t)kTileCost * ntiles * nheavy) / kUnitCost + nheavy + 1;
 }
 
@@ -394,13 +404,13 @@ void launch_num_units(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, i
                       const int32_t* bidx, const uint32_t* bitmap, int64_t stride, int4* units, int64_t room,
                       unsigned long long* counters, int* flags, const LaunchCtx& lc) {
   if (nheavy == 0) return;
-  cudaMemsetAsync(counters, 0, 3 * sizeof(unsigned long long), lc.stream);
+  cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), lc.stream);
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nheavy + 7) / 8, (int64_t)lc.sms * 8));
   k_cut_units<<<blocks, 256, 0, lc.stream>>>(heavy_rows, nheavy, big_slot, tile_cnt, ntiles, A.rp, units, room,
-                                             counters);
+                                             counters, flags);
 #define SPG_NU(R, S)                                                                                            \
   num_unit_one<R, S>(A, B, units, room, counters, ntiles, c_rp, c_col, c_val, bidx, bitmap, stride, big_slot, \
-                     counters + 2, flags, lc)
+                     counters + 1, flags, lc)
   if (B.rp32) {
     if (bitmap) SPG_NU(true, true);
     else SPG_NU(true, false);

@@ -844,7 +844,9 @@ __global__ void k_row_lengths(const int64_t* rp, int64_t rows, int64_t* len) {
 // big_slot[heavy_rows[h]] = h; one warp per heavy row then counts the row's
 // entries per column tile (tile_cnt[h * ntiles + t], zeroed beforehand) from
 // the run starts of its sorted columns: a tile's count is the distance from
-// its first entry to the next tile's first entry (or the row end).
+// its first entry to the next tile's first entry (or the row end).  A count past
+// the tile's columns (columns repeated, C not a product's) raises a flag and is
+// cut: the kernels behind rely on a tile fitting its unit.
 __global__ void k_tile_counts_from_cols(const int32_t* heavy_rows, int64_t nheavy, const int64_t* c_rp,
                                         const int32_t* c_col, int ntiles, int32_t* big_slot, int32_t* tile_cnt,
                                         int* flags) {
@@ -858,6 +860,10 @@ __global__ void k_tile_counts_from_cols(const int32_t* heavy_rows, int64_t nheav
     const int64_t s = c_rp[row], e = c_rp[row + 1];
     int pend_t = -1;     // tile whose run is still open (uniform)
     int64_t pend_p = 0;  // its first entry
+    auto close = [&](int t, int64_t n) {
+      if (n > kTileCols) raise_flag(flags, kFlagCountDiff);
+      cnt[t] = (int32_t)(n < kTileCols ? n : kTileCols);
+    };
     for (int64_t base = s; base < e; base += 32) {
       const int64_t p = base + lane;
       int t = -1;
@@ -873,7 +879,7 @@ __global__ void k_tile_counts_from_cols(const int32_t* heavy_rows, int64_t nheav
       const unsigned fm = __ballot_sync(kFull, first);
       if (fm) {
         const int lead = __ffs(fm) - 1;
-        if (pend_t >= 0 && lane == 0) cnt[pend_t] = (int32_t)(base + lead - pend_p);
+        if (pend_t >= 0 && lane == 0) close(pend_t, base + lead - pend_p);
         if (first) {
           const unsigned later = fm & ~((2u << lane) - 1u);
           if (later) cnt[t] = (int32_t)(__ffs(later) - 1 - lane);
@@ -883,7 +889,7 @@ __global__ void k_tile_counts_from_cols(const int32_t* heavy_rows, int64_t nheav
         pend_p = base + last;
       }
     }
-    if (pend_t >= 0 && lane == 0) cnt[pend_t] = (int32_t)(e - pend_p);
+    if (pend_t >= 0 && lane == 0) close(pend_t, e - pend_p);
   }
 }
 

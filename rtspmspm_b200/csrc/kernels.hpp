@@ -242,7 +242,7 @@ void launch_num_tile(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, in
 // holds room = heavy_unit_bound(nheavy, ntiles, entries of those rows);
 // bidx as above; bitmap: the rows' column bitmaps at big_slot * stride words
 // (from launch_sym_dense), or null (each unit finds its columns itself);
-// counters: three device words.
+// counters: two device words.
 int64_t heavy_unit_bound(int64_t nheavy, int ntiles, int64_t entries);
 void launch_num_units(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, int64_t nheavy, const int32_t* big_slot,
                       const int32_t* tile_cnt, int ntiles, const int64_t* c_rp, int32_t* c_col, float* c_val,
