@@ -180,8 +180,8 @@ spg_status spg_multiply_into_host(spg_ctx* ctx, const spg_csr* A, const spg_csr*
  * are counted from C's sorted columns).  C->col_idx is rewritten with the
  * same columns.  As with cuSPARSE's reuse, the caller guarantees that A and
  * B keep the structure C was computed from; a differing count of distinct
- * columns in a row (in a run of column tiles holding entries of C, for rows
- * beyond the warp tables) fails the call with SPG_ERR_INVALID_ARG.
+ * columns in a row (in a column tile holding entries of C, for rows beyond
+ * the warp tables) fails the call with SPG_ERR_INVALID_ARG.
  * report->products is not computed (0).
  * Replaces: cusparseSpGEMMreuse_compute after the structure phase
  * (cuSparse/src/main.cpp:98-296, second compute with new values :286-296).

@@ -378,6 +378,7 @@ struct Pipeline {
   DevBuf bitmap;      // uint32 nbig * bitmap_stride(), or empty
   int64_t h_off[kNumBins + 1] = {};
   int64_t nbig = 0;
+  int64_t whole_max = 0;  // launch_num_units' whole_max (value-only recompute)
 
   Pipeline(spg_ctx* c, const DevMat& a, const DevMat& b, const spg_tuning& t)
       : ctx(c), lc(launch_ctx(c)), A(a), B(b), tune(t), bp(bin_params(t)), rows(a.view.rows), cols(b.view.cols) {
@@ -619,7 +620,7 @@ struct Pipeline {
         DevBuf units;
         SPG_TRY(units.alloc(ctx, (size_t)room * sizeof(int4)));
         launch_num_units(A.view, B.view, bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(),
-                         ntiles, c_rp, c_col, c_val, bidx.as<int32_t>(), bitmap.as<uint32_t>(), bitmap_stride(),
+                         ntiles, c_rp, c_col, c_val, bidx.as<int32_t>(), bitmap.as<uint32_t>(), bitmap_stride(), whole_max,
                          units.as<int4>(), room, ctx->d_counter + 8, ctx->d_flags, lc);
         ++ctx->launches;
       }
@@ -1001,23 +1002,41 @@ spg_status multiply_reuse_device(spg_ctx* ctx, const DevMat& A, const DevMat& B,
   }
   launch_row_lengths(P.nnz.as<int64_t>(), rows, P.prod.as<int64_t>(), lc);
   ctx->launches += 2;
-  P.bin(P.prod.as<int64_t>(), kBinNumeric);
-  SPG_TRY(P.fetch_offsets());
-  const int64_t nheavy = P.bin_size(kBinHeavy);
-  if (nheavy > 0) {
-    const size_t tb = (size_t)nheavy * P.ntiles * 4;
-    SPG_TRY(P.tile_cnt.alloc(ctx, tb));
-    SPG_TRY(P.tile_off.alloc(ctx, tb));
-    SPG_CUDA(ctx, cudaMemsetAsync(P.tile_cnt.get(), 0, tb, ctx->stream));
-    launch_tile_counts_from_cols(P.bin_rows(kBinHeavy), nheavy, P.nnz.as<int64_t>(), C->col_idx, P.ntiles,
-                                 P.big_slot.as<int32_t>(), P.tile_cnt.as<int32_t>(), ctx->d_flags, lc);
-    ++ctx->launches;
-  }
-  tm.mark(SPG_STAGE_NUMERIC);
-  SPG_TRY(P.numeric(P.nnz.as<int64_t>(), C->col_idx, C->val, C->nnz, rep));
-  tm.finish(rep);
+  // rows that leave the warp tables early are held to what the tables hold
+  // them to: their count of distinct columns, whichever these are
+  P.whole_max = P.bp.warp_cap;
   int f = 0;
-  SPG_TRY(read_flags(ctx, &f));
+  for (int pass = 0;; ++pass) {
+    if (pass > 0) tm.mark(SPG_STAGE_BINNING);
+    P.bin(P.prod.as<int64_t>(), kBinNumeric);
+    SPG_TRY(P.fetch_offsets());
+    const int64_t nheavy = P.bin_size(kBinHeavy);
+    if (nheavy > 0) {
+      const size_t tb = (size_t)nheavy * P.ntiles * 4;
+      SPG_TRY(P.tile_cnt.alloc(ctx, tb));
+      SPG_TRY(P.tile_off.alloc(ctx, tb));
+      SPG_CUDA(ctx, cudaMemsetAsync(P.tile_cnt.get(), 0, tb, ctx->stream));
+      launch_tile_counts_from_cols(P.bin_rows(kBinHeavy), nheavy, P.nnz.as<int64_t>(), C->col_idx, P.ntiles,
+                                   P.big_slot.as<int32_t>(), P.tile_cnt.as<int32_t>(), ctx->d_flags, lc);
+      ++ctx->launches;
+    }
+    tm.mark(SPG_STAGE_NUMERIC);
+    spg_report pass_rep{};
+    SPG_TRY(P.numeric(P.nnz.as<int64_t>(), C->col_idx, C->val, C->nnz, &pass_rep));
+    SPG_TRY(read_flags(ctx, &f));
+    // the units also need C's columns where they were; a row whose columns
+    // moved is settled by the tables, which read only its length
+    if ((f & (kFlagCountDiff | kFlagBadIndex)) && nheavy > 0 && pass == 0 && P.bp.heavy_min < P.bp.warp_cap) {
+      P.bp.heavy_min = INT64_MAX;
+      continue;
+    }
+    if (rep) {
+      std::memcpy(rep->bin_rows, pass_rep.bin_rows, sizeof rep->bin_rows);
+      rep->rows_heavy = pass_rep.rows_heavy;
+    }
+    break;
+  }
+  tm.finish(rep);
   if (rep) {
     rep->device_flags |= f;
     rep->nnz_c = C->nnz;

@@ -192,7 +192,11 @@ __device__ __forceinline__ int list_segments(const DCsr& A, const DCsr& B, int64
 
 // One CTA per unit, one atomic ticket each.  STORED: the symbolic pass left
 // the rows' column bitmaps in `bitmap` (big_slot order, `stride` words a
-// row); else the unit's products are walked once to set the bits.  Then A's
+// row); else the unit's products are walked once to set the bits and the
+// columns found are compared with tile_cnt, tile by tile (in a value-only
+// recompute they come from A and B, the counts from C).  For rows of at most
+// whole_max entries that walk also takes in the empty tiles up to the next unit,
+// or the row's ends, so that no product of such a row goes unseen.  Then A's
 // row is walked in canonical order, segment by segment with a barrier after
 // each: a segment's columns are distinct, so the CTA's threads add its
 // products at once.  A thread's first two products of segment i + 2 are
@@ -203,6 +207,7 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
                                                            const int64_t* c_rp, int32_t* c_col, float* c_val,
                                                            const int32_t* bidx, const uint32_t* bitmap,
                                                            int64_t stride, const int32_t* big_slot,
+                                                           const int32_t* tile_cnt, int64_t whole_max,
                                                            unsigned long long* ticket, int* flags) {
   using Off = typename RowOff<R32>::T;
   extern __shared__ __align__(16) uint32_t sm_unit[];
@@ -232,8 +237,21 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
       for (int i = tid; i < words; i += kUnitThreads) bits[i].x = bm[i];
     } else {
       for (int i = tid; i < words; i += kUnitThreads) bits[i].x = 0u;
+      int g0 = t0, g1 = t1;  // the tiles looked at
+      const int64_t entries = c_rp[row + 1] - c_rp[row];
+      const bool whole = entries <= whole_max;
+      if (whole) {
+        const int32_t* tc = tile_cnt + (int64_t)big_slot[row] * ntiles;
+        while (g0 > 0) {
+          const int t = g0 - 1 - lane;
+          const unsigned filled = __ballot_sync(kFull, t >= 0 && tc[t] > 0);
+          g0 = filled ? g0 - (__ffs(filled) - 1) : max(0, g0 - 32);
+          if (filled) break;
+        }
+        if (un.w + n == entries) g1 = ntiles;
+      }
       for (int64_t base = s; base < e; base += kUnitThreads) {
-        const int cnt = list_segments<R32>(A, B, base, e, t0, t1, ntiles, bidx, sl);
+        const int cnt = list_segments<R32>(A, B, base, e, g0, g1, ntiles, bidx, sl);
         for (int i = wib; i < cnt; i += kUnitWarps) {
           const int4 sg = sl.seg[i];
           const Off sb = segment_start<Off>(sg);
@@ -244,7 +262,7 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
               const uint32_t bit = 1u << (off & 31);
               if (!(bits[off >> 5].x & bit)) atomicOr(&bits[off >> 5].x, bit);
             } else {
-              raise_flag(flags, kFlagBadIndex);
+              raise_flag(flags, whole ? kFlagCountDiff : kFlagBadIndex);
             }
           }
         }
@@ -278,6 +296,20 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
     }
     for (int i = tid; i < n; i += kUnitThreads) acc[i] = 0.f;
     __syncthreads();
+    if (!STORED) {
+      // C's columns of such a unit stay as they are: a second look at the row
+      // counts them again
+      const int32_t* tc = tile_cnt + (int64_t)big_slot[row] * ntiles + t0;
+      bool differ = false;
+      for (int j = tid; j < nt; j += kUnitThreads) {
+        const uint32_t upto = j + 1 < nt ? bits[(j + 1) * kTileWords].y : (uint32_t)found;
+        differ |= (int)(upto - bits[j * kTileWords].y) != tc[j];
+      }
+      if (__syncthreads_or(differ)) {
+        if (tid == 0) raise_flag(flags, kFlagCountDiff);
+        continue;
+      }
+    }
     // a column's accumulator; one outside the unit is noted (and lands on any)
     uint32_t far = 0;
     auto locate = [&](int32_t c) -> int {
@@ -389,28 +421,29 @@ template <bool R32, bool STORED>
 static void num_unit_one(const DCsr& A, const DCsr& B, const int4* units, int64_t room,
                          const unsigned long long* nunits, int ntiles,
                          const int64_t* c_rp, int32_t* c_col, float* c_val, const int32_t* bidx,
-                         const uint32_t* bitmap, int64_t stride, const int32_t* big_slot, unsigned long long* ticket,
-                         int* flags, const LaunchCtx& lc) {
+                         const uint32_t* bitmap, int64_t stride, const int32_t* big_slot, const int32_t* tile_cnt,
+                         int64_t whole_max, unsigned long long* ticket, int* flags, const LaunchCtx& lc) {
   const size_t smem = (size_t)kUnitWords * 4;
   cudaFuncSetAttribute(k_num_unit<R32, STORED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_num_unit<R32, STORED>, kUnitThreads, smem);
   k_num_unit<R32, STORED><<<lc.sms * std::max(1, per_sm), kUnitThreads, smem, lc.stream>>>(
-      A, B, units, room, nunits, ntiles, c_rp, c_col, c_val, bidx, bitmap, stride, big_slot, ticket, flags);
+      A, B, units, room, nunits, ntiles, c_rp, c_col, c_val, bidx, bitmap, stride, big_slot, tile_cnt, whole_max,
+      ticket, flags);
 }
 
 void launch_num_units(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, int64_t nheavy, const int32_t* big_slot,
                       const int32_t* tile_cnt, int ntiles, const int64_t* c_rp, int32_t* c_col, float* c_val,
-                      const int32_t* bidx, const uint32_t* bitmap, int64_t stride, int4* units, int64_t room,
-                      unsigned long long* counters, int* flags, const LaunchCtx& lc) {
+                      const int32_t* bidx, const uint32_t* bitmap, int64_t stride, int64_t whole_max, int4* units,
+                      int64_t room, unsigned long long* counters, int* flags, const LaunchCtx& lc) {
   if (nheavy == 0) return;
   cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), lc.stream);
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nheavy + 7) / 8, (int64_t)lc.sms * 8));
   k_cut_units<<<blocks, 256, 0, lc.stream>>>(heavy_rows, nheavy, big_slot, tile_cnt, ntiles, A.rp, units, room,
                                              counters, flags);
 #define SPG_NU(R, S)                                                                                            \
-  num_unit_one<R, S>(A, B, units, room, counters, ntiles, c_rp, c_col, c_val, bidx, bitmap, stride, big_slot, \
-                     counters + 1, flags, lc)
+  num_unit_one<R, S>(A, B, units, room, counters, ntiles, c_rp, c_col, c_val, bidx, bitmap, stride, big_slot,   \
+                     tile_cnt, whole_max, counters + 1, flags, lc)
   if (B.rp32) {
     if (bitmap) SPG_NU(true, true);
     else SPG_NU(true, false);
