@@ -48,8 +48,14 @@ spg_status DevBuf::alloc_from(spg_ctx* ctx, size_t bytes, cudaMemPool_t pool) {
   reset();
   ctx_ = ctx;
   if (bytes == 0) return SPG_OK;
+  const cudaError_t before = cudaPeekAtLastError();
   cudaError_t e = cudaMallocFromPoolAsync(&ptr_, bytes, pool, ctx->stream);
   if (e == cudaErrorMemoryAllocation) {
+    // a launch refused earlier in the call stays its error
+    if (before != cudaSuccess) {
+      ptr_ = nullptr;
+      return cuda_status(ctx, before, "an earlier launch");
+    }
     // what either pool holds in reserve may be what the other lacks
     (void)cudaGetLastError();
     cudaStreamSynchronize(ctx->stream);

@@ -376,12 +376,14 @@ spg_status heavy_staged(spg_ctx* ctx, const DCsr& A, const DCsr& B, const int32_
   const size_t cnt_smem = (size_t)kStageWarps * ntiles * 4;
   const size_t tile_smem = (size_t)kTileWarps * kTileWarpWords * 4;
   const size_t off_smem = (size_t)ntiles * 4;
+  // one value for every call: the limit is shared by all threads' contexts
+  constexpr int kMostSmem = kStageWarps * kStageMaxTiles * 4;
   if (B.rp32) {
-    cudaFuncSetAttribute(k_heavy_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cnt_smem);
-    cudaFuncSetAttribute(k_heavy_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cnt_smem);
+    cudaFuncSetAttribute(k_heavy_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
+    cudaFuncSetAttribute(k_heavy_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
   } else {
-    cudaFuncSetAttribute(k_heavy_count<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cnt_smem);
-    cudaFuncSetAttribute(k_heavy_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cnt_smem);
+    cudaFuncSetAttribute(k_heavy_count<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
+    cudaFuncSetAttribute(k_heavy_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
   }
   cudaFuncSetAttribute(k_heavy_accumulate, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem);
   int acc_per_sm = 0, cs_per_sm = 0;

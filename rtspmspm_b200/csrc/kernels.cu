@@ -1688,13 +1688,20 @@ void launch_sym_block(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t
   else sym_block_one<false>(A, B, rows, nrows, log_table, slot_base, nnz, big_slot, tile_cnt, ntiles, flags, lc);
 }
 
+// Columns up to which rows take 512-thread CTAs, in bitmap words.
+constexpr int kNarrowWords = 12288;
+
 template <bool R32, int THREADS>
 static void sym_dense_one(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, int64_t slot_base,
                           int64_t* nnz, int32_t* big_slot, int32_t* tile_cnt, int ntiles, uint32_t* bitmap, int* flags,
                           int max_words, const LaunchCtx& lc) {
   auto kernel = k_sym_dense<R32, THREADS>;
   const size_t smem = (size_t)max_words * sizeof(uint32_t);
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit belongs to the kernel, not to the thread or its context: one
+  // value for every call, or a narrow product on another thread would lower it
+  // between this call and its launch
+  constexpr int kMostWords = THREADS == 512 ? kNarrowWords : kDenseWindowWords;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostWords * (int)sizeof(uint32_t));
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, smem);
   const int blocks = (int)std::min<int64_t>(nrows, (int64_t)lc.sms * std::max(1, per_sm));
@@ -1713,7 +1720,7 @@ void launch_sym_dense(const DCsr& A, const DCsr& B, const int32_t* rows, int64_t
   const int max_words = (int)std::min<int64_t>(kDenseWindowWords, (int64_t)ntiles * kTileWords);
 #define SPG_SD(R, T) \
   sym_dense_one<R, T>(A, B, rows, nrows, slot_base, nnz, big_slot, tile_cnt, ntiles, bitmap, flags, max_words, lc)
-  const bool narrow = max_words <= 12288;
+  const bool narrow = max_words <= kNarrowWords;
   if (B.rp32) {
     if (narrow) SPG_SD(true, 512);
     else SPG_SD(true, 1024);

@@ -116,9 +116,9 @@ __global__ void __launch_bounds__(256) k_sym_span(DCsr A, DCsr B, const int32_t*
 
 // CTAs of 4 warps, as many an SM as fit, no more than the rows need.
 constexpr int kSpanWarps = 4;
+static_assert(kSpanWarps * span_bin_words(kNumSpanBins - 1) * 4 <= 48 * 1024, "within every kernel's default limit");
 template <typename Kernel>
 static int span_grid(Kernel kernel, size_t smem, int64_t nrows, const LaunchCtx& lc) {
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSpanWarps * 32, smem);
   return (int)std::max<int64_t>(
