@@ -85,67 +85,48 @@ constexpr uint64_t kScratchIdle = uint64_t(4) << 30;
 struct ScratchPool {
   cudaMemPool_t pool = nullptr;
   unsigned long long driver_ctx = 0;  // the driver context it belongs to
-  int contexts = 0;
+  int contexts = 0;                   // of that driver context
 };
 std::mutex g_scratch_mutex;
 ScratchPool g_scratch[kMaxDevices];
 
-// A number of the current driver context that no other context of the process
-// has or had (a device reset ends one, and the pools in it), or 0.
-unsigned long long driver_ctx_id() {
-  void* get = nullptr;
-  void* id = nullptr;
-  cudaDriverEntryPointQueryResult r;
-  unsigned long long v = 0;
-  CUcontext cur = nullptr;
-  if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &get, cudaEnableDefault, &r) != cudaSuccess || !get ||
-      cudaGetDriverEntryPoint("cuCtxGetId", &id, cudaEnableDefault, &r) != cudaSuccess || !id) {
-    (void)cudaGetLastError();
-    return 0;
-  }
-  if (reinterpret_cast<decltype(&cuCtxGetCurrent)>(get)(&cur) != CUDA_SUCCESS || !cur) return 0;
-  if (reinterpret_cast<decltype(&cuCtxGetId)>(id)(cur, &v) != CUDA_SUCCESS) return 0;
-  return v;
-}
-
-// The device is current and its driver context exists.
-cudaError_t scratch_acquire(int device, cudaMemPool_t* out) {
+// The device is current and `driver_ctx` names its driver context.  Contexts
+// of an ended driver context (a device reset) are counted no more: their pool
+// went with it.
+cudaError_t scratch_acquire(int device, unsigned long long driver_ctx, cudaMemPool_t* out) {
   if (device >= kMaxDevices) return cudaDeviceGetDefaultMemPool(out, device);
   std::lock_guard<std::mutex> hold(g_scratch_mutex);
   ScratchPool& s = g_scratch[device];
-  if (s.contexts == 0) {
-    const unsigned long long now = driver_ctx_id();
-    if (s.pool && s.driver_ctx != now) s.pool = nullptr;  // gone with its driver context
-    if (!s.pool) {
-      cudaMemPoolProps props{};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = device;
-      cudaError_t e = cudaMemPoolCreate(&s.pool, &props);
-      if (e != cudaSuccess) {
-        s.pool = nullptr;
-        return e;
-      }
-      uint64_t keep = kScratchKeep;
-      e = cudaMemPoolSetAttribute(s.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-      if (e != cudaSuccess) {
-        cudaMemPoolDestroy(s.pool);
-        s.pool = nullptr;
-        return e;
-      }
-      s.driver_ctx = now;
+  if (s.driver_ctx != driver_ctx) s = ScratchPool{};
+  if (!s.pool) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaError_t e = cudaMemPoolCreate(&s.pool, &props);
+    if (e != cudaSuccess) {
+      s.pool = nullptr;
+      return e;
     }
+    uint64_t keep = kScratchKeep;
+    e = cudaMemPoolSetAttribute(s.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(s.pool);
+      s.pool = nullptr;
+      return e;
+    }
+    s.driver_ctx = driver_ctx;
   }
   ++s.contexts;
   *out = s.pool;
   return cudaSuccess;
 }
 
-void scratch_release(int device) {
+void scratch_release(int device, unsigned long long driver_ctx) {
   if (device >= kMaxDevices) return;
   std::lock_guard<std::mutex> hold(g_scratch_mutex);
   ScratchPool& s = g_scratch[device];
-  if (--s.contexts > 0) return;
+  if (s.driver_ctx != driver_ctx || s.contexts == 0 || --s.contexts > 0) return;
   if (s.driver_ctx != 0) {
     cudaMemPoolTrimTo(s.pool, kScratchIdle);
   } else {  // it could not be told from one of an ended context
@@ -155,6 +136,27 @@ void scratch_release(int device) {
 }
 
 }  // namespace
+
+unsigned long long driver_ctx_id() {
+  struct Entry {
+    void* current = nullptr;
+    void* id = nullptr;
+    Entry() {
+      cudaDriverEntryPointQueryResult r;
+      if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &current, cudaEnableDefault, &r) != cudaSuccess ||
+          cudaGetDriverEntryPoint("cuCtxGetId", &id, cudaEnableDefault, &r) != cudaSuccess || !id) {
+        (void)cudaGetLastError();
+        current = nullptr;
+      }
+    }
+  };
+  static const Entry entry;
+  unsigned long long v = 0;
+  CUcontext cur = nullptr;
+  if (!entry.current || reinterpret_cast<decltype(&cuCtxGetCurrent)>(entry.current)(&cur) != CUDA_SUCCESS || !cur)
+    return 0;
+  return reinterpret_cast<decltype(&cuCtxGetId)>(entry.id)(cur, &v) == CUDA_SUCCESS ? v : 0;
+}
 
 void DevBuf::reset() {
   if (ptr_ && ctx_) cudaFreeAsync(ptr_, ctx_->stream);
@@ -1120,7 +1122,8 @@ spg_status spg_create(spg_ctx** out, int32_t device) {
   SPG_CUDA(ctx.get(), cudaHostAlloc((void**)&ctx->h_stage, 64 * sizeof(int64_t), cudaHostAllocMapped));
   SPG_CUDA(ctx.get(), cudaHostGetDevicePointer((void**)&ctx->h_stage_dev, ctx->h_stage, 0));
   ctx->tuning = default_tuning();
-  SPG_CUDA(ctx.get(), scratch_acquire(device, &ctx->scratch));
+  ctx->driver_ctx = driver_ctx_id();
+  SPG_CUDA(ctx.get(), scratch_acquire(device, ctx->driver_ctx, &ctx->scratch));
   *out = ctx.release();
   return SPG_OK;
 }
@@ -1146,7 +1149,7 @@ spg_status spg_destroy(spg_ctx* ctx) {
   cudaEventDestroy(ctx->ev_start);
   cudaEventDestroy(ctx->ev_end);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
-  scratch_release(ctx->device);
+  scratch_release(ctx->device, ctx->driver_ctx);
   delete ctx;
   return SPG_OK;
 }

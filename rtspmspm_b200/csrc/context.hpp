@@ -24,6 +24,7 @@ struct spg_ctx {
   cudaStream_t upload_stream = nullptr;  // host-to-device copies of input row chunks (created on first use)
   cudaMemPool_t pool = nullptr;     // results (the device's default pool)
   cudaMemPool_t scratch = nullptr;  // a call's work memory (shared by the device's contexts)
+  unsigned long long driver_ctx = 0;  // driver_ctx_id() at its creation
   cudaEvent_t ev_start = nullptr, ev_end = nullptr;  // StageTimer's
   std::string last_error;
   std::string gpu_name;
@@ -129,7 +130,7 @@ class DevLayout {
   int n_ = 0;
 };
 
-inline LaunchCtx launch_ctx(const spg_ctx* ctx) { return LaunchCtx{ctx->stream, ctx->sms, ctx->device}; }
+inline LaunchCtx launch_ctx(const spg_ctx* ctx) { return LaunchCtx{ctx->stream, ctx->sms, ctx->device, ctx->driver_ctx}; }
 
 // Enqueues copies of `bytes` (a multiple of 4) device bytes each into the
 // mapped staging words at host_dst (inside ctx->h_stage), at most

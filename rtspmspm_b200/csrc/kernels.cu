@@ -1511,30 +1511,33 @@ struct LaunchShape {
 // The shape of a kernel instantiation and the shared memory it may ask for.
 // wpb <= 0 selects auto_wpb; its answer is computed once (the first device
 // that launches the kernel decides; all devices here are alike) and the
-// shared-memory limit is raised once a device, since the driver calls behind
-// both cost a small product as much as its launches.
+// shared-memory limit is raised once a driver context, since the driver calls
+// behind both cost a small product as much as its launches.
 class LaunchCache {
  public:
   template <typename Kernel>
-  LaunchShape get(Kernel kernel, int wpb, size_t smem_per_warp, int max_w, int device) {
-    const uint64_t bit = device < 64 ? uint64_t(1) << device : 0;
-    if (!(raised_.load(std::memory_order_acquire) & bit)) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess)
-        raised_.fetch_or(bit, std::memory_order_release);
+  LaunchShape get(Kernel kernel, int wpb, size_t smem_per_warp, int max_w, const LaunchCtx& lc) {
+    std::atomic<unsigned long long>* raised = lc.device < kDevices && lc.driver_ctx ? &raised_[lc.device] : nullptr;
+    if (!raised || raised->load(std::memory_order_acquire) != lc.driver_ctx) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess &&
+          raised)
+        raised->store(lc.driver_ctx, std::memory_order_release);
     }
     int packed = wpb > 0 ? 0 : shape_.load(std::memory_order_relaxed);
     if (packed == 0) {
       const int w = wpb > 0 ? std::min(wpb, max_w) : auto_wpb(kernel, smem_per_warp, max_w);
       int per_sm = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, w * 32, (size_t)w * smem_per_warp);
+      const cudaError_t e =
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, w * 32, (size_t)w * smem_per_warp);
       packed = w | (std::max(1, per_sm) << 8);
-      if (wpb <= 0) shape_.store(packed, std::memory_order_relaxed);
+      if (wpb <= 0 && e == cudaSuccess && per_sm > 0) shape_.store(packed, std::memory_order_relaxed);
     }
     return LaunchShape{packed & 0xff, packed >> 8};
   }
 
  private:
-  std::atomic<uint64_t> raised_{0};
+  static constexpr int kDevices = 64;
+  std::atomic<unsigned long long> raised_[kDevices] = {};  // the driver context it is raised in
   std::atomic<int> shape_{0};
 };
 
@@ -1564,8 +1567,8 @@ void launch_small_count(const DCsr& A, const DCsr& B, int64_t* prod, int64_t* nn
   const size_t per_warp = (size_t)(1u << kSmallLogT) * 4;
   static LaunchCache cache[2];
   const LaunchShape sh = B.rp32
-                             ? cache[1].get(k_small_count<true>, 0, per_warp, kSmallCountWarps, lc.device)
-                             : cache[0].get(k_small_count<false>, 0, per_warp, kSmallCountWarps, lc.device);
+                             ? cache[1].get(k_small_count<true>, 0, per_warp, kSmallCountWarps, lc)
+                             : cache[0].get(k_small_count<false>, 0, per_warp, kSmallCountWarps, lc);
   const int blocks = grid_for(A.rows, sh.wpb, 1, lc.sms * sh.per_sm);
   const size_t smem = sh.wpb * per_warp;
   if (B.rp32) k_small_count<true><<<blocks, sh.wpb * 32, smem, lc.stream>>>(A, B, prod, nnz, stop, flags);
@@ -1645,7 +1648,7 @@ static void sym_warp_one(const DCsr& A, const DCsr& B, const int32_t* rows, int6
                          const LaunchCtx& lc, int wpb) {
   static LaunchCache cache;
   const size_t per_warp = (size_t)(1 << LOGT) * sizeof(int32_t);
-  const LaunchShape sh = cache.get(k_sym_warp<LOGT, R32>, wpb, per_warp, wpb > 0 ? 16 : 8, lc.device);
+  const LaunchShape sh = cache.get(k_sym_warp<LOGT, R32>, wpb, per_warp, wpb > 0 ? 16 : 8, lc);
   const int blocks = grid_for(nrows, sh.wpb, 1, lc.sms * sh.per_sm);
   k_sym_warp<LOGT, R32><<<blocks, sh.wpb * 32, sh.wpb * per_warp, lc.stream>>>(A, B, rows, nrows, nnz, flags);
 }
@@ -1736,7 +1739,7 @@ static void num_warp_one(const DCsr& A, const DCsr& B, const int32_t* rows, int6
                          int32_t* c_col, float* c_val, int* flags, const LaunchCtx& lc, int wpb, const EscArgs& esc) {
   static LaunchCache cache;
   const size_t per_warp = (size_t)numeric_words<LOGT>() * 4;
-  const LaunchShape sh = cache.get(k_num_warp<LOGT, R32>, wpb, per_warp, wpb_for(LOGT, wpb > 0 ? 16 : 8), lc.device);
+  const LaunchShape sh = cache.get(k_num_warp<LOGT, R32>, wpb, per_warp, wpb_for(LOGT, wpb > 0 ? 16 : 8), lc);
   const int blocks = grid_for(nrows, sh.wpb, 1, lc.sms * sh.per_sm);
   k_num_warp<LOGT, R32><<<blocks, sh.wpb * 32, sh.wpb * per_warp, lc.stream>>>(A, B, rows, nrows, c_rp, c_col, c_val, esc.prod,
                                                                 esc.min_prod, flags);
@@ -1767,7 +1770,7 @@ static void num_warp_learned_one(const DCsr& A, const DCsr& B, const int32_t* ro
   static LaunchCache cache;
   const size_t per_warp = (size_t)numeric_words<LOGT>() * 4;
   const LaunchShape sh =
-      cache.get(k_num_warp_learned<LOGT, R32>, wpb, per_warp, wpb_for(LOGT, wpb > 0 ? 16 : 8), lc.device);
+      cache.get(k_num_warp_learned<LOGT, R32>, wpb, per_warp, wpb_for(LOGT, wpb > 0 ? 16 : 8), lc);
   const int blocks = grid_for(nrows, sh.wpb, 1, lc.sms * sh.per_sm);
   k_num_warp_learned<LOGT, R32><<<blocks, sh.wpb * 32, sh.wpb * per_warp, lc.stream>>>(A, B, rows, nrows, cap, slab_off, slab_col,
                                                                         slab_val, nnz_out, retry_rows, retry_count,
@@ -1806,7 +1809,7 @@ static void num_esc_one(int bin, const DCsr& A, const DCsr& B, const int32_t* ro
   const size_t per_warp = (size_t)words * 4;
   const int fit = std::min(8, (int)(200 * 1024 / per_warp));
   static LaunchCache cache[kNumEscBins];
-  const LaunchShape sh = cache[bin - kBinEsc].get(kernel, wpb, per_warp, fit, lc.device);
+  const LaunchShape sh = cache[bin - kBinEsc].get(kernel, wpb, per_warp, fit, lc);
   const int blocks = grid_for(nrows, sh.wpb, 1, lc.sms * sh.per_sm);
   kernel<<<blocks, sh.wpb * 32, sh.wpb * per_warp, lc.stream>>>(A, B, rows, nrows, prod, words, off, out_col, out_val, cap, nnz,
                                                       retry, retry_count, flags);

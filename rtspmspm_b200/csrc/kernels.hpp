@@ -117,7 +117,13 @@ struct LaunchCtx {
   cudaStream_t stream;
   int sms;
   int device;
+  unsigned long long driver_ctx;  // driver_ctx_id() of the device's context
 };
+
+// A number of the current driver context that no other context of the process
+// has or had, or 0.  A device reset ends a context and with it what was set or
+// made there: kernels' shared-memory limits, memory pools.
+unsigned long long driver_ctx_id();
 
 void launch_widen_rp(const int32_t* in, int64_t n, int64_t* out, const LaunchCtx& lc);
 void launch_narrow_rp(const int64_t* in, int64_t n, int32_t* out, const LaunchCtx& lc);

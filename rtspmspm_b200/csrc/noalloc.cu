@@ -140,7 +140,7 @@ extern "C" spg_status spg_multiply_noalloc(void* stream, const spg_csr* A, const
     return err(errbuf, errlen, st, "cudaGetSymbolAddress of the scratch array failed");
   int sms = 0;
   NA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const LaunchCtx lc{static_cast<cudaStream_t>(stream), sms, dev};
+  const LaunchCtx lc{static_cast<cudaStream_t>(stream), sms, dev, driver_ctx_id()};
   const cudaStream_t s = lc.stream;
   const int64_t rows = A->rows;
   int64_t* arp = reinterpret_cast<int64_t*>(base + kOffArp);
