@@ -72,15 +72,15 @@ spg_status DevBuf::alloc_from(spg_ctx* ctx, size_t bytes, cudaMemPool_t pool) {
 
 namespace {
 
-// One scratch pool a device, shared by its contexts.  It keeps up to
-// kScratchKeep bytes between calls (an R-MAT scale 18 product works in 3.5 GB,
-// scale 20 in 9 GB); more goes back to the device at the next synchronisation.
-// When the last context goes it keeps kScratchIdle of them for the next one: a
-// program with one context at a time would otherwise map its work memory anew
-// on each context's first call (ER 4096 0.3 -> 0.6 ms, 50,021 x 30,011 x
-// 70,001 0.8 -> 1.3 ms, R-MAT scale 18 53 -> 57 ms).
+// One scratch pool a device, shared by its contexts.  Between calls it keeps up
+// to half the device's memory (an R-MAT scale 18 product works in 3.5 GB, the
+// learned product of a 224^3 stencil in 15 GB; past the limit memory goes back at
+// every synchronisation and is mapped anew by every call: that product 60 -> 86
+// ms with 12 GB kept).  When the last context goes it keeps kScratchIdle bytes
+// for the next one: a program with one context at a time would otherwise map
+// its work memory anew on each context's first call (ER 4096 0.3 -> 0.6 ms,
+// 50,021 x 30,011 x 70,001 0.8 -> 1.3 ms, R-MAT scale 18 53 -> 57 ms).
 constexpr int kMaxDevices = 64;
-constexpr uint64_t kScratchKeep = uint64_t(12) << 30;
 constexpr uint64_t kScratchIdle = uint64_t(4) << 30;
 struct ScratchPool {
   cudaMemPool_t pool = nullptr;
@@ -93,7 +93,7 @@ ScratchPool g_scratch[kMaxDevices];
 // The device is current and `driver_ctx` names its driver context.  Contexts
 // of an ended driver context (a device reset) are counted no more: their pool
 // went with it.
-cudaError_t scratch_acquire(int device, unsigned long long driver_ctx, cudaMemPool_t* out) {
+cudaError_t scratch_acquire(int device, unsigned long long driver_ctx, uint64_t keep, cudaMemPool_t* out) {
   if (device >= kMaxDevices) return cudaDeviceGetDefaultMemPool(out, device);
   std::lock_guard<std::mutex> hold(g_scratch_mutex);
   ScratchPool& s = g_scratch[device];
@@ -108,7 +108,6 @@ cudaError_t scratch_acquire(int device, unsigned long long driver_ctx, cudaMemPo
       s.pool = nullptr;
       return e;
     }
-    uint64_t keep = kScratchKeep;
     e = cudaMemPoolSetAttribute(s.pool, cudaMemPoolAttrReleaseThreshold, &keep);
     if (e != cudaSuccess) {
       cudaMemPoolDestroy(s.pool);
@@ -1123,7 +1122,7 @@ spg_status spg_create(spg_ctx** out, int32_t device) {
   SPG_CUDA(ctx.get(), cudaHostGetDevicePointer((void**)&ctx->h_stage_dev, ctx->h_stage, 0));
   ctx->tuning = default_tuning();
   ctx->driver_ctx = driver_ctx_id();
-  SPG_CUDA(ctx.get(), scratch_acquire(device, ctx->driver_ctx, &ctx->scratch));
+  SPG_CUDA(ctx.get(), scratch_acquire(device, ctx->driver_ctx, prop.totalGlobalMem / 2, &ctx->scratch));
   *out = ctx.release();
   return SPG_OK;
 }
