@@ -16,7 +16,10 @@
  *    (spg_csr.index_bits).  Input rows must be sorted by column with no
  *    duplicates (spg_mtx_read produces that form from any .mtx file).
  *  - One context per host thread; calls on a context are ordered on its
- *    CUDA stream.  All memory the library allocates belongs to the context.
+ *    CUDA stream.  All memory the library allocates belongs to the context,
+ *    but for work memory: the contexts of a device share a pool for it, which
+ *    keeps up to half the device's memory between calls, and up to 4 GB when
+ *    the last of them is gone.  spg_trim_memory gives it back.
  *  - Values are accumulated in FP32 in the canonical per-row order (k
  *    ascending through A's row, then j ascending through B's row k; the
  *    product is rounded to FP32 before the add), so results are identical
@@ -132,6 +135,9 @@ typedef struct spg_report {
  * optixSpMSpM.cpp:174-187; cusparseCreate cuSparse/src/main.cpp:437). */
 spg_status spg_create(spg_ctx** ctx, int32_t device);
 spg_status spg_destroy(spg_ctx* ctx);
+/* Gives the device's work memory that no call is using back to the device
+ * (SPG_OK also when there is none); waits for the device's work first. */
+spg_status spg_trim_memory(int32_t device);
 const char* spg_last_error(const spg_ctx* ctx);
 const char* spg_status_string(spg_status status);
 /* Use a caller stream (cudaStream_t passed as void*); NULL restores the

@@ -111,6 +111,7 @@ SIGNATURES = [
     ("spg_status_string", ctypes.c_char_p, [ctypes.c_int32]),
     ("spg_create", ctypes.c_int32, [_P(_vp), ctypes.c_int32]),
     ("spg_destroy", ctypes.c_int32, [_vp]),
+    ("spg_trim_memory", ctypes.c_int32, [ctypes.c_int32]),
     ("spg_last_error", ctypes.c_char_p, [_vp]),
     ("spg_set_stream", ctypes.c_int32, [_vp, _vp]),
     ("spg_get_stream", _vp, [_vp]),

@@ -193,6 +193,12 @@ class Engine:
             self.L.spg_destroy(self.ctx)
             self.ctx = None
 
+    def trim_memory(self) -> None:
+        """Gives the device's work memory that no call is using back to the device."""
+        st = self.L.spg_trim_memory(self.device)
+        if st != _lib.SPG_OK:
+            raise SpgError(st, "spg_trim_memory")
+
     def __enter__(self):
         return self
 
