@@ -393,7 +393,6 @@ struct Pipeline {
   DevBuf nnz;         // int64 rows+1 (becomes C's row pointers)
   DevBuf span;        // int32 rows: span words (plain method)
   DevBuf tile_cnt;    // int32 nbig * ntiles
-  DevBuf tile_off;    // int32 nbig * ntiles
   DevBuf bitmap;      // uint32 nbig * bitmap_stride(), or empty
   int64_t h_off[kNumBins + 1] = {};
   int64_t nbig = 0;
@@ -500,7 +499,6 @@ struct Pipeline {
     if (nbig > 0) {
       const size_t tb = (size_t)nbig * ntiles * 4;
       SPG_TRY(tile_cnt.alloc(ctx, tb));
-      SPG_TRY(tile_off.alloc(ctx, tb));
       SPG_CUDA(ctx, cudaMemsetAsync(tile_cnt.get(), 0, tb, ctx->stream));
       // when one bitmap window holds a row and the budget all big rows'
       // bitmaps, every big row takes the bitmap kernel and leaves its bitmap
@@ -541,9 +539,6 @@ struct Pipeline {
     return st;
   }
 
-  // Numeric pass for the rows in the current (numeric) binning, into C.
-  // Numeric pass; `row_prod` (the rows' products, or nullptr) lets the warp
-  // bins take expand-sort-fold rows.
   // Expand-sort-fold settings from the tuning (esc_min_prod 0: the default
   // threshold, -1: off).
   EscArgs esc_args(const int64_t* row_prod) const {
@@ -561,13 +556,16 @@ struct Pipeline {
   // when the path does not apply (buckets or alignment).
   spg_status numeric_tiles(const int64_t* c_rp, int32_t* c_col, float* c_val, const int32_t* bidx, bool* done) {
     const int64_t nheavy = bin_size(kBinHeavy);
+    // rows with a slot: the symbolic pass's, or the bin's (value-only recompute)
+    const int64_t nslots = std::max(nbig, nheavy);
     if (tune.heavy_path == 2 && !bulk_aligned(B.view)) return SPG_OK;
     // the list of non-empty (row, tile) units for the tile kernel, when it
     // fits: rows of wide products touch a small part of their tiles
     const size_t work_bytes = (size_t)nheavy * (size_t)ntiles * 8;
     const bool use_list = tune.heavy_path == 2 && ntiles > 1 && work_bytes <= kWorkListMaxBytes &&
                           room_for(work_bytes, 4);
-    DevBuf nz, work;
+    DevBuf nz, work, tile_off;  // tile_off: int32, as tile_cnt
+    SPG_TRY(tile_off.alloc(ctx, (size_t)nslots * (size_t)ntiles * 4));
     if (use_list) SPG_TRY(nz.alloc(ctx, (size_t)(nheavy + 1) * 8));
     launch_tile_offsets(bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles,
                         tile_off.as<int32_t>(), use_list ? nz.as<int64_t>() : nullptr, lc);
@@ -597,6 +595,9 @@ struct Pipeline {
     return SPG_OK;
   }
 
+  // Numeric pass for the rows in the current (numeric) binning, into C (c_nnz
+  // entries); `row_prod` (the rows' products, or nullptr) lets the warp bins
+  // take expand-sort-fold rows.
   spg_status numeric(const int64_t* c_rp, int32_t* c_col, float* c_val, int64_t c_nnz, spg_report* rep,
                      const int64_t* row_prod = nullptr) {
     const EscArgs esc = esc_args(row_prod);
@@ -1033,7 +1034,6 @@ spg_status multiply_reuse_device(spg_ctx* ctx, const DevMat& A, const DevMat& B,
     if (nheavy > 0) {
       const size_t tb = (size_t)nheavy * P.ntiles * 4;
       SPG_TRY(P.tile_cnt.alloc(ctx, tb));
-      SPG_TRY(P.tile_off.alloc(ctx, tb));
       SPG_CUDA(ctx, cudaMemsetAsync(P.tile_cnt.get(), 0, tb, ctx->stream));
       launch_tile_counts_from_cols(P.bin_rows(kBinHeavy), nheavy, P.nnz.as<int64_t>(), C->col_idx, P.ntiles,
                                    P.big_slot.as<int32_t>(), P.tile_cnt.as<int32_t>(), ctx->d_flags, lc);

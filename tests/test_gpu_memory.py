@@ -1,4 +1,6 @@
-"""Work memory kept between calls goes back to the device on request."""
+"""Work memory: what a call takes, and that what is kept between calls goes back
+to the device on request."""
+import numpy as np
 import pytest
 
 from rtspmspm_b200 import DeviceCsr, Engine, _lib, gen
@@ -34,3 +36,25 @@ def test_trim_memory_gives_work_memory_back():
     assert L.spg_trim_memory(0) == _lib.SPG_OK
     assert L.spg_trim_memory(-1) == _lib.SPG_ERR_INVALID_ARG
     assert L.spg_trim_memory(1 << 20) == _lib.SPG_ERR_INVALID_ARG
+
+
+def test_heavy_rows_take_one_word_a_tile():
+    """40,000 heavy rows over 684 column tiles (past the width of the stored
+    bitmaps): their tile counts are 109 MB, the rest of the call's work memory
+    some 30 MB."""
+    rows, per, cols = 40000, 1100, 1400000
+    rng = np.random.default_rng(0)
+    b = np.sort(rng.integers(0, cols, (64, per)), axis=1)
+    B = gen.coo_to_csr(64, cols, np.repeat(np.arange(64), per), b.ravel(), np.ones(64 * per, np.float32))
+    A = gen.coo_to_csr(rows, 64, np.repeat(np.arange(rows), 2), np.arange(2 * rows) % 64,
+                       np.ones(2 * rows, np.float32))
+    with Engine(0) as eng:
+        dA, dB = DeviceCsr.from_host(A), DeviceCsr.from_host(B)
+        eng.trim_memory()
+        C, rep = eng.multiply(dA, dB, algo="plain", skip_validation=True)
+        assert rep["rows_heavy"] == rows
+        held = _free()
+        eng.trim_memory()
+        took = _free() - held
+        assert (100 << 20) < took < (200 << 20), took
+        C.free()
