@@ -434,20 +434,30 @@ struct Pipeline {
   // Big rows of the last symbolic binning, and whether their bitmaps fit the
   // budget.
   int64_t big_rows() const { return bin_size(kBinBlock) + bin_size(kBinDense); }
+  size_t bitmap_bytes() const { return (size_t)big_rows() * (size_t)bitmap_stride() * 4; }
   bool bitmaps_fit() const {
-    const size_t bytes = (size_t)big_rows() * (size_t)bitmap_stride() * 4;
-    return tune.heavy_path == 0 && bitmap_stride() <= kDenseWindowWords && bytes <= kBitmapMaxBytes && room_for(bytes, 8);
+    return tune.heavy_path == 0 && bitmap_stride() <= kDenseWindowWords && bitmap_bytes() <= kBitmapMaxBytes &&
+           room_for(bitmap_bytes(), 8);
   }
 
-  // True when `bytes` are less than a part of the device's free memory.  The
-  // driver's answer can take a millisecond, so a few tens of MB are not asked
-  // about.
-  static bool room_for(size_t bytes, size_t part) {
+  // True when `bytes` of work memory are already mapped and free, or less than a
+  // part of the device's free memory.  The driver is asked for that only when
+  // the pool has to grow: its answer takes 0.1 ms on a quiet machine and tens
+  // on a busy one (R-MAT 16: calls of 6 ms took 6 to 89).
+  bool room_for(size_t bytes, size_t part) const {
     if (bytes <= (size_t(64) << 20)) return true;
+    uint64_t reserved = 0, used = 0;
+    if (cudaMemPoolGetAttribute(ctx->scratch, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        cudaMemPoolGetAttribute(ctx->scratch, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+        reserved >= used && reserved - used >= bytes)
+      return true;
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     return bytes < free_b / part;
   }
+
+  // The status of an allocation that the call can do without.
+  static spg_status optional(spg_status st) { return st == SPG_ERR_OUT_OF_MEMORY ? SPG_OK : st; }
 
   void bin(const int64_t* key, int mode, const EscArgs& esc = EscArgs{}) {
     launch_binning(key, rows, cols, mode, bp, bin_of_row.as<uint8_t>(), counts(), offsets(), cursors(),
@@ -477,11 +487,14 @@ struct Pipeline {
   spg_status symbolic(const int64_t* key) {
     bin(key, kBinSymbolic);
     SPG_TRY(fetch_offsets());
-    if (big_rows() > 0 && bp.heavy_min < bp.warp_cap && !bitmaps_fit()) {
-      // only rows with a stored bitmap gain from leaving the warp tables early
+    bool fit = big_rows() > 0 && bitmaps_fit();
+    // only rows with a stored bitmap gain from leaving the warp tables early
+    // (past 128 * warp_cap columns none does, big_row)
+    if (big_rows() > 0 && !fit && bp.heavy_min < bp.warp_cap && cols <= 128 * bp.warp_cap) {
       bp.heavy_min = INT64_MAX;
       bin(key, kBinSymbolic);
       SPG_TRY(fetch_offsets());
+      fit = big_rows() > 0 && bitmaps_fit();
     }
     for (int b = kBinSpan; b < kBinSpan + kNumSpanBins; ++b) {
       if (bin_size(b) == 0) continue;
@@ -503,7 +516,7 @@ struct Pipeline {
       // when one bitmap window holds a row and the budget all big rows'
       // bitmaps, every big row takes the bitmap kernel and leaves its bitmap
       // for the units (which else walk their products once more for it)
-      if (bitmaps_fit()) SPG_TRY(bitmap.alloc(ctx, (size_t)nbig * (size_t)bitmap_stride() * 4));
+      if (fit) SPG_TRY(optional(bitmap.alloc(ctx, bitmap_bytes())));
       if (bitmap.get()) {
         launch_sym_dense(A.view, B.view, bin_rows(kBinBlock), nbig, 0, nnz.as<int64_t>(), big_slot.as<int32_t>(),
                          tile_cnt.as<int32_t>(), ntiles, bitmap.as<uint32_t>(), ctx->d_flags, lc);
@@ -629,7 +642,9 @@ struct Pipeline {
       const size_t bidx_bytes = (size_t)B.view.rows * (size_t)(ntiles + 1) * 4;
       const bool use_index = ntiles > 1 && bidx_bytes <= kBlockedIndexMaxBytes && room_for(bidx_bytes, 4);
       if (use_index) {
-        SPG_TRY(bidx.alloc(ctx, bidx_bytes));
+        SPG_TRY(optional(bidx.alloc(ctx, bidx_bytes)));
+      }
+      if (bidx.get()) {
         launch_build_blocked_index(B.view, ntiles, bidx.as<int32_t>(), lc);
         ++ctx->launches;
       }
