@@ -101,6 +101,11 @@ typedef struct spg_opts {
 #define SPG_STAGE_DOWNLOAD  10
 #define SPG_STAGE_COUNT     12
 
+/* Indices of spg_report.bin_rows: 0 to 7 the warp hash tables of 2^5 to 2^12
+ * slots, 8 and 9 the CTA-wide ones, then: */
+#define SPG_BIN_HEAVY 10  /* heavy rows */
+#define SPG_BIN_EMPTY 11  /* rows without products, or not of this pass */
+#define SPG_BIN_FOLD  12  /* rows expanded, sorted and folded in launches of their own */
 #define SPG_NUM_BINS 16
 
 /*
@@ -116,7 +121,7 @@ typedef struct spg_report {
     int64_t rows_predicted;             /* learned: rows sized by the MLP */
     int64_t rows_overflow;              /* learned: rows re-run by the exact fallback */
     int64_t rows_heavy;                 /* rows on the column-tiled heavy path */
-    int64_t bin_rows[SPG_NUM_BINS];     /* numeric rows per accumulator bin */
+    int64_t bin_rows[SPG_NUM_BINS];     /* rows per accumulator of the exact numeric pass */
     int32_t algo;
     int32_t device_flags;               /* bit set of SPG_FLAG_* raised by kernels */
     int32_t kernel_launches;            /* launches issued by this call */

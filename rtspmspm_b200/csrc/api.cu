@@ -662,7 +662,10 @@ struct Pipeline {
       ++ctx->launches;
     }
     if (rep) {
-      for (int b = 0; b < kNumBins && b < SPG_NUM_BINS; ++b) rep->bin_rows[b] += bin_size(b);
+      for (int b = 0; b < kBinEsc; ++b) rep->bin_rows[b] += bin_size(b);
+      rep->bin_rows[SPG_BIN_HEAVY] += nheavy;
+      rep->bin_rows[SPG_BIN_EMPTY] += bin_size(kBinEmpty);
+      for (int b = kBinEsc; b < kBinEsc + kNumEscBins; ++b) rep->bin_rows[SPG_BIN_FOLD] += bin_size(b);
       rep->rows_heavy += nheavy;
     }
     return SPG_OK;
