@@ -291,6 +291,10 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_mlp_predict(const __nv_bflo
 // bin_gate, its predicted bin says beyond the warp tables, or when it is past
 // heavy_min and the heavy-row units take it (big_row) but not the fold;
 // force_overflow sets cap = 1 (every row then overflows and is re-run).
+// UNITS: there are heavy-row units (none in a batch, whose plan keeps its 61
+// registers without them, four CTAs an SM: 20 products of 20,000 rows 222 us,
+// with them 269).
+template <bool UNITS>
 __device__ __forceinline__ void capacity_of(int64_t p, int64_t cols, float o0, float o1, float margin, int slack,
                                             int64_t learn_cap, int bin_gate, int force_overflow, int64_t heavy_min,
                                             int esc_min, int64_t& cap, uint8_t& ex) {
@@ -304,7 +308,7 @@ __device__ __forceinline__ void capacity_of(int64_t p, int64_t cols, float o0, f
   int64_t c = cd >= (double)u ? u : (int64_t)cd;
   if (c < 1) c = 1;
   if (force_overflow) c = 1;
-  const bool units = c > heavy_min && big_row(c, cols, learn_cap, heavy_min) &&
+  const bool units = UNITS && c > heavy_min && big_row(c, cols, learn_cap, heavy_min) &&
                      !(fold_big(p, (int64_t)pred) && esc_wanted(p, c, esc_min, esc_bin_products(kNumEscBins - 1)));
   if (c > learn_cap || units || (bin_gate && o1 > (float)kMaxLogT + 0.5f)) {
     ex = 1;
@@ -374,7 +378,7 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_learned_plan(DCsr A, DCsr B
       if (ra < rows) {
         int64_t c;
         uint8_t ex;
-        capacity_of(tprod[wib][ia], tcols[wib][ia], o[0], o[1], margin, slack, learn_cap, bin_gate, force_overflow,
+        capacity_of<!BATCH>(tprod[wib][ia], tcols[wib][ia], o[0], o[1], margin, slack, learn_cap, bin_gate, force_overflow,
                     heavy_min, esc_min, c, ex);
         prod[ra] = tprod[wib][ia];
         cap[ra] = c;
@@ -384,7 +388,7 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_learned_plan(DCsr A, DCsr B
       if (rb < rows) {
         int64_t c;
         uint8_t ex;
-        capacity_of(tprod[wib][ib], tcols[wib][ib], o[2], o[3], margin, slack, learn_cap, bin_gate, force_overflow,
+        capacity_of<!BATCH>(tprod[wib][ib], tcols[wib][ib], o[2], o[3], margin, slack, learn_cap, bin_gate, force_overflow,
                     heavy_min, esc_min, c, ex);
         prod[rb] = tprod[wib][ib];
         cap[rb] = c;
