@@ -206,6 +206,7 @@ BinParams bin_params(const spg_tuning& t) {
   // symbolic CTA table at load <= 2/3
   int blg = ilog2_floor(std::max(1024, std::min(32768, t.block_table_max)));
   bp.block_cap = ((int64_t)1 << blg) * 2 / 3;
+  bp.esc_prod = esc_bin_products(kNumEscBins - 1);
   // CTA-wide numeric hash bins (tables at load <= 1/2: their key and
   // order-word arrays are the row sort's buffers) for rows of more than
   // block_min_nnz entries, when set: measured slower than the warp tables
@@ -552,12 +553,10 @@ struct Pipeline {
     return st;
   }
 
-  // Expand-sort-fold settings from the tuning (esc_min_prod 0: the default
-  // threshold, -1: off).
   EscArgs esc_args(const int64_t* row_prod) const {
     EscArgs e;
     e.prod = row_prod;
-    e.min_prod = tune.esc_min_prod < 0 ? 0 : (tune.esc_min_prod == 0 ? kEscMinProd : tune.esc_min_prod);
+    e.min_prod = esc_min_products(tune);
     return e;
   }
 

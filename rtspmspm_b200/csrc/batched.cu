@@ -425,6 +425,15 @@ constexpr int kQSymSmall = 0, kQSymLarge = 1, kQNumSmall = 2, kQNumMid = 3, kQNu
 // beyond the queue's tables: their products run one by one instead.
 constexpr int64_t kBatchMaxBound = 4096;
 constexpr int kBatchCtaLogT = 13;  // CTA tables: 2^13 slots at load <= 1/2
+// Expand-sort-fold bins of a batch, up to 2,048 products: longer rows run
+// faster in the CTA tables.  Eight products of 3,000 rows of 1,600 | 2,500 |
+// 3,600 products with 77 to 98 | 68 to 82 | 66 to 91 % of them distinct, plain:
+// folded 2.1 to 2.4 | 4.9 to 5.0 | 7.1 to 7.7 ms a call, in the tables 2.7 to 3.5
+// | 3.4 to 3.9 | 4.5 to 6.4.
+constexpr int kBatchEscBins = 4;
+// The learned method's, up to 1,152 products: of the rows of 1,600 above 4.12 and
+// 4.45 ms folded, 3.98 and 4.48 in the tables.
+constexpr int kBatchEscBinsLearned = 3;
 
 BatchQueue queue_of(int which) {
   BatchQueue q{};
@@ -521,6 +530,7 @@ size_t esc_smem(int i) { return (size_t)esc_warps(i) * esc_bin_words(esc_bin_pro
 
 struct BatchPlan {
   int64_t max_cols = 1;                 // most columns of a batched product
+  int esc_bins = 0;                     // expand-sort-fold bins in use
   int esc_grid[2][kNumEscBins] = {};    // CTAs of each expand-sort-fold launch (plain, learned form)
   std::vector<uintptr_t> key;
   int n = 0;
@@ -647,7 +657,7 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
     a.c_val = p->c_val;
     a.lo = lo;
     a.prod = p->prod;
-    a.esc_min = p->tune.esc_min_prod < 0 ? 0 : (p->tune.esc_min_prod == 0 ? kEscMinProd : p->tune.esc_min_prod);
+    a.esc_min = esc_min_products(p->tune);
     a.counter = p->qcount + which;
     a.flags = ctx->d_flags;
     cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), lc.stream);
@@ -657,10 +667,9 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
   };
   EscArgs esc;
   esc.prod = p->prod;
-  esc.min_prod = p->tune.esc_min_prod < 0 ? 0 : (p->tune.esc_min_prod == 0 ? kEscMinProd : p->tune.esc_min_prod);
+  esc.min_prod = esc_min_products(p->tune);
   auto run_esc = [&](bool learned) {
-    if (esc.min_prod == 0) return;
-    for (int i = kNumEscBins - 1; i >= 0; --i) {
+    for (int i = p->esc_bins - 1; i >= 0; --i) {
       const int threads = esc_warps(i) * 32, grid = p->esc_grid[learned ? 1 : 0][i];
       const int words = esc_bin_words(esc_bin_products(i));
       if (learned)
@@ -848,6 +857,7 @@ spg_status build_plan(spg_ctx* ctx, int n, const spg_csr* A, const spg_csr* B, c
   // products with rows beyond the queue's tables go through the single path
   int64_t cbase = 0, rpbase = 0;
   p->c_base.assign((size_t)n, 0);
+  int64_t most = 0;  // largest bound of a batched row
   for (int m = 0; m < n; ++m) {
     BatchMat& M = p->mats[(size_t)m];
     // the persistent kernels use 32-bit row offsets of B (nnz(B) < 2^31)
@@ -858,6 +868,7 @@ spg_status build_plan(spg_ctx* ctx, int n, const spg_csr* A, const spg_csr* B, c
     } else {
       p->batched.push_back(m);
       p->max_cols = std::max(p->max_cols, M.B.cols);
+      most = std::max(most, (int64_t)hmax[(size_t)m]);
     }
     M.c_base = cbase;
     M.rp_base = rpbase;
@@ -865,6 +876,13 @@ spg_status build_plan(spg_ctx* ctx, int n, const spg_csr* A, const spg_csr* B, c
     if ((int64_t)hmax[(size_t)m] <= kBatchMaxBound && M.B.rp32) cbase += (int64_t)hsum[(size_t)m];
     rpbase += A[m].rows + 1;
   }
+  // a folded row has at most twice as many products as its bound; bins past
+  // that are not launched (3 us each) and get no row
+  const int esc_min = esc_min_products(p->tune);
+  const int esc_bins = p->learned ? kBatchEscBinsLearned : kBatchEscBins;
+  for (int low = esc_min - 1; esc_min > 0 && p->esc_bins < esc_bins && low < 2 * most;)
+    low = esc_bin_products(p->esc_bins++);
+  p->bp_num.esc_prod = p->bp_lrn.esc_prod = p->esc_bins > 0 ? esc_bin_products(p->esc_bins - 1) : 0;
   if (!p->individual.empty()) {
     // rows of individually-run products are removed from the global space
     std::vector<int32_t> keep_rows;

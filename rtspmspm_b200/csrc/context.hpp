@@ -132,6 +132,11 @@ class DevLayout {
 
 inline LaunchCtx launch_ctx(const spg_ctx* ctx) { return LaunchCtx{ctx->stream, ctx->sms, ctx->device, ctx->driver_ctx}; }
 
+// Smallest product count of an expand-sort-fold row (0: none is folded).
+inline int esc_min_products(const spg_tuning& t) {
+  return t.esc_min_prod < 0 ? 0 : (t.esc_min_prod == 0 ? kEscMinProd : t.esc_min_prod);
+}
+
 // Enqueues copies of `bytes` (a multiple of 4) device bytes each into the
 // mapped staging words at host_dst (inside ctx->h_stage), at most
 // StageCopies::kMax in one launch; valid after the next stream

@@ -151,7 +151,7 @@ __device__ __forceinline__ int bin_of(int64_t key, int64_t cols, int mode, const
   // the symbolic pass counted the tiles of the rows it found big
   const bool heavy = mode == kBinNumeric && key > bp.heavy_min && !spanned &&
                      big_row(u, cols, bp.warp_cap, bp.heavy_min);
-  if (key <= bp.esc_cap && (!heavy || fold_big(prod, key)) && esc_wanted(prod, key, esc_min, esc_bin_products(kNumEscBins - 1)) &&
+  if (key <= bp.esc_cap && (!heavy || fold_big(prod, key)) && esc_wanted(prod, key, esc_min, bp.esc_prod) &&
       ceil_log2_i64(cols) + ceil_log2_i64(prod) <= 31) {
     int b = 0;
     while (prod > esc_bin_products(b)) ++b;

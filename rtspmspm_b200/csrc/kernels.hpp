@@ -72,6 +72,7 @@ struct BinParams {
   int64_t blk_small_cap;
   int64_t blk_large_cap;
   int64_t esc_cap;     // most entries of a row in the expand-sort-fold bins
+  int esc_prod;        // and most products (esc_bin_products of the last bin in use; 0: none)
   int64_t heavy_min;   // rows of more entries may be heavy below warp_cap too (big_row)
 };
 
