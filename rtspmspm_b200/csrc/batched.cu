@@ -85,16 +85,32 @@ struct BatchQueue {
   int rows_per_tile[kQueueMax];
 };
 
-// tile_pref[i] = tiles of queue slots before i (tile_pref[nq] = all).
-__global__ void k_queue_prefix(const int64_t* bin_off, BatchQueue q, int64_t* tile_pref) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
+// The queues that one binning feeds.
+constexpr int kGroupMax = 3;
+struct QueueGroup {
+  int n;
+  int which[kGroupMax];  // number of each queue
+  BatchQueue q[kGroupMax];
+};
+
+// Queue w of the group: tile_pref[w][i] = tiles of its slots before i
+// (tile_pref[w][nq] = all) and its ticket counter set to zero.  One launch a
+// group, a thread a queue: a launch and a memset less for each of the other
+// queues pay for the expand-sort-fold launches in a batch of small products.
+__global__ void k_queue_prefix(const int64_t* bin_off, QueueGroup g, int64_t* tile_pref,
+                               unsigned long long* counter) {
+  if (blockIdx.x == 0 && (int)threadIdx.x < g.n) {
+    const BatchQueue& q = g.q[threadIdx.x];
+    const int w = g.which[threadIdx.x];
+    int64_t* pref = tile_pref + w * (kQueueMax + 1);
     int64_t t = 0;
     for (int i = 0; i < q.nq; ++i) {
-      tile_pref[i] = t;
+      pref[i] = t;
       const int64_t rows = bin_off[q.bins[i] + 1] - bin_off[q.bins[i]];
       t += (rows + q.rows_per_tile[i] - 1) / q.rows_per_tile[i];
     }
-    tile_pref[q.nq] = t;
+    pref[q.nq] = t;
+    counter[w] = 0ull;
   }
 }
 
@@ -660,10 +676,18 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
     a.esc_min = esc_min_products(p->tune);
     a.counter = p->qcount + which;
     a.flags = ctx->d_flags;
-    cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), lc.stream);
-    k_queue_prefix<<<1, 32, 0, lc.stream>>>(offsets, a.q, const_cast<int64_t*>(a.tile_pref));
     queue_dispatch(which, learned, &a, p->grid[learned ? 1 : 0][which], queue_smem(which), lc.stream);
-    launches += 2;
+    ++launches;
+  };
+  auto run_queues = [&](std::initializer_list<int> group, bool learned) {
+    QueueGroup g{};
+    for (int which : group) {
+      g.which[g.n] = which;
+      g.q[g.n++] = queue_of(which);
+    }
+    k_queue_prefix<<<1, 32, 0, lc.stream>>>(offsets, g, p->tile_pref, p->qcount);
+    ++launches;
+    for (int which : group) run_queue(which, learned);
   };
   EscArgs esc;
   esc.prod = p->prod;
@@ -687,8 +711,7 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
     launch_binning(sym_key, R, INT64_MAX, kBinSymbolic, p->bp_sym, p->bin_of_row, counts, offsets, cursors,
                    p->lists, lc);
     launches += 3;
-    run_queue(kQSymLarge, false);
-    run_queue(kQSymSmall, false);
+    run_queues({kQSymLarge, kQSymSmall}, false);
   };
   if (!p->learned) {
     exact_stages(p->bound);
@@ -697,9 +720,7 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
     launch_excl_scan(p->nnz, R, p->nnz, p->scan_tmp, lc);
     launches += 7;
     run_esc(false);
-    run_queue(kQNumLarge, false);
-    run_queue(kQNumMid, false);
-    run_queue(kQNumSmall, false);
+    run_queues({kQNumLarge, kQNumMid, kQNumSmall}, false);
   } else {
     cudaMemsetAsync(p->lcount, 0, 2 * sizeof(unsigned long long), lc.stream);
     cudaMemsetAsync(p->need, 0, (size_t)std::max<int64_t>(R, 1), lc.stream);
@@ -710,9 +731,7 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
     launch_excl_scan(p->cap, R, p->slab_off, p->scan_tmp, lc);
     launches += 8;
     run_esc(true);
-    run_queue(kQNumLarge, true);
-    run_queue(kQNumMid, true);
-    run_queue(kQNumSmall, true);
+    run_queues({kQNumLarge, kQNumMid, kQNumSmall}, true);
     // the exact path for rows predicted beyond the tables and overflowed rows
     launch_mark_rows(p->retry, p->lcount + 1, p->need, lc);
     launch_mask_key(p->bound, p->need, R, p->mkey, lc);
@@ -723,9 +742,7 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
                    lc);
     launch_excl_scan(p->nnz, R, p->nnz, p->scan_tmp, lc);
     launches += 8;
-    run_queue(kQNumLarge, false);
-    run_queue(kQNumMid, false);
-    run_queue(kQNumSmall, false);
+    run_queues({kQNumLarge, kQNumMid, kQNumSmall}, false);
     k_batch_compact<<<blocks_for(R, 8), 256, 0, lc.stream>>>(p->d_mats, p->row_mat, R, p->need, p->slab_off,
                                                             p->slab_col, p->slab_val, p->nnz, p->c_col, p->c_val);
     ++launches;
