@@ -84,8 +84,9 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_hist(CooIn in, int64_t n
 // to count and scan (2^26 entries: 6.5 against 6.0 ms a call), 1,024 and 16
 // entries a lane were slower.  off:
 // exclusive scan of hist (digit-major), the first output position of each
-// (digit, tile).  Dynamic shared memory: kSortTile keys and values.
-template <bool FIRST>
+// (digit, tile).  ALONE: the only tile, which needs none (one entry: 82 -> 68 us a
+// call) and raises the flags that the counting kernel does.  Dynamic shared memory: kSortTile keys and values.
+template <bool FIRST, bool ALONE>
 __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(CooIn in, int64_t n, int shift, int64_t ntiles,
                                                                 const int64_t* off, uint64_t* kout, float* vout) {
   __shared__ int base[kSortWarps][kDigits];
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(CooIn in, int64_
 #pragma unroll
   for (int j = 0; j < kSortItems; ++j) {
     const int64_t i = w0 + j * 32 + lane;
-    k[j] = i < n ? entry_key<FIRST>(in, i, false) : 0;
+    k[j] = i < n ? entry_key<FIRST>(in, i, ALONE) : 0;
     v[j] = i < n ? in.val[i] : 0.f;
   }
   // the warp's count per digit and, from the counts so far, each entry's rank
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(CooIn in, int64_
   for (int q = threadIdx.x; q < cnt; q += kSortThreads) {
     const uint64_t key = sk[q];
     const int d = (int)((key >> shift) & 0xffu);
-    const int64_t pos = off[(int64_t)d * ntiles + blockIdx.x] + (q - first[d]);
+    const int64_t pos = ALONE ? q : off[(int64_t)d * ntiles + blockIdx.x] + (q - first[d]);
     kout[pos] = key;
     vout[pos] = sv[q];
   }
@@ -265,17 +266,21 @@ spg_status coo_to_csr_device(spg_ctx* ctx, int64_t rows, int64_t cols, int64_t n
   std::vector<int> shifts;
   for (int s = 0; s < cbits; s += 8) shifts.push_back(s);
   for (int s = 0; s < rbits; s += 8) shifts.push_back(32 + s);
-  if (shifts.empty()) shifts.push_back(0);  // a 1 x 1 matrix: the pass checks the entries and makes their keys
+  // a 1 x 1 matrix or a single entry: one pass that checks the entries and makes their keys
+  if (shifts.empty() || n == 1) shifts.assign(1, 0);
   CooIn in{ri, ci, rows, cols, ctx->d_flags, nullptr, vi};
   const uint64_t* kin = nullptr;  // the sorted entries
   const float* vin = nullptr;
   if (n > 0) {
     uint64_t* kout = k0.as<uint64_t>();
     float* vout = v0.as<float>();
+    const bool alone = ntiles == 1;
     auto pass = [&](auto hist_kernel, auto scatter_kernel, int shift) -> spg_status {
       SPG_CUDA(ctx, cudaFuncSetAttribute(scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kScatterSmem));
-      hist_kernel<<<(unsigned)ntiles, kSortThreads, 0, lc.stream>>>(in, n, shift, ntiles, hist.as<int64_t>());
-      launch_excl_scan(hist.as<int64_t>(), kDigits * ntiles, hist.as<int64_t>(), tmp.as<int64_t>(), lc);
+      if (!alone) {
+        hist_kernel<<<(unsigned)ntiles, kSortThreads, 0, lc.stream>>>(in, n, shift, ntiles, hist.as<int64_t>());
+        launch_excl_scan(hist.as<int64_t>(), kDigits * ntiles, hist.as<int64_t>(), tmp.as<int64_t>(), lc);
+      }
       scatter_kernel<<<(unsigned)ntiles, kSortThreads, kScatterSmem, lc.stream>>>(in, n, shift, ntiles,
                                                                                   hist.as<int64_t>(), kout, vout);
       in.key = kin = kout;
@@ -285,8 +290,10 @@ spg_status coo_to_csr_device(spg_ctx* ctx, int64_t rows, int64_t cols, int64_t n
       return SPG_OK;
     };
     for (size_t i = 0; i < shifts.size(); ++i) {
-      if (i == 0) SPG_TRY(pass(k_radix_hist<true>, k_radix_scatter<true>, shifts[i]));
-      else SPG_TRY(pass(k_radix_hist<false>, k_radix_scatter<false>, shifts[i]));
+      const auto first = alone ? k_radix_scatter<true, true> : k_radix_scatter<true, false>;
+      const auto later = alone ? k_radix_scatter<false, true> : k_radix_scatter<false, false>;
+      if (i == 0) SPG_TRY(pass(k_radix_hist<true>, first, shifts[i]));
+      else SPG_TRY(pass(k_radix_hist<false>, later, shifts[i]));
     }
   }
   // runs of equal keys -> unique entries
