@@ -397,6 +397,7 @@ struct Pipeline {
   DevBuf bitmap;      // uint32 nbig * bitmap_stride(), or empty
   int64_t h_off[kNumBins + 1] = {};
   int64_t nbig = 0;
+  bool c_known = false;   // the units take their columns from C (value-only recompute, first pass)
   int64_t whole_max = 0;  // launch_num_units' whole_max (value-only recompute)
 
   Pipeline(spg_ctx* c, const DevMat& a, const DevMat& b, const spg_tuning& t)
@@ -654,8 +655,8 @@ struct Pipeline {
         DevBuf units;
         SPG_TRY(units.alloc(ctx, (size_t)room * sizeof(int4)));
         launch_num_units(A.view, B.view, bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(),
-                         ntiles, c_rp, c_col, c_val, bidx.as<int32_t>(), bitmap.as<uint32_t>(), bitmap_stride(), whole_max,
-                         units.as<int4>(), room, ctx->d_counter + 8, ctx->d_flags, lc);
+                         ntiles, c_rp, c_col, c_val, bidx.as<int32_t>(), bitmap.as<uint32_t>(), bitmap_stride(),
+                         c_known, whole_max, units.as<int4>(), room, ctx->d_counter + 8, ctx->d_flags, lc);
         ++ctx->launches;
       }
       ++ctx->launches;
@@ -1045,6 +1046,7 @@ spg_status multiply_reuse_device(spg_ctx* ctx, const DevMat& A, const DevMat& B,
   int f = 0;
   for (int pass = 0;; ++pass) {
     if (pass > 0) tm.mark(SPG_STAGE_BINNING);
+    P.c_known = pass == 0;
     P.bin(P.prod.as<int64_t>(), kBinNumeric);
     SPG_TRY(P.fetch_offsets());
     const int64_t nheavy = P.bin_size(kBinHeavy);
@@ -1060,9 +1062,10 @@ spg_status multiply_reuse_device(spg_ctx* ctx, const DevMat& A, const DevMat& B,
     spg_report pass_rep{};
     SPG_TRY(P.numeric(P.nnz.as<int64_t>(), C->col_idx, C->val, C->nnz, &pass_rep));
     SPG_TRY(read_flags(ctx, &f));
-    // the units also need C's columns where they were; a row whose columns
-    // moved is settled by the tables, which read only its length
-    if ((f & (kFlagCountDiff | kFlagBadIndex)) && nheavy > 0 && pass == 0 && P.bp.heavy_min < P.bp.warp_cap) {
+    // the units need C's columns where they were; a row whose columns moved is
+    // settled by the tables, which read only its length, and past these by units
+    // that find its columns
+    if ((f & (kFlagCountDiff | kFlagBadIndex)) && nheavy > 0 && pass == 0) {
       P.bp.heavy_min = INT64_MAX;
       continue;
     }

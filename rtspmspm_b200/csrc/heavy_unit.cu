@@ -33,6 +33,15 @@ namespace spg {
 // side so that one load brings both.
 constexpr int kTileCost = 2 * kTileWords;
 constexpr int kUnitWarps = kUnitThreads / 32;
+// A unit that marks its columns itself leaves segments of at most this many
+// products to one lane each (6,479 rows of which 900 have 3,000 segments, most of
+// 2 or 3 products in a unit, call 6.75 -> 6.48 ms).
+constexpr int kLaneSegment = 16;
+// Where three of four segments of the walk's 128 hold at most this many products,
+// runs of them are added by one warp, 32 products a step: a step of the whole CTA
+// for 2 or 3 products costs its four warps 160 instructions (the product above
+// 5.36 -> 2.86 ms, its new values, with columns from C, 5.14 -> 2.78).
+constexpr int kPackSegment = 8;
 // Rows of A of more entries than this are cut first and taken first: their
 // units run longest.
 constexpr int64_t kLongRow = 1024;
@@ -161,11 +170,12 @@ __device__ __forceinline__ Off segment_start(const int4& s) {
 // entries of A's row, in order, and empty ones behind them.
 struct SegmentList {
   int4 seg[kUnitThreads + 5];
-  int cnt[kUnitWarps];
+  int cnt[kUnitWarps];         // a warp's segments; those of at most kPackSegment products << 16
+  unsigned small[kUnitWarps];  // one bit a segment: such a one (small_segments)
 };
 
 // Fills `sl` with A entries [base, base + kUnitThreads) of the unit; returns
-// the number of segments.
+// the number of segments (and the small ones << 16).
 template <bool R32>
 __device__ __forceinline__ int list_segments(const DCsr& A, const DCsr& B, int64_t base, int64_t e, int t0, int t1,
                                              int ntiles, const int32_t* bidx, SegmentList& sl) {
@@ -176,7 +186,8 @@ __device__ __forceinline__ int list_segments(const DCsr& A, const DCsr& B, int64
   float a;
   unit_segment<R32>(A, B, base + threadIdx.x, e, t0, t1, ntiles, bidx, bs, len, a);
   const unsigned m = __ballot_sync(kFull, len > 0);
-  if (lane == 0) sl.cnt[wib] = __popc(m);
+  const unsigned few = __ballot_sync(kFull, len > 0 && len <= kPackSegment);
+  if (lane == 0) sl.cnt[wib] = __popc(m) | __popc(few) << 16;
   __syncthreads();  // also: the previous list has been walked
   int at = 0, cnt = 0;
 #pragma unroll
@@ -184,25 +195,131 @@ __device__ __forceinline__ int list_segments(const DCsr& A, const DCsr& B, int64
     at += w < wib ? sl.cnt[w] : 0;
     cnt += sl.cnt[w];
   }
+  at &= 0xffff;
   if (len > 0) sl.seg[at + __popc(m & ((1u << lane) - 1u))] = pack_segment<Off>(bs, len, a);
-  if (threadIdx.x < 5) sl.seg[cnt + threadIdx.x] = make_int4(0, 0, 0, 0);
+  if (threadIdx.x < 5) sl.seg[(cnt & 0xffff) + threadIdx.x] = make_int4(0, 0, 0, 0);
   __syncthreads();
   return cnt;
 }
 
-// One CTA per unit, one atomic ticket each.  STORED: the symbolic pass left
-// the rows' column bitmaps in `bitmap` (big_slot order, `stride` words a
-// row); else the unit's products are walked once to set the bits and the
-// columns found are compared with tile_cnt, tile by tile (in a value-only
-// recompute they come from A and B, the counts from C).  For rows of at most
-// whole_max entries that walk also takes in the empty tiles up to the next unit,
-// or the row's ends, so that no product of such a row goes unseen.  Then A's
+// A column's accumulator in a unit; one outside its columns, or with CHECK not
+// one of C's, is noted in `far` (and lands on any).
+template <bool CHECK>
+__device__ __forceinline__ int locate_column(const uint2* bits, int32_t c, int32_t c0, uint32_t span, uint32_t& far) {
+  uint32_t off = (uint32_t)(c - c0);
+  far = max(far, off);
+  off = min(off, span - 1u);
+  const uint2 w = bits[off >> 5];
+  const uint32_t bit = 1u << (off & 31);
+  if (CHECK && !(w.x & bit)) far = 0xffffffffu;
+  return (int)w.y + __popc(w.x & (bit - 1u));
+}
+
+// What an accumulator holds before its first product where every one has to get
+// one: a NaN that no sum is (adds give 0x7fffffff).
+constexpr uint32_t kUntouched = 0xffabcdefu;
+template <bool CHECK>
+__device__ __forceinline__ float added_to(float s, float p) {
+  if (CHECK && __float_as_uint(s) == kUntouched) s = 0.f;
+  return add_rn(s, p);
+}
+
+// Adds the products of a list of mostly small segments, in order: runs of small
+// ones by one warp, 32 products a step, the others by the CTA.  The unit's bitmap
+// of `words` words and its accumulators are in sm_unit.  Returns locate_column's
+// `far`.  Not inlined: in the kernel its registers would cost every unit one or
+// two of nine CTAs an SM (R-MAT 18, 3 edges: 4.72 -> 4.91 ms a call).
+template <typename Off, bool CHECK>
+__device__ __noinline__ uint32_t add_small_segments(const int32_t* col, const float* val, int words, SegmentList& sl,
+                                                    int cnt, int32_t c0, uint32_t span) {
+  extern __shared__ __align__(16) uint32_t sm_unit[];
+  const uint2* bits = reinterpret_cast<const uint2*>(sm_unit);
+  float* acc = reinterpret_cast<float*>(sm_unit) + 2 * words;
+  const int tid = threadIdx.x, lane = lane_id(), wib = tid >> 5;
+  uint32_t far = 0;
+  const int mine = tid < cnt ? sl.seg[tid].z : 0;
+  const unsigned few = __ballot_sync(kFull, mine > 0 && mine <= kPackSegment);
+  if (lane == 0) sl.small[wib] = few;
+  __syncthreads();
+  for (int i = 0; i < cnt;) {
+    const unsigned rest = ~(sl.small[i >> 5] >> (i & 31));
+    const int run = min(rest ? __ffs(rest) - 1 : 32, 32 - (i & 31));
+    if (run == 0) {
+      const int4 sg = sl.seg[i];
+      const Off sb = segment_start<Off>(sg);
+      const float a = __int_as_float(sg.w);
+      for (int q = tid; q < sg.z; q += kUnitThreads) {
+        const int at = locate_column<CHECK>(bits, col[sb + q], c0, span, far);
+        acc[at] = added_to<CHECK>(acc[at], prod_rn(a, val[sb + q]));
+      }
+      ++i;
+    } else {
+      if (wib == 0) {
+        const int4 own = lane < run ? sl.seg[i + lane] : make_int4(0, 0, 0, 0);
+        const Off ob = segment_start<Off>(own);
+        const int incl = warp_incl_scan(own.z);
+        const int total = __shfl_sync(kFull, incl, 31);
+        for (int p0 = 0; p0 < total; p0 += 4 * 32) {
+          int32_t c4[4];
+          float p4[4];
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            if (p0 + x * 32 >= total) break;
+            // lanes past the end take the last product and drop it
+            const int t = min(p0 + x * 32 + lane, total - 1);
+            const int from = warp_upper_bound(incl, t);
+            const Off q = __shfl_sync(kFull, ob, from) + (Off)(t - __shfl_sync(kFull, incl - own.z, from));
+            c4[x] = col[q];
+            p4[x] = prod_rn(__int_as_float(__shfl_sync(kFull, own.w, from)), val[q]);
+          }
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            if (p0 + x * 32 >= total) break;
+            const int at = locate_column<CHECK>(bits, c4[x], c0, span, far);
+            const bool act = p0 + x * 32 + lane < total;
+            // products on one column: the first lane adds them in their order
+            const unsigned grp = __match_any_sync(kFull, act ? at : -1 - lane);
+            const bool lead = act && (grp & ((1u << lane) - 1u)) == 0u;
+            unsigned later = grp & ~(1u << lane);
+            float s = 0.f;
+            if (lead) s = added_to<CHECK>(acc[at], p4[x]);
+            while (__any_sync(kFull, lead && later)) {
+              const int next = later ? __ffs(later) - 1 : lane;
+              const float v = __shfl_sync(kFull, p4[x], next);
+              if (lead && later) s = add_rn(s, v);
+              later &= later - 1;
+            }
+            if (lead) acc[at] = s;
+            __syncwarp();
+          }
+        }
+      }
+      i += run;
+    }
+    __syncthreads();
+  }
+  return far;
+}
+
+// Where a unit's columns come from.
+enum UnitColumns {
+  kStored,  // the rows' bitmaps of the symbolic pass (big_slot order, `stride` words a row)
+  kFromC,   // c_col (value-only recompute)
+  kMarked,  // a walk over its products; compared with tile_cnt, tile by tile
+};
+
+// One CTA per unit, one atomic ticket each.  With columns from C every product
+// has to fall on one of them and every accumulator, kUntouched at first, has to
+// get one; a unit where that fails raises a flag, its columns as they were.  For
+// rows of at most whole_max entries the walk over the products also takes in the
+// empty tiles up to the next unit, or the row's ends, so that no product of such
+// a row goes unseen (kFromC, kMarked).  Then A's
 // row is walked in canonical order, segment by segment with a barrier after
 // each: a segment's columns are distinct, so the CTA's threads add its
 // products at once.  A thread's first two products of segment i + 2 are
 // loaded and those of segment i + 1 located while segment i is added.
-template <bool R32, bool STORED>
-__global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const int4* units, int64_t room,
+template <bool R32, UnitColumns FROM>
+__global__ void __launch_bounds__(kUnitThreads, R32 ? 9 : 8) k_num_unit(DCsr A, DCsr B, const int4* units, int64_t room,
                                                            const unsigned long long* nunits, int ntiles,
                                                            const int64_t* c_rp, int32_t* c_col, float* c_val,
                                                            const int32_t* bidx, const uint32_t* bitmap,
@@ -231,15 +348,11 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
     const int words = nt * kTileWords;
     float* acc = reinterpret_cast<float*>(bits + words);
     const int64_t s = A.rp[row], e = A.rp[row + 1];
-    // the columns
-    if (STORED) {
-      const uint32_t* bm = bitmap + (int64_t)big_slot[row] * stride + (int64_t)t0 * kTileWords;
-      for (int i = tid; i < words; i += kUnitThreads) bits[i].x = bm[i];
-    } else {
-      for (int i = tid; i < words; i += kUnitThreads) bits[i].x = 0u;
-      int g0 = t0, g1 = t1;  // the tiles looked at
+    int g0 = t0, g1 = t1;  // the tiles looked at
+    bool whole = false;
+    if (FROM != kStored) {
       const int64_t entries = c_rp[row + 1] - c_rp[row];
-      const bool whole = entries <= whole_max;
+      whole = entries <= whole_max;
       if (whole) {
         const int32_t* tc = tile_cnt + (int64_t)big_slot[row] * ntiles;
         while (g0 > 0) {
@@ -250,21 +363,50 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
         }
         if (un.w + n == entries) g1 = ntiles;
       }
+    }
+    const int64_t out = c_rp[row] + un.w;
+    // the columns
+    if (FROM == kStored) {
+      const uint32_t* bm = bitmap + (int64_t)big_slot[row] * stride + (int64_t)t0 * kTileWords;
+      for (int i = tid; i < words; i += kUnitThreads) bits[i].x = bm[i];
+    } else {
+      for (int i = tid; i < words; i += kUnitThreads) bits[i].x = 0u;
+    }
+    if (FROM == kFromC) {
+      __syncthreads();
+      for (int i = tid; i < n; i += kUnitThreads) {
+        const uint32_t off = (uint32_t)(c_col[out + i] - c0);
+        if (off < span) atomicOr(&bits[off >> 5].x, 1u << (off & 31));
+        else raise_flag(flags, kFlagCountDiff);
+      }
+    }
+    if (FROM == kMarked) {
       for (int64_t base = s; base < e; base += kUnitThreads) {
-        const int cnt = list_segments<R32>(A, B, base, e, g0, g1, ntiles, bidx, sl);
-        for (int i = wib; i < cnt; i += kUnitWarps) {
-          const int4 sg = sl.seg[i];
-          const Off sb = segment_start<Off>(sg);
-#pragma unroll 4
-          for (int q = lane; q < sg.z; q += 32) {
-            const uint32_t off = (uint32_t)(B.col[sb + q] - c0);
-            if (off < span) {
-              const uint32_t bit = 1u << (off & 31);
-              if (!(bits[off >> 5].x & bit)) atomicOr(&bits[off >> 5].x, bit);
-            } else {
-              raise_flag(flags, whole ? kFlagCountDiff : kFlagBadIndex);
-            }
+        const int cnt = list_segments<R32>(A, B, base, e, g0, g1, ntiles, bidx, sl) & 0xffff;
+        auto mark = [&](int32_t c) {
+          const uint32_t off = (uint32_t)(c - c0);
+          if (off < span) {
+            const uint32_t bit = 1u << (off & 31);
+            if (!(bits[off >> 5].x & bit)) atomicOr(&bits[off >> 5].x, bit);
+          } else {
+            raise_flag(flags, whole ? kFlagCountDiff : kFlagBadIndex);
           }
+        };
+        // the warp's segments, one a lane: short ones by their lane, the others by
+        // the warp
+        const int mine = lane * kUnitWarps + wib;
+        const int4 own = mine < cnt ? sl.seg[mine] : make_int4(0, 0, 0, 0);
+        const Off ob = segment_start<Off>(own);
+        if (own.z <= kLaneSegment) {
+#pragma unroll 4
+          for (int q = 0; q < own.z; ++q) mark(B.col[ob + q]);
+        }
+        for (unsigned todo = __ballot_sync(kFull, own.z > kLaneSegment); todo; todo &= todo - 1) {
+          const int from = __ffs(todo) - 1;
+          const int len = __shfl_sync(kFull, own.z, from);
+          const Off sb = __shfl_sync(kFull, ob, from);
+#pragma unroll 4
+          for (int q = lane; q < len; q += 32) mark(B.col[sb + q]);
         }
       }
     }
@@ -294,9 +436,9 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
       __syncthreads();
       continue;
     }
-    for (int i = tid; i < n; i += kUnitThreads) acc[i] = 0.f;
+    for (int i = tid; i < n; i += kUnitThreads) acc[i] = FROM == kFromC ? __uint_as_float(kUntouched) : 0.f;
     __syncthreads();
-    if (!STORED) {
+    if (FROM == kMarked) {
       // C's columns of such a unit stay as they are: a second look at the row
       // counts them again
       const int32_t* tc = tile_cnt + (int64_t)big_slot[row] * ntiles + t0;
@@ -310,18 +452,18 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
         continue;
       }
     }
-    // a column's accumulator; one outside the unit is noted (and lands on any)
     uint32_t far = 0;
-    auto locate = [&](int32_t c) -> int {
-      uint32_t off = (uint32_t)(c - c0);
-      far = max(far, off);
-      off = min(off, span - 1u);
-      const uint2 w = bits[off >> 5];
-      return (int)w.y + __popc(w.x & ((1u << (off & 31)) - 1u));
-    };
+    auto locate = [&](int32_t c) { return locate_column<FROM == kFromC>(bits, c, c0, span, far); };
+    auto added = [&](int at, float p) { return added_to<FROM == kFromC>(acc[at], p); };
     const int first = wib << 5;  // the warp's first product of a segment
     for (int64_t base = s; base < e; base += kUnitThreads) {
-      const int cnt = list_segments<R32>(A, B, base, e, t0, t1, ntiles, bidx, sl);
+      const int listed = FROM == kFromC ? list_segments<R32>(A, B, base, e, g0, g1, ntiles, bidx, sl)
+                                        : list_segments<R32>(A, B, base, e, t0, t1, ntiles, bidx, sl);
+      const int cnt = listed & 0xffff;
+      if (cnt >= 32 && (listed >> 16) * 4 >= cnt * 3) {
+        far = max(far, add_small_segments<Off, FROM == kFromC>(B.col, B.val, words, sl, cnt, c0, span));
+        continue;
+      }
       // products tid and kUnitThreads + tid of three segments: one being
       // added, one located, one on its way
       int4 sg[3];
@@ -352,10 +494,10 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
         const int len = sg[u].z;
         if (first >= len) return;
         const float a = __int_as_float(sg[u].w);
-        const float r0 = add_rn(acc[at[u][0]], prod_rn(a, vv[u][0]));
+        const float r0 = added(at[u][0], prod_rn(a, vv[u][0]));
         if (tid < len) acc[at[u][0]] = r0;
         if (first + kUnitThreads >= len) return;
-        const float r1 = add_rn(acc[at[u][1]], prod_rn(a, vv[u][1]));
+        const float r1 = added(at[u][1], prod_rn(a, vv[u][1]));
         if (tid + kUnitThreads < len) acc[at[u][1]] = r1;
         if (first + 2 * kUnitThreads >= len) return;
         const Off sb = segment_start<Off>(sg[u]);
@@ -373,7 +515,7 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
           for (int x = 0; x < 4; ++x) a4[x] = locate(c4[x]);
           float cur[4];
 #pragma unroll
-          for (int x = 0; x < 4; ++x) cur[x] = add_rn(acc[a4[x]], prod_rn(a, v4[x]));
+          for (int x = 0; x < 4; ++x) cur[x] = added(a4[x], prod_rn(a, v4[x]));
 #pragma unroll
           for (int x = 0; x < 4; ++x)
             if (q0 + x * kUnitThreads + lane < len) acc[a4[x]] = cur[x];
@@ -394,9 +536,12 @@ __global__ void __launch_bounds__(kUnitThreads) k_num_unit(DCsr A, DCsr B, const
     }
     if (far >= span) raise_flag(flags, kFlagBadIndex);
     // values, then the columns laid out in the accumulators' place
-    const int64_t out = c_rp[row] + un.w;
-    for (int i = tid; i < n; i += kUnitThreads) c_val[out + i] = acc[i];
+    for (int i = tid; i < n; i += kUnitThreads) {
+      c_val[out + i] = acc[i];
+      if (FROM == kFromC && __float_as_uint(acc[i]) == kUntouched) raise_flag(flags, kFlagCountDiff);
+    }
     __syncthreads();
+    if (FROM == kFromC) continue;
     int32_t* cols = reinterpret_cast<int32_t*>(acc);
     for (int i = tid; i < words; i += kUnitThreads) {
       const uint2 w = bits[i];
@@ -417,39 +562,41 @@ int64_t heavy_unit_bound(int64_t nheavy, int ntiles, int64_t entries) {
   return 2 * (entries + (int64_t)kTileCost * ntiles * nheavy) / kUnitCost + nheavy + 1;
 }
 
-template <bool R32, bool STORED>
+template <bool R32, UnitColumns FROM>
 static void num_unit_one(const DCsr& A, const DCsr& B, const int4* units, int64_t room,
                          const unsigned long long* nunits, int ntiles,
                          const int64_t* c_rp, int32_t* c_col, float* c_val, const int32_t* bidx,
                          const uint32_t* bitmap, int64_t stride, const int32_t* big_slot, const int32_t* tile_cnt,
                          int64_t whole_max, unsigned long long* ticket, int* flags, const LaunchCtx& lc) {
   const size_t smem = (size_t)kUnitWords * 4;
-  cudaFuncSetAttribute(k_num_unit<R32, STORED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k_num_unit<R32, FROM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_num_unit<R32, STORED>, kUnitThreads, smem);
-  k_num_unit<R32, STORED><<<lc.sms * std::max(1, per_sm), kUnitThreads, smem, lc.stream>>>(
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_num_unit<R32, FROM>, kUnitThreads, smem);
+  k_num_unit<R32, FROM><<<lc.sms * std::max(1, per_sm), kUnitThreads, smem, lc.stream>>>(
       A, B, units, room, nunits, ntiles, c_rp, c_col, c_val, bidx, bitmap, stride, big_slot, tile_cnt, whole_max,
       ticket, flags);
 }
 
 void launch_num_units(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, int64_t nheavy, const int32_t* big_slot,
                       const int32_t* tile_cnt, int ntiles, const int64_t* c_rp, int32_t* c_col, float* c_val,
-                      const int32_t* bidx, const uint32_t* bitmap, int64_t stride, int64_t whole_max, int4* units,
+                      const int32_t* bidx, const uint32_t* bitmap, int64_t stride, bool c_known, int64_t whole_max, int4* units,
                       int64_t room, unsigned long long* counters, int* flags, const LaunchCtx& lc) {
   if (nheavy == 0) return;
   cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), lc.stream);
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nheavy + 7) / 8, (int64_t)lc.sms * 8));
   k_cut_units<<<blocks, 256, 0, lc.stream>>>(heavy_rows, nheavy, big_slot, tile_cnt, ntiles, A.rp, units, room,
                                              counters, flags);
-#define SPG_NU(R, S)                                                                                            \
-  num_unit_one<R, S>(A, B, units, room, counters, ntiles, c_rp, c_col, c_val, bidx, bitmap, stride, big_slot,   \
+#define SPG_NU(R, F)                                                                                            \
+  num_unit_one<R, F>(A, B, units, room, counters, ntiles, c_rp, c_col, c_val, bidx, bitmap, stride, big_slot,   \
                      tile_cnt, whole_max, counters + 1, flags, lc)
   if (B.rp32) {
-    if (bitmap) SPG_NU(true, true);
-    else SPG_NU(true, false);
+    if (bitmap) SPG_NU(true, kStored);
+    else if (c_known) SPG_NU(true, kFromC);
+    else SPG_NU(true, kMarked);
   } else {
-    if (bitmap) SPG_NU(false, true);
-    else SPG_NU(false, false);
+    if (bitmap) SPG_NU(false, kStored);
+    else if (c_known) SPG_NU(false, kFromC);
+    else SPG_NU(false, kMarked);
   }
 #undef SPG_NU
 }

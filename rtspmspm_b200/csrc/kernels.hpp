@@ -248,15 +248,16 @@ void launch_num_tile(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, in
 // Heavy rows as units of consecutive column tiles (heavy_unit.cu).  `units`
 // holds room = heavy_unit_bound(nheavy, ntiles, entries of those rows);
 // bidx as above; bitmap: the rows' column bitmaps at big_slot * stride words
-// (from launch_sym_dense), or null (each unit finds its columns itself and
-// compares them with tile_cnt; in rows of at most whole_max entries it sees every
-// product, also those outside the tiles with entries); counters: two device
-// words.
+// (from launch_sym_dense), or null: with c_known the columns are those in c_col,
+// which stays as it is (a product on another column or an entry without a product
+// raises a flag), else each unit finds its columns itself and compares them with
+// tile_cnt.  Either way rows of at most whole_max entries see every product, also
+// those outside the tiles with entries.  counters: two device words.
 int64_t heavy_unit_bound(int64_t nheavy, int ntiles, int64_t entries);
 void launch_num_units(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, int64_t nheavy, const int32_t* big_slot,
                       const int32_t* tile_cnt, int ntiles, const int64_t* c_rp, int32_t* c_col, float* c_val,
-                      const int32_t* bidx, const uint32_t* bitmap, int64_t stride, int64_t whole_max, int4* units,
-                      int64_t room, unsigned long long* counters, int* flags, const LaunchCtx& lc);
+                      const int32_t* bidx, const uint32_t* bitmap, int64_t stride, bool c_known, int64_t whole_max,
+                      int4* units, int64_t room, unsigned long long* counters, int* flags, const LaunchCtx& lc);
 void launch_compact_rows(const int32_t* rows, int64_t nrows, const uint8_t* need_exact, const int64_t* slab_off,
                          const int32_t* slab_col, const float* slab_val, const int64_t* c_rp, int32_t* c_col,
                          float* c_val, const LaunchCtx& lc);
