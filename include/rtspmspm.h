@@ -416,7 +416,8 @@ typedef struct spg_tuning {
                                   8192) use a CTA-wide hash table; 0 or -1 (default): off,
                                   warp tables and heavy-row tiles only */
     int32_t esc_min_prod;      /* rows of at least this many products (0: default 32) whose
-                                  output keeps half of them or more, and that fit the warp's
+                                  output keeps half of them or more (of fewer than 128 more:
+                                  80 % of 50, all of fewer than 48), and that fit the warp's
                                   table memory, are expanded, sorted on their columns and
                                   folded instead of hashed; -1: off */
     int32_t small_rows;        /* products whose A has at most this many rows (0: default 8192;

@@ -207,6 +207,7 @@ BinParams bin_params(const spg_tuning& t) {
   int blg = ilog2_floor(std::max(1024, std::min(32768, t.block_table_max)));
   bp.block_cap = ((int64_t)1 << blg) * 2 / 3;
   bp.esc_prod = esc_bin_products(kNumEscBins - 1);
+  bp.early_max = (int64_t)std::floor((double)(1 << std::min(kEarlyLog, bp.warp_log_max)) * bp.max_load);
   // CTA-wide numeric hash bins (tables at load <= 1/2: their key and
   // order-word arrays are the row sort's buffers) for rows of more than
   // block_min_nnz entries, when set: measured slower than the warp tables
@@ -369,6 +370,9 @@ constexpr size_t kBlockedIndexMaxBytes = size_t(4) << 30;
 // Largest set of column bitmaps the symbolic pass leaves for the heavy-row
 // units (bytes).
 constexpr size_t kBitmapMaxBytes = size_t(8) << 30;
+// Learned products of fewer rows keep those of up to kLearnedEarlyMin entries.
+constexpr int64_t kLearnedEarlyMin = 1024;
+constexpr int64_t kEarlyLearnedRows = 2048;
 // Largest list of non-empty heavy-row tiles (bytes).
 constexpr size_t kWorkListMaxBytes = size_t(4) << 30;
 
@@ -397,6 +401,7 @@ struct Pipeline {
   DevBuf bitmap;      // uint32 nbig * bitmap_stride(), or empty
   int64_t h_off[kNumBins + 1] = {};
   int64_t nbig = 0;
+  bool early = false;     // the last symbolic pass's kBinEarlySym rows are among its big ones
   bool c_known = false;   // the units take their columns from C (value-only recompute, first pass)
   int64_t whole_max = 0;  // launch_num_units' whole_max (value-only recompute)
 
@@ -428,14 +433,24 @@ struct Pipeline {
   // Products of every row and, for the symbolic binning, their span words.
   spg_status products() {
     SPG_TRY(span.alloc(ctx, (size_t)std::max<int64_t>(rows, 1) * 4));
-    launch_row_products(A.view, B.view, prod.as<int64_t>(), lc, span.as<int32_t>());
+    launch_row_products(A.view, B.view, prod.as<int64_t>(), lc, span.as<int32_t>(), bp.warp_cap,
+                        bp.heavy_min);
+    ++ctx->launches;
+    return SPG_OK;
+  }
+
+  // Span words of the listed rows.
+  spg_status listed_spans(const int32_t* list, const unsigned long long* count) {
+    SPG_TRY(span.alloc(ctx, (size_t)std::max<int64_t>(rows, 1) * 4));
+    launch_listed_spans(A.view, B.view, list, count, prod.as<int64_t>(), span.as<int32_t>(), bp.warp_cap,
+                        bp.heavy_min, lc);
     ++ctx->launches;
     return SPG_OK;
   }
 
   // Big rows of the last symbolic binning, and whether their bitmaps fit the
   // budget.
-  int64_t big_rows() const { return bin_size(kBinBlock) + bin_size(kBinDense); }
+  int64_t big_rows() const { return bin_size(kBinBlock) + bin_size(kBinDense) + (early ? bin_size(kBinEarlySym) : 0); }
   size_t bitmap_bytes() const { return (size_t)big_rows() * (size_t)bitmap_stride() * 4; }
   bool bitmaps_fit() const {
     return tune.heavy_path == 0 && bitmap_stride() <= kDenseWindowWords && bitmap_bytes() <= kBitmapMaxBytes &&
@@ -485,15 +500,26 @@ struct Pipeline {
   int64_t bin_size(int b) const { return h_off[b + 1] - h_off[b]; }
   const int32_t* bin_rows(int b) { return lists.as<int32_t>() + h_off[b]; }
 
+  // Whether n rows that may leave the warp tables early do, beside `others` that
+  // do for certain.
+  static bool take_early(int64_t n, int64_t others) { return n > 0 && (others > 0 || n >= kEarlyRows); }
+
+  // The numeric binning's rows for the units (or, opted for, the tiles).
+  bool early_heavy() const { return take_early(bin_size(kBinEarly), bin_size(kBinHeavy)); }
+  const int32_t* heavy_rows() { return bin_rows(early_heavy() ? kBinEarly : kBinHeavy); }
+  int64_t heavy_size() const { return bin_size(kBinHeavy) + (early_heavy() ? bin_size(kBinEarly) : 0); }
+
   // Exact symbolic pass over rows whose key (products) is > 0.
   spg_status symbolic(const int64_t* key) {
     bin(key, kBinSymbolic);
     SPG_TRY(fetch_offsets());
+    early = take_early(bin_size(kBinEarlySym), bin_size(kBinBlock) + bin_size(kBinDense));
     bool fit = big_rows() > 0 && bitmaps_fit();
     // only rows with a stored bitmap gain from leaving the warp tables early
     // (past 128 * warp_cap columns none does, big_row)
     if (big_rows() > 0 && !fit && bp.heavy_min < bp.warp_cap && cols <= 128 * bp.warp_cap) {
       bp.heavy_min = INT64_MAX;
+      early = false;
       bin(key, kBinSymbolic);
       SPG_TRY(fetch_offsets());
       fit = big_rows() > 0 && bitmaps_fit();
@@ -509,8 +535,16 @@ struct Pipeline {
                       wpb);
       ++ctx->launches;
     }
-    const int64_t nblock = bin_size(kBinBlock), ndense = bin_size(kBinDense);
-    nbig = nblock + ndense;
+    if (!early && bin_size(kBinEarlySym) > 0) {
+      // tables for as many products as the warp tables take (bin_of)
+      launch_sym_warp(bp.warp_log_max, A.view, B.view, bin_rows(kBinEarlySym),
+                      bin_size(kBinEarlySym), nnz.as<int64_t>(), ctx->d_flags, lc, wpb);
+      ++ctx->launches;
+      bp.heavy_min = std::max(bp.heavy_min, bp.early_max);
+    }
+    const int64_t nblock = bin_size(kBinBlock);
+    nbig = big_rows();
+    const int64_t ndense = nbig - nblock;
     if (nbig > 0) {
       const size_t tb = (size_t)nbig * ntiles * 4;
       SPG_TRY(tile_cnt.alloc(ctx, tb));
@@ -558,6 +592,8 @@ struct Pipeline {
     EscArgs e;
     e.prod = row_prod;
     e.min_prod = esc_min_products(tune);
+    e.per_margin = esc_per_margin(tune);
+    e.slack = tune.predict_slack;
     return e;
   }
 
@@ -568,7 +604,7 @@ struct Pipeline {
   // rescan their row with bulk copies of long segments.  *done stays false
   // when the path does not apply (buckets or alignment).
   spg_status numeric_tiles(const int64_t* c_rp, int32_t* c_col, float* c_val, const int32_t* bidx, bool* done) {
-    const int64_t nheavy = bin_size(kBinHeavy);
+    const int64_t nheavy = heavy_size();
     // rows with a slot: the symbolic pass's, or the bin's (value-only recompute)
     const int64_t nslots = std::max(nbig, nheavy);
     if (tune.heavy_path == 2 && !bulk_aligned(B.view)) return SPG_OK;
@@ -580,16 +616,16 @@ struct Pipeline {
     DevBuf nz, work, tile_off;  // tile_off: int32, as tile_cnt
     SPG_TRY(tile_off.alloc(ctx, (size_t)nslots * (size_t)ntiles * 4));
     if (use_list) SPG_TRY(nz.alloc(ctx, (size_t)(nheavy + 1) * 8));
-    launch_tile_offsets(bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles,
+    launch_tile_offsets(heavy_rows(), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles,
                         tile_off.as<int32_t>(), use_list ? nz.as<int64_t>() : nullptr, lc);
     ++ctx->launches;
     if (tune.heavy_path == 1)
-      return heavy_staged(ctx, A.view, B.view, bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(),
+      return heavy_staged(ctx, A.view, B.view, heavy_rows(), nheavy, big_slot.as<int32_t>(),
                           tile_cnt.as<int32_t>(), tile_off.as<int32_t>(), ntiles, c_rp, c_col, c_val, done);
     if (use_list) {
       SPG_TRY(work.alloc(ctx, work_bytes));
       launch_excl_scan(nz.as<int64_t>(), nheavy, nz.as<int64_t>(), scan_tmp.as<int64_t>(), lc);
-      launch_tile_worklist(bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles,
+      launch_tile_worklist(heavy_rows(), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(), ntiles,
                            nz.as<int64_t>(), work.as<int64_t>(), lc);
       ctx->launches += 5;
     }
@@ -599,7 +635,7 @@ struct Pipeline {
       launch_build_tile_occupancy(B.view.rows, bidx, ntiles, tocc.as<uint32_t>(), lc);
       ++ctx->launches;
     }
-    launch_num_tile(A.view, B.view, bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(),
+    launch_num_tile(A.view, B.view, heavy_rows(), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(),
                     tile_off.as<int32_t>(), ntiles, c_rp, c_col, c_val, bidx, tocc.as<uint32_t>(),
                     use_list ? work.as<int64_t>() : nullptr, use_list ? nz.as<int64_t>() + nheavy : nullptr,
                     ctx->d_counter, ctx->d_flags, lc);
@@ -614,25 +650,32 @@ struct Pipeline {
   spg_status numeric(const int64_t* c_rp, int32_t* c_col, float* c_val, int64_t c_nnz, spg_report* rep,
                      const int64_t* row_prod = nullptr) {
     const EscArgs esc = esc_args(row_prod);
+    // early rows that stay go with the rows of the table that holds them, unless
+    // other bins lie between
+    const int early_bin = std::min(kEarlyLog, bp.warp_log_max) - kMinLogT;
+    const int64_t nearly = early_heavy() ? 0 : bin_size(kBinEarly);
+    const bool joined = h_off[early_bin + 1] == h_off[kBinEarly];
+    if (nearly > 0 && !joined) {
+      launch_num_warp(kMinLogT + early_bin, A.view, B.view, bin_rows(kBinEarly), nearly, c_rp, c_col, c_val,
+                      ctx->d_flags, lc, wpb);
+      ++ctx->launches;
+    }
     for (int b = 0; b < kNumWarpBins; ++b) {
-      if (bin_size(b) == 0) continue;
-      launch_num_warp(kMinLogT + b, A.view, B.view, bin_rows(b), bin_size(b), c_rp, c_col, c_val, ctx->d_flags, lc,
+      const int64_t n = bin_size(b) + (joined && b == early_bin ? nearly : 0);
+      if (n == 0) continue;
+      launch_num_warp(kMinLogT + b, A.view, B.view, bin_rows(b), n, c_rp, c_col, c_val, ctx->d_flags, lc,
                       wpb, esc);
       ++ctx->launches;
     }
-    for (int b = kBinEsc; b < kBinEsc + kNumEscBins; ++b) {
-      if (bin_size(b) == 0) continue;
-      launch_num_esc(b, A.view, B.view, bin_rows(b), bin_size(b), row_prod, c_rp, c_col, c_val, nullptr, nullptr,
-                     nullptr, nullptr, ctx->d_flags, lc, wpb);
-      ++ctx->launches;
-    }
+    ctx->launches += launch_num_esc(h_off, A.view, B.view, lists.as<int32_t>(), row_prod, c_rp, c_col, c_val, nullptr,
+                                    nullptr, nullptr, nullptr, ctx->d_flags, lc, wpb);
     // rows above the efficient warp tables: CTA-wide hash tables
     for (int b : {kBinBlock, kBinDense}) {
       if (bin_size(b) == 0) continue;
       launch_num_block(b, A.view, B.view, bin_rows(b), bin_size(b), c_rp, c_col, c_val, ctx->d_flags, lc);
       ++ctx->launches;
     }
-    const int64_t nheavy = bin_size(kBinHeavy);
+    const int64_t nheavy = heavy_size();
     if (nheavy > 0) {
       // the blocked index reads every row of B
       if (B.complete) SPG_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, B.complete, 0));
@@ -654,7 +697,7 @@ struct Pipeline {
         const int64_t room = heavy_unit_bound(nheavy, ntiles, c_nnz);
         DevBuf units;
         SPG_TRY(units.alloc(ctx, (size_t)room * sizeof(int4)));
-        launch_num_units(A.view, B.view, bin_rows(kBinHeavy), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(),
+        launch_num_units(A.view, B.view, heavy_rows(), nheavy, big_slot.as<int32_t>(), tile_cnt.as<int32_t>(),
                          ntiles, c_rp, c_col, c_val, bidx.as<int32_t>(), bitmap.as<uint32_t>(), bitmap_stride(),
                          c_known, whole_max, units.as<int4>(), room, ctx->d_counter + 8, ctx->d_flags, lc);
         ++ctx->launches;
@@ -663,6 +706,7 @@ struct Pipeline {
     }
     if (rep) {
       for (int b = 0; b < kBinEsc; ++b) rep->bin_rows[b] += bin_size(b);
+      rep->bin_rows[early_bin] += nearly;
       rep->bin_rows[SPG_BIN_HEAVY] += nheavy;
       rep->bin_rows[SPG_BIN_EMPTY] += bin_size(kBinEmpty);
       for (int b = kBinEsc; b < kBinEsc + kNumEscBins; ++b) rep->bin_rows[SPG_BIN_FOLD] += bin_size(b);
@@ -775,6 +819,10 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
     l.add(&retry, r * 4);
     SPG_TRY(l.alloc(ctx, learned_block));
   }
+  // a small product's rows leave the tables later: predicted past them they are
+  // walked twice, and few of them gain from it (R-MAT 10, 31 such rows of 1,024:
+  // 552 -> 465 us)
+  if (rows < kEarlyLearnedRows) P.bp.heavy_min = std::max(P.bp.heavy_min, std::min(kLearnedEarlyMin, P.bp.warp_cap));
   // products, features and the tensor-core MLP in one pass over A
   tm.mark(SPG_STAGE_MLP);
   // d_counter: [1] products, [2] overflowed rows, [3] rows predicted heavy
@@ -824,13 +872,10 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
                             P.esc_args(P.prod.as<int64_t>()));
     ++ctx->launches;
   }
-  for (int b = kBinEsc; b < kBinEsc + kNumEscBins; ++b) {
-    if (P.bin_size(b) == 0) continue;
-    launch_num_esc(b, P.A.view, P.B.view, P.bin_rows(b), P.bin_size(b), P.prod.as<int64_t>(), slab_off.as<int64_t>(),
-                   slab_col.as<int32_t>(), slab_val.as<float>(), cap.as<int64_t>(), P.nnz.as<int64_t>(),
-                   retry.as<int32_t>(), ctx->d_counter + 2, ctx->d_flags, lc, P.wpb);
-    ++ctx->launches;
-  }
+  ctx->launches += launch_num_esc(P.h_off, P.A.view, P.B.view, P.lists.as<int32_t>(), P.prod.as<int64_t>(),
+                                  slab_off.as<int64_t>(), slab_col.as<int32_t>(), slab_val.as<float>(),
+                                  cap.as<int64_t>(), P.nnz.as<int64_t>(), retry.as<int32_t>(), ctx->d_counter + 2,
+                                  ctx->d_flags, lc, P.wpb);
   for (int b : {kBinBlock, kBinDense}) {
     if (P.bin_size(b) == 0) continue;
     launch_num_block_learned(b, P.A.view, P.B.view, P.bin_rows(b), P.bin_size(b), cap.as<int64_t>(),
@@ -880,6 +925,9 @@ spg_status multiply_learned(spg_ctx* ctx, Pipeline& P, spg_csr* C, const spg_opt
     launch_mark_rows(retry.as<int32_t>(), ctx->d_counter + 2, need.as<uint8_t>(), lc);
     launch_mask_key(P.prod.as<int64_t>(), need.as<uint8_t>(), rows, key.as<int64_t>(), lc);
     ctx->launches += 2;
+    // rows that outgrew their capacity are counted as in the plain method; the
+    // others were predicted to be heavy
+    if (light > 0) SPG_TRY(P.listed_spans(retry.as<int32_t>(), ctx->d_counter + 2));
     SPG_TRY(P.symbolic(key.as<int64_t>()));
     launch_mask_key(P.nnz.as<int64_t>(), need.as<uint8_t>(), rows, key.as<int64_t>(), lc);
     P.bin(key.as<int64_t>(), kBinNumeric, P.esc_args(P.prod.as<int64_t>()));
@@ -1049,12 +1097,12 @@ spg_status multiply_reuse_device(spg_ctx* ctx, const DevMat& A, const DevMat& B,
     P.c_known = pass == 0;
     P.bin(P.prod.as<int64_t>(), kBinNumeric);
     SPG_TRY(P.fetch_offsets());
-    const int64_t nheavy = P.bin_size(kBinHeavy);
+    const int64_t nheavy = P.heavy_size();
     if (nheavy > 0) {
       const size_t tb = (size_t)nheavy * P.ntiles * 4;
       SPG_TRY(P.tile_cnt.alloc(ctx, tb));
       SPG_CUDA(ctx, cudaMemsetAsync(P.tile_cnt.get(), 0, tb, ctx->stream));
-      launch_tile_counts_from_cols(P.bin_rows(kBinHeavy), nheavy, P.nnz.as<int64_t>(), C->col_idx, P.ntiles,
+      launch_tile_counts_from_cols(P.heavy_rows(), nheavy, P.nnz.as<int64_t>(), C->col_idx, P.ntiles,
                                    P.big_slot.as<int32_t>(), P.tile_cnt.as<int32_t>(), ctx->d_flags, lc);
       ++ctx->launches;
     }

@@ -134,7 +134,7 @@ template <int LOGT, bool NUMERIC, bool LEARNED>
 __device__ __forceinline__ void warp_tile(const BatchMat* mats, const int32_t* row_mat, const int32_t* lists,
                                           int64_t first, int64_t last, int32_t* sm, int64_t* nnz,
                                           const int64_t* gscan, int32_t* c_col, float* c_val, const LearnedOut& lo,
-                                          const int64_t* prod, int esc_min, int ecap, int* flags) {
+                                          EscArgs esc, int ecap, int* flags) {
   constexpr int T = 1 << LOGT;
   const int lane = lane_id();
   int32_t* keys = sm;
@@ -163,10 +163,10 @@ __device__ __forceinline__ void warp_tile(const BatchMat* mats, const int32_t* r
       if (lane == 0) nnz[g] = cnt;
     } else if (LEARNED) {
       const int c = (int)lo.cap[g];
-      if (esc_wanted(prod[g], c, esc_min, ecap)) {
+      if (esc_wanted(esc.prod[g], esc_guess(c, esc.prod[g], esc.per_margin, esc.slack), esc.min_prod, ecap)) {
         // expand-sort-fold row in the warp's slot (its table wiped after)
         const int64_t off = lo.slab_off[g];
-        const int n = esc_row<true>(M.A, M.B, r, (int)prod[g], keys, c, lo.slab_col + off, lo.slab_val + off);
+        const int n = esc_row<true>(M.A, M.B, r, (int)esc.prod[g], keys, c, lo.slab_col + off, lo.slab_val + off);
         esc_wipe(keys, T);
         if (n >= 0) {
           if (lane == 0) {
@@ -194,8 +194,8 @@ __device__ __forceinline__ void warp_tile(const BatchMat* mats, const int32_t* r
     } else {
       const int64_t off = M.c_base + (gscan[g] - gscan[M.row_start]);
       const int64_t want = gscan[g + 1] - gscan[g];
-      if (esc_wanted(prod[g], want, esc_min, ecap)) {
-        const int n = esc_row<true>(M.A, M.B, r, (int)prod[g], keys, want, c_col + off, c_val + off);
+      if (esc_wanted(esc.prod[g], want, esc.min_prod, ecap)) {
+        const int n = esc_row<true>(M.A, M.B, r, (int)esc.prod[g], keys, want, c_col + off, c_val + off);
         esc_wipe(keys, T);
         if (n >= 0) {
           if (n != want && lane == 0) raise_flag(flags, kFlagCountDiff);
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kBlkThreads, MINB) k_batch_queue(const BatchMa
                                                                    const int64_t* bound, int64_t* nnz,
                                                                    const int64_t* gscan, int32_t* c_col,
                                                                    float* c_val, LearnedOut lo,
-                                                                   const int64_t* prod, int esc_min,
+                                                                   EscArgs esc,
                                                                    unsigned long long* counter, int* flags) {
   extern __shared__ int32_t sm_q[];
   __shared__ unsigned long long sh_tile;
@@ -326,8 +326,8 @@ __global__ void __launch_bounds__(kBlkThreads, MINB) k_batch_queue(const BatchMa
 #define SPG_WT(LL)                                                                                          \
   if (L == LL && LL >= LMIN && LL <= LMAX)                                                                  \
     warp_tile<(LL >= LMIN && LL <= LMAX) ? LL : LMIN, NUMERIC, LEARNED>(mats, row_mat, lists, first, last, slot, \
-                                                                        nnz, gscan, c_col, c_val, lo, prod,       \
-                                                                        NUMERIC ? esc_min : 0, ecap, flags);
+                                                                        nnz, gscan, c_col, c_val, lo, esc, ecap,  \
+                                                                        flags);
     SPG_WT(5) SPG_WT(6) SPG_WT(7) SPG_WT(8) SPG_WT(9) SPG_WT(10) SPG_WT(11)
 #undef SPG_WT
   }
@@ -445,11 +445,10 @@ constexpr int kBatchCtaLogT = 13;  // CTA tables: 2^13 slots at load <= 1/2
 // faster in the CTA tables.  Eight products of 3,000 rows of 1,600 | 2,500 |
 // 3,600 products with 77 to 98 | 68 to 82 | 66 to 91 % of them distinct, plain:
 // folded 2.1 to 2.4 | 4.9 to 5.0 | 7.1 to 7.7 ms a call, in the tables 2.7 to 3.5
-// | 3.4 to 3.9 | 4.5 to 6.4.
+// | 3.4 to 3.9 | 4.5 to 6.4.  Learned: of 1,600 products 4.12 to 4.45 ms folded,
+// 3.98 to 4.48 in the tables; six of 20,000 rows of 900 products, a tenth of them
+// past 1,152, 3.0 and 3.3.
 constexpr int kBatchEscBins = 4;
-// The learned method's, up to 1,152 products: of the rows of 1,600 above 4.12 and
-// 4.45 ms folded, 3.98 and 4.48 in the tables.
-constexpr int kBatchEscBinsLearned = 3;
 
 BatchQueue queue_of(int which) {
   BatchQueue q{};
@@ -507,8 +506,7 @@ struct QueueArgs {
   int32_t* c_col;
   float* c_val;
   LearnedOut lo;
-  const int64_t* prod;
-  int esc_min;
+  EscArgs esc;
   unsigned long long* counter;
   int* flags;
 };
@@ -518,7 +516,7 @@ const void* queue_launch(const QueueArgs* a, int grid, size_t smem, cudaStream_t
   auto k = k_batch_queue<NUMERIC, LEARNED, LMIN, LMAX, CTA, MINB>;
   if (a)
     k<<<grid, kBlkThreads, smem, st>>>(a->mats, a->row_mat, a->lists, a->bin_off, a->q, a->tile_pref, a->bound,
-                                       a->nnz, a->gscan, a->c_col, a->c_val, a->lo, a->prod, a->esc_min, a->counter,
+                                       a->nnz, a->gscan, a->c_col, a->c_val, a->lo, a->esc, a->counter,
                                        a->flags);
   return (const void*)k;
 }
@@ -658,6 +656,7 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
   int64_t* offsets = p->binmeta + kNumBins;
   int64_t* cursors = p->binmeta + 2 * kNumBins + 1;
   const LearnedOut lo{p->cap, p->slab_off, p->slab_col, p->slab_val, p->retry, p->lcount ? p->lcount + 1 : nullptr};
+  const EscArgs esc{p->prod, esc_min_products(p->tune), esc_per_margin(p->tune), p->tune.predict_slack};
   auto run_queue = [&](int which, bool learned) {
     QueueArgs a{};
     a.mats = p->d_mats;
@@ -672,8 +671,7 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
     a.c_col = p->c_col;
     a.c_val = p->c_val;
     a.lo = lo;
-    a.prod = p->prod;
-    a.esc_min = esc_min_products(p->tune);
+    a.esc = esc;
     a.counter = p->qcount + which;
     a.flags = ctx->d_flags;
     queue_dispatch(which, learned, &a, p->grid[learned ? 1 : 0][which], queue_smem(which), lc.stream);
@@ -689,9 +687,6 @@ void enqueue(spg_ctx* ctx, BatchPlan* p) {
     ++launches;
     for (int which : group) run_queue(which, learned);
   };
-  EscArgs esc;
-  esc.prod = p->prod;
-  esc.min_prod = esc_min_products(p->tune);
   auto run_esc = [&](bool learned) {
     for (int i = p->esc_bins - 1; i >= 0; --i) {
       const int threads = esc_warps(i) * 32, grid = p->esc_grid[learned ? 1 : 0][i];
@@ -896,8 +891,7 @@ spg_status build_plan(spg_ctx* ctx, int n, const spg_csr* A, const spg_csr* B, c
   // a folded row has at most twice as many products as its bound; bins past
   // that are not launched (3 us each) and get no row
   const int esc_min = esc_min_products(p->tune);
-  const int esc_bins = p->learned ? kBatchEscBinsLearned : kBatchEscBins;
-  for (int low = esc_min - 1; esc_min > 0 && p->esc_bins < esc_bins && low < 2 * most;)
+  for (int low = esc_min - 1; esc_min > 0 && p->esc_bins < kBatchEscBins && low < 2 * most;)
     low = esc_bin_products(p->esc_bins++);
   p->bp_num.esc_prod = p->bp_lrn.esc_prod = p->esc_bins > 0 ? esc_bin_products(p->esc_bins - 1) : 0;
   if (!p->individual.empty()) {

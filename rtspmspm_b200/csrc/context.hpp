@@ -137,6 +137,9 @@ inline int esc_min_products(const spg_tuning& t) {
   return t.esc_min_prod < 0 ? 0 : (t.esc_min_prod == 0 ? kEscMinProd : t.esc_min_prod);
 }
 
+// EscArgs::per_margin (0: no capacity below a row's products is folded).
+inline float esc_per_margin(const spg_tuning& t) { return t.predict_margin > 0.f ? 1.f / t.predict_margin : 0.f; }
+
 // Enqueues copies of `bytes` (a multiple of 4) device bytes each into the
 // mapped staging words at host_dst (inside ctx->h_stage), at most
 // StageCopies::kMax in one launch; valid after the next stream

@@ -26,10 +26,21 @@ constexpr int kNumEscBins = 5;
 // (32-bit words of shared memory a warp of it takes: esc_bin_words, warp_row.cuh)
 constexpr int esc_bin_products(int i) { return i == 0 ? 320 : i == 1 ? 640 : i == 2 ? 1152 : i == 3 ? 2048 : 4010; }
 // Symbolic: rows with a bitmap of their column span (span.cu), by its words.
-constexpr int kBinSpan = kBinEsc;
+constexpr int kBinSpan = kBinEsc + 1;
 constexpr int kNumSpanBins = 3;
+// The largest class ends at 65,536 columns because a warp's 8 KB leave an SM 28
+// warps; a class of 3,072 words would pay from about 480 products a row (80,000
+// columns, symbolic stage at 288 | 480 | 1,024 products 0.51 | 0.65 | 1.16 ms hashed,
+// 0.50 | 0.58 | 0.64 in it), but not in the place of this one (60,000 columns, 1,024
+// products 0.47 -> 0.63).
+constexpr int kSpanMinProd = 64;  // fewest products of such a row
 constexpr int span_bin_words(int i) { return i == 0 ? 576 : i == 1 ? 1216 : 2048; }
-constexpr int kBinHeavy = kBinEsc + kNumEscBins;  // numeric: column-tiled heavy rows
+// Rows of at most early_max columns that may leave the warp tables early
+// (big_row): behind the other big rows of a symbolic binning, before those of a
+// numeric one, so that either list goes on without a gap.
+constexpr int kBinEarlySym = kBinEsc;
+constexpr int kBinEarly = kBinEsc + kNumEscBins;
+constexpr int kBinHeavy = kBinEarly + 1;          // numeric: column-tiled heavy rows
 constexpr int kBinEmpty = kBinHeavy + 1;          // no products
 constexpr int kNumBins = kBinEmpty + 1;
 
@@ -73,6 +84,7 @@ struct BinParams {
   int64_t blk_large_cap;
   int64_t esc_cap;     // most entries of a row in the expand-sort-fold bins
   int esc_prod;        // and most products (esc_bin_products of the last bin in use; 0: none)
+  int64_t early_max;   // most entries of a row that a table of 2^kEarlyLog slots holds
   int64_t heavy_min;   // rows of more entries may be heavy below warp_cap too (big_row)
 };
 
@@ -82,15 +94,24 @@ struct BinParams {
 // from 2,048 entries 2.31, 2.53 and 1.84 ms, from 1,024 1.86, 1.79 and 1.14,
 // from 512 1.52, 1.53 and 0.80, from 256 1.46, 1.52 and 0.81.
 constexpr int64_t kHeavyMin = 512;
-// A row bounded by u entries goes the way of the heavy rows (symbolic bitmap,
-// units) when it is past the warp tables, or past heavy_min while its columns'
-// bitmap has at most 4 words an entry: clearing and counting it then costs no
-// more than hashing.
+// Those that a table of 2^kEarlyLog slots holds (early_max columns) leave only
+// beside others past it or when they are kEarlyRows or more: the units' launches take 40 us a call, and fewer rows
+// are one wave of tables (new values of 3,000 rows, 151 of them of 513 to 560
+// entries, 251 -> 203 us, of R-MAT 10, 31 of its 1,024 rows, 376 -> 335).
+constexpr int kEarlyLog = 11;
+constexpr int64_t kEarlyRows = 256;
+// A row bounded by u entries, `likely` of them distinct if its products fell at
+// random on the columns they can reach, goes the way of the heavy rows (symbolic
+// bitmap, units) when it is past the warp tables, or likely past heavy_min while
+// its columns' bitmap has at most 4 words an entry: clearing and counting it
+// then costs no more than hashing.  Rows of many products on few columns stay
+// (60,000 rows of 720 products in bands of 300 columns, counted in bitmaps and
+// then hashed all the same: 1,635 us a call, hashed twice 1,260).
 #ifdef __CUDACC__
 __host__ __device__
 #endif
-inline bool big_row(int64_t u, int64_t cols, int64_t warp_cap, int64_t heavy_min) {
-  return u > warp_cap || (u > heavy_min && cols <= 128 * u);
+inline bool big_row(int64_t u, int64_t likely, int64_t cols, int64_t warp_cap, int64_t heavy_min) {
+  return u > warp_cap || (likely > heavy_min && cols <= 128 * u);
 }
 
 // Whether such a row (prod products, out entries) is folded all the same: up to
@@ -130,8 +151,13 @@ void launch_widen_rp(const int32_t* in, int64_t n, int64_t* out, const LaunchCtx
 void launch_narrow_rp(const int64_t* in, int64_t n, int32_t* out, const LaunchCtx& lc);
 void launch_validate(const DCsr& M, int64_t nnz, int* flags, const LaunchCtx& lc);
 // Products of every row and, when `span` is given, the words of its column
-// span's bitmap (span_words; 0: none).
-void launch_row_products(const DCsr& A, const DCsr& B, int64_t* prod, const LaunchCtx& lc, int32_t* span = nullptr);
+// span's bitmap: 0 unknown, below 0 (for rows past heavy_min) when the row takes
+// no span bin.  Rows of more than `most` possible columns have none.
+void launch_row_products(const DCsr& A, const DCsr& B, int64_t* prod, const LaunchCtx& lc, int32_t* span = nullptr,
+                         int64_t most = 0, int64_t heavy_min = INT64_MAX);
+// The same words for the `count` (on the device) listed rows, 0 for all others.
+void launch_listed_spans(const DCsr& A, const DCsr& B, const int32_t* rows, const unsigned long long* count,
+                         const int64_t* prod, int32_t* span, int64_t most, int64_t heavy_min, const LaunchCtx& lc);
 
 // Small products (at most kSmallMaxRows rows of A, every row of at most
 // 2^kSmallLogT products): products and exact counts per row in one launch
@@ -163,6 +189,8 @@ constexpr int kEscMinProd = 32;
 struct EscArgs {
   const int64_t* prod = nullptr;
   int min_prod = 0;
+  float per_margin = 0.f;  // learned: 1 / margin and slack of a capacity (esc_guess)
+  int slack = 0;
 };
 void launch_sum(const int64_t* v, int64_t n, unsigned long long* out, const LaunchCtx& lc);
 // Rows into bins by their key; with `esc`, numeric and learned binnings send
@@ -192,12 +220,13 @@ void launch_num_warp_learned(int log_t, const DCsr& A, const DCsr& B, const int3
 // Span bitmaps: exact counts of the rows of a symbolic bin.
 void launch_sym_span(int bin, const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, int64_t* nnz,
                      int* flags, const LaunchCtx& lc);
-// Expand-sort-fold pass over the rows of bin kBinEsc + i: into C (off = its
-// row pointers, cap = null; the counts are checked) or into the slab (off = its
-// offsets; rows of more than cap[row] entries to `retry`, nnz -1).
-void launch_num_esc(int bin, const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, const int64_t* prod,
-                    const int64_t* off, int32_t* out_col, float* out_val, const int64_t* cap, int64_t* nnz,
-                    int32_t* retry, unsigned long long* retry_count, int* flags, const LaunchCtx& lc, int wpb);
+// Expand-sort-fold pass over the rows of the bins kBinEsc .. (bin_off: the
+// binning's offsets into `lists`, on the host): into C (off = its row pointers,
+// cap = null; the counts are checked) or into the slab (off = its offsets; rows of
+// more than cap[row] entries to `retry`, nnz -1).  Returns its launches.
+int launch_num_esc(const int64_t* bin_off, const DCsr& A, const DCsr& B, const int32_t* lists, const int64_t* prod,
+                   const int64_t* off, int32_t* out_col, float* out_val, const int64_t* cap, int64_t* nnz,
+                   int32_t* retry, unsigned long long* retry_count, int* flags, const LaunchCtx& lc, int wpb);
 // CTA-wide hash numeric pass over the rows of bin kBinBlock (2^12-slot
 // tables) or kBinDense (2^14) of a numeric / learned binning.
 void launch_num_block(int bin, const DCsr& A, const DCsr& B, const int32_t* rows, int64_t nrows, const int64_t* c_rp,

@@ -308,8 +308,13 @@ __device__ __forceinline__ void capacity_of(int64_t p, int64_t cols, float o0, f
   int64_t c = cd >= (double)u ? u : (int64_t)cd;
   if (c < 1) c = 1;
   if (force_overflow) c = 1;
-  const bool units = UNITS && c > heavy_min && big_row(c, cols, learn_cap, heavy_min) &&
-                     !(fold_big(p, (int64_t)pred) && esc_wanted(p, c, esc_min, esc_bin_products(kNumEscBins - 1)));
+  bool units = false;
+  if (UNITS && c > heavy_min) {
+    const int64_t likely = min(c, (int64_t)((float)cols * (1.f - expf(-(float)p / (float)cols))));
+    units = big_row(c, likely, cols, learn_cap, heavy_min) &&
+            !(fold_big(p, (int64_t)pred) &&
+              esc_wanted(p, esc_guess(c, p, 1.f / margin, slack), esc_min, esc_bin_products(kNumEscBins - 1)));
+  }
   if (c > learn_cap || units || (bin_gate && o1 > (float)kMaxLogT + 0.5f)) {
     ex = 1;
     c = 0;

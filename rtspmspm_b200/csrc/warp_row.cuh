@@ -486,30 +486,107 @@ __device__ __forceinline__ void next_row(int32_t* keys, int& epoch) {
 // few words.  A stable radix sort ranks every word of every pass with
 // __match_any_sync, which takes an SM about 70 cycles for 30 distinct digits.
 constexpr int kEscBuckets = 256;
-// A fuller bucket than this sends the row to a bitonic sort (columns crowded
-// into few of the ranges).
+// A fuller bucket than this sends the row to another sort (columns crowded into
+// few of the ranges): bitonic, or radix in the learned method's kernel, which folds
+// rows that its prediction takes for distinct (27-point grid of 200 x 200 x 4, 4.32
+// -> 2.64 ms a call).  Elsewhere the mere call of it costs the rows that are not
+// crowded 2 % (65,536 rows of 1,024 products 1.97 -> 2.01 ms).
 constexpr int kEscCrowd = 64;
 // Largest P that `words` 32-bit words of a warp's shared memory hold: two
 // word buffers, the values and the bucket counts.
-__host__ __device__ __forceinline__ int esc_capacity(int words) { return (words - kEscBuckets) / 3; }
+constexpr int esc_capacity(int words) { return (words - kEscBuckets) / 3; }
+// Warp tables whose memory holds fewer products leave folding out: the small
+// tables' kernels run faster without its code (1,000,000 rows of 6 products,
+// numeric 0.62 -> 0.51 ms).
+constexpr int kEscTableMin = 128;
 
 // Words of a warp of an expand-sort-fold bin holding rows of up to P products.
 constexpr int esc_bin_words(int P) { return (3 * P + kEscBuckets + 3) / 4 * 4; }
 
-// True when a row of `prod` products and at least `out` output entries
-// (its exact count, or the learned capacity) takes the expand-sort-fold
-// path: esc_min > 0 (0 turns it off), prod in [esc_min, cap] and at least
-// half of the products distinct.
+// True when a row of `prod` products and `out` output entries (its exact count,
+// or esc_guess of the learned capacity) takes the expand-sort-fold path: esc_min
+// > 0 (0 turns it off), prod in [esc_min, cap] and enough of the products
+// distinct: half of them from 128 products on, more of fewer (81 % at 48), all of
+// fewer than 48.  A hash row's time falls with the columns it keeps, a folded
+// row's does not: rows of 49 | 64 | 81 | 100 | 144 products break even at about
+// 82 | 73 | 70 | 58 | 48 % (columns close to one another; spread out earlier),
+// 36 products hardly at all; star stencils of 49 products on 25 columns 0.25 ms
+// hashed, 0.32 folded.
 __device__ __forceinline__ bool esc_wanted(int64_t prod, int64_t out, int esc_min, int cap) {
-  return esc_min > 0 && prod >= esc_min && prod <= cap && 2 * out >= prod;
+  if (esc_min <= 0 || prod < esc_min || prod > cap) return false;
+  return prod >= 128 ? 2 * out >= prod : prod >= 48 ? 256 * out >= prod * (256 - prod) : out >= prod;
+}
+
+// Output entries behind a learned capacity, margin * prediction + slack: the
+// prediction, or all products when the capacity was cut to them.  The capacity
+// itself would fold rows that keep a third of their products (27-point grid of
+// 200 x 200 x 4: 3.82 -> 4.32 ms a call, now 2.64).
+__device__ __forceinline__ int64_t esc_guess(int64_t cap, int64_t prod, float per_margin, int slack) {
+  return cap >= prod ? cap : (int64_t)((float)((int)cap - slack) * per_margin);
+}
+
+// Stable LSD radix sort of a row's P columns in buf (as much room again, the values
+// and kEscBuckets counters behind them), 8-bit digits: their words ((column - lo)
+// << ib) | position in order, at the word of buf returned.  Not inlined, for its
+// registers (5 to 8 % of the fold's other rows).
+static __device__ __noinline__ int esc_radix_sort(uint32_t* buf, int P, uint32_t lo, uint32_t span) {
+  uint32_t* wa = buf;
+  uint32_t* wb = buf + P;
+  int* hist = reinterpret_cast<int*>(buf + 3 * P);
+  const int span_bits = 32 - __clz(span);
+  const int ib = 32 - __clz((uint32_t)(P - 1));
+  static_assert(kEscBuckets == 256, "a counter per digit");
+  const int lane = lane_id();
+  const unsigned lt = (1u << lane) - 1u;
+  for (int i = lane; i < P; i += 32) wa[i] = ((wa[i] - lo) << ib) | (uint32_t)i;
+  __syncwarp();
+  uint32_t* src = wa;
+  uint32_t* dst = wb;
+  for (int shift = ib; shift < ib + span_bits; shift += 8) {
+    for (int b = lane; b < 256; b += 32) hist[b] = 0;
+    __syncwarp();
+    for (int i = lane; i < P; i += 32) atomicAdd(&hist[(src[i] >> shift) & 255u], 1);
+    __syncwarp();
+    int loc[8];
+    int sum = 0;
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      loc[x] = hist[lane * 8 + x];
+      sum += loc[x];
+    }
+    int run = warp_incl_scan(sum) - sum;
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      hist[lane * 8 + x] = run;
+      run += loc[x];
+    }
+    __syncwarp();
+    for (int i0 = 0; i0 < P; i0 += 32) {
+      const int i = i0 + lane;
+      const bool act = i < P;
+      const uint32_t v = act ? src[i] : 0u;
+      const int dig = act ? (int)((v >> shift) & 255u) : -1 - lane;
+      const unsigned grp = __match_any_sync(kFull, dig);
+      const int leader = __ffs(grp) - 1;
+      int at = 0;
+      if (act && lane == leader) at = atomicAdd(&hist[dig], __popc(grp));
+      at = __shfl_sync(kFull, at, leader);
+      if (act) dst[at + __popc(grp & lt)] = v;
+    }
+    __syncwarp();
+    uint32_t* t = src;
+    src = dst;
+    dst = t;
+  }
+  return (int)(src - buf);
 }
 
 // Writes the row (P >= 1 products) sorted into out_col/out_val (its first
 // `limit` entries) and returns its entry count, or -1, having written
 // nothing, when its column span and positions need more than 31 bits (the
 // caller hashes the row then).  `buf` holds esc_capacity(words) >= P; its
-// contents are scratch afterwards.
-template <bool R32>
+// contents are scratch afterwards.  RADIX: a crowded row is radix sorted.
+template <bool R32, bool RADIX = false>
 __device__ __forceinline__ int esc_row(const DCsr& A, const DCsr& B, int32_t row, int P, int32_t* buf, int64_t limit,
                                        int32_t* out_col, float* out_val) {
   using Off = typename RowOff<R32>::T;
@@ -606,6 +683,8 @@ __device__ __forceinline__ int esc_row(const DCsr& A, const DCsr& B, int32_t row
       for (int j = b0; j < b1; ++j) at += wb[j] < w;
       wa[at] = w;
     }
+  } else if (RADIX) {
+    src = wa + esc_radix_sort(wa, P, (uint32_t)lo, span);
   } else {
     for (int i = lane; i < P; i += 32) wa[i] = ((wa[i] - (uint32_t)lo) << ib) | (uint32_t)i;
     __syncwarp();
