@@ -16,8 +16,9 @@
 // a few products: R-MAT 16 7.0 -> 3.6 ms, R-MAT 18 35.4 -> 22.7 ms.
 // Measured and dropped (R-MAT 17, 7.0 ms as kept): units of 6,800 / 9,000
 // words 7.6 / 8.7 ms (fewer CTAs an SM), 256 threads 9.3, 64 threads 8.0, one
-// warp per unit 9.0 at R-MAT 16's scale of 4.8, runs of short segments added
-// by one warp 8.0, mbarriers in place of the CTA barrier 7.7 (more
+// warp per unit about 1.9 times the CTA (R-MAT 16), every run of short segments
+// added by one warp 8.0 (kPackSegment), no barrier between two segments of at most
+// 32 products 1.02 to 1.03 times, mbarriers in place of the CTA barrier 7.7 (more
 // instructions than the waits they take away).
 //
 // Reference counterpart: the any-hit multiply-accumulate into a dense row
@@ -579,8 +580,8 @@ static void num_unit_one(const DCsr& A, const DCsr& B, const int4* units, int64_
 
 void launch_num_units(const DCsr& A, const DCsr& B, const int32_t* heavy_rows, int64_t nheavy, const int32_t* big_slot,
                       const int32_t* tile_cnt, int ntiles, const int64_t* c_rp, int32_t* c_col, float* c_val,
-                      const int32_t* bidx, const uint32_t* bitmap, int64_t stride, bool c_known, int64_t whole_max, int4* units,
-                      int64_t room, unsigned long long* counters, int* flags, const LaunchCtx& lc) {
+                      const int32_t* bidx, const uint32_t* bitmap, int64_t stride, bool c_known, int64_t whole_max,
+                      int4* units, int64_t room, unsigned long long* counters, int* flags, const LaunchCtx& lc) {
   if (nheavy == 0) return;
   cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), lc.stream);
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nheavy + 7) / 8, (int64_t)lc.sms * 8));
